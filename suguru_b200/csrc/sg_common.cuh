@@ -115,15 +115,17 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// Asynchronous copy of one 4- or 8-byte element from global to shared memory
+// Asynchronous copy of one 4-, 8- or 16-byte element from global to shared memory
 // (cp.async, no register round trip): a staging loop issues all of its
 // copies before any completes; stage_wait() waits for this thread's copies,
 // and a barrier after it publishes them to the block.
 template <class T>
 __device__ __forceinline__ void stage_async(T* dst, const T* src) {
-  static_assert(sizeof(T) == 4 || sizeof(T) == 8, "element size");
+  static_assert(sizeof(T) == 4 || sizeof(T) == 8 || sizeof(T) == 16, "element size");
   const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-  if constexpr (sizeof(T) == 4)
+  if constexpr (sizeof(T) == 16)
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(d), "l"(src) : "memory");
+  else if constexpr (sizeof(T) == 4)
     asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(d), "l"(src) : "memory");
   else
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(d), "l"(src) : "memory");

@@ -154,17 +154,16 @@ struct sg_ctx {
   struct PoissonState {
     bool ready = false;
     double* r = nullptr;     // real FFT input / output [ktot][jtot][itot]
-    void* c = nullptr;       // modes [ktot][jtot][nmp] (double2), nmp = itot/2 + 1 rounded up to 8
-    // elimination tables per row type e = 0..3 (sg_poisson.cu): pivots z and
-    // multipliers d, [ktot][jtot][nmp] each, for the shift they were made with
+    void* c = nullptr;       // modes [itot/2 + 1][ktot][jtot] (double2)
+    // elimination pivots per row type e = 0..3 (sg_poisson.cu), laid out as
+    // the modes, for the shift they were made with
     double* zt[4] = {nullptr, nullptr, nullptr, nullptr};
-    double* dt[4] = {nullptr, nullptr, nullptr, nullptr};
     double tshift[4] = {0, 0, 0, 0};
     bool tvalid[4] = {false, false, false, false};
     double* tab = nullptr;   // xrt [itot/2 + 1], yrt [jtot]
-    double2* w = nullptr;    // twiddles of the row and column FFTs, then the row split's W^k
-    double2* wpost = nullptr;
-    alignas(8) unsigned char plan_x[128], plan_y[128];  // FFT plans (factorisations), see sg_poisson.cu
+    double2* w = nullptr;    // twiddle tables
+    double2* wpost = nullptr;  // the row split's W^k
+    alignas(8) unsigned char plans[512];  // FFT plans, see sg_poisson.cu
   } pois;
   // indicator function (sg_indicator.cu), set up by sg_set_indicator_params
   struct IndState {

@@ -1,18 +1,23 @@
 // sg_poisson.cu -- solver1d (solver.f90:43-157) after initsolver(e)
 // (initsolver.f90:11-130) on the GPU: periodic x and y by a real 2-D FFT of
 // every z plane, then for every (x, y) mode the reference's tridiagonal
-// elimination in z, one thread per mode in FP64, then the inverse FFT.
+// elimination in z in FP64, then the inverse FFT.
 //
 // The FFTs are the library's own (the reference's fft.f / 2DECOMP transforms
-// are FFTPACK-style mixed-radix FFTs): self-sorting (Stockham) mixed-radix
-// passes in shared memory, FP64, with twiddle factors tabulated once on the
-// host.  Per plane, forward: a real-to-complex transform of every x row (a
-// complex FFT of half length on x_even + i x_odd, then the usual split into the
-// itot/2 + 1 modes), then a complex FFT of every y column of those modes;
-// inverse: the y columns, then complex-to-real rows.  Both directions are
+// are FFTPACK-style mixed-radix FFTs): self-sorting (Stockham) passes, FP64,
+// with twiddle factors tabulated once on the host.  Both directions are
 // unnormalised, so that the pair multiplies by itot * jtot (the convention of
 // the callers).  Any itot/2 and jtot whose prime factors are at most
 // kMaxRadix are accepted.
+//
+// Modes lie [m][k][j] (x mode, level, y): the rows' kernels transpose as they
+// write and read (runs of the CTA's rows), so that the y transforms run on
+// contiguous sequences and the elimination on tiles of neighbouring columns.
+// A solve is five launches: rows_r2c, cols, tri_tile, cols, rows_c2r.
+// (A cluster of eight CTAs holding one x mode's whole plane over distributed
+// shared memory, for cols, tri_tile, cols in one launch, moves a third of
+// the bytes but took 119 us against 89 us at 256 x 256 x 128: 33 clusters
+// fit at once, and their loads, exchanges and sweeps run in lockstep.)
 //
 // The rows of initsolver(e), built in the kernel in the reference's order:
 //   a = c = dzi^2, b = -(a + c);
@@ -22,13 +27,14 @@
 //   e = 3:    b(kmax) = 1, a(1) = a(kmax) = c(kmax) = 0 (w = 0 at the top
 //             face), then b -= Rep/dt and b(kmax) = 1 again;
 // the eigenvalues xrt + yrt of the mode join b except in the last row of
-// e = 3.  The elimination keeps the reference's operations and roundings
-// (no fused multiply-add): for e = 0, 1 the mean mode's last pivot is then
+// e = 3.  The pivots keep the reference's operations and roundings (no
+// fused multiply-add): for e = 0, 1 the mean mode's last pivot is then
 // exactly zero whenever it is in exact arithmetic, and that mode's top value
 // is set to zero, as the reference does.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "sg_common.cuh"
@@ -74,348 +80,186 @@ __device__ __forceinline__ Rows solver_row(int k, int kmax, int e, double dzi, d
   return r;
 }
 
-// The elimination split in two.  Its pivots and multipliers depend only on
-// the mode's eigenvalue, the row type e and the shift, not on the right-hand
-// side, so tri_coeff_kernel runs the reference's forward recurrence for them
-// once per (e, shift) and tabulates, per plane k and mode slot,
+// The elimination split in two.  Its pivots depend only on the mode's
+// eigenvalue, the row type e and the shift, not on the right-hand side, so
+// tri_coeff_kernel runs the reference's forward recurrence for them once per
+// (e, shift) and tabulates, per x mode m, level k and y mode j ([m][k][j]),
 //   z_k = 1 / (b_k + lam - a_k d_{k-1})  (k < kmax-1; d_{-1} = 0),
-//   d_k = c_k z_k                        (k < kmax-1),
 //   z_{kmax-1} = bb - a d_{kmax-2}        (the last pivot itself, bb = b + lam
 //                                          except for e = 3),
-// with the same operations in the same order (no fused multiply-add), so a
-// solve with the tables gives the bits of the one-pass elimination.  The
-// solve (tri_apply_kernel) is then two first-order sweeps per mode:
+// with the same operations in the same order (no fused multiply-add: the mean
+// mode's exact zero depends on it).  The multipliers d_k = c_k z_k = dzi^2 z_k
+// (k < kmax-1) are one multiplication and are not stored.  A solve with the
+// table is two first-order sweeps per mode,
 //   q_0 = r_0 z_0, q_k = (r_k - a_k q_{k-1}) z_k, the last row divided by its
 //   pivot (or set to zero when the pivot is exactly zero: the mean mode of
 //   the Neumann rows, as the reference does), then x_k = q_k - d_k x_{k+1}.
-// A thread per mode; the columns of neighbouring threads are adjacent in
-// memory, and the loads of the next kPre planes are issued ahead of the
-// dependent arithmetic (a ring of registers).  Modes are laid out [k][j][m]
-// with nmp >= nxm slots per y row; slots m >= nxm are padding and skipped.
-constexpr int kPre = 32;
-
-__global__ void __launch_bounds__(128) tri_coeff_kernel(int kmax, int jtot, int nmp, int nxm, int e, double dzi,
-                                                        double shift, const double* __restrict__ xrt,
-                                                        const double* __restrict__ yrt, double* __restrict__ zt,
-                                                        double* __restrict__ dt) {
-  const long nm = (long)jtot * nmp;
-  const long m = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= nm || m % nmp >= nxm) return;
-  const double lam = __dadd_rn(xrt[m % nmp], yrt[m / nmp]);
+__global__ void __launch_bounds__(128) tri_coeff_kernel(int kmax, int jtot, int nxm, int e, double dzi, double shift,
+                                                        const double* __restrict__ xrt,
+                                                        const double* __restrict__ yrt, double* __restrict__ zt) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= nxm * jtot) return;
+  const int m = q / jtot, j = q - m * jtot;
+  const double lam = __dadd_rn(xrt[m], yrt[j]);
+  double* zm = zt + (long)m * kmax * jtot + j;
   Rows r = solver_row(0, kmax, e, dzi, shift);
   double z = __drcp_rn(__dadd_rn(r.b, lam));
   double dk = __dmul_rn(r.c, z);
-  zt[m] = z;
-  dt[m] = dk;
+  zm[0] = z;
   for (int k = 1; k < kmax - 1; ++k) {
     r = solver_row(k, kmax, e, dzi, shift);
     z = __drcp_rn(__dsub_rn(__dadd_rn(r.b, lam), __dmul_rn(r.a, dk)));
     dk = __dmul_rn(r.c, z);
-    zt[k * nm + m] = z;
-    dt[k * nm + m] = dk;
+    zm[(long)k * jtot] = z;
   }
   r = solver_row(kmax - 1, kmax, e, dzi, shift);
   const double bb = e == 3 ? r.b : __dadd_rn(r.b, lam);
-  zt[(kmax - 1) * nm + m] = __dsub_rn(bb, __dmul_rn(r.a, dk));
+  zm[(long)(kmax - 1) * jtot] = __dsub_rn(bb, __dmul_rn(r.a, dk));
 }
 
-__global__ void __launch_bounds__(128) tri_apply_kernel(int kmax, int jtot, int nmp, int nxm, int e, double dzi,
-                                                        const double* __restrict__ zt, const double* __restrict__ dt,
-                                                        double2* __restrict__ c) {
-  const long nm = (long)jtot * nmp;
-  const long m = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (m >= nm || m % nmp >= nxm) return;
-  // a_k of solver_row: 0 in row 0, dzi^2 in rows 1 .. kmax-2, and in row
-  // kmax-1 dzi^2 except for e = 3 (the identity row of w at the top)
-  const double a = __dmul_rn(dzi, dzi), a_last = e == 3 ? 0.0 : a;
-  double2 ring[kPre];
-  double zring[kPre];
+template <int V>
+using Const = std::integral_constant<int, V>;
+
+// The two sweeps of one real column (the real or the imaginary parts of a
+// mode's levels: the elimination's coefficients are real) at c[k cs], its
+// pivots at z[k zs]; a = dzi^2 is both a_k (k = 1 .. kmax-2) and c_k.  Bound
+// by the chain from level to level, so each sweep is one fused multiply-add
+// per level on it (8 cycles; the products r_k z_k and a z_k are off it) and
+// runs in blocks of B levels without branches, the next block's loads ahead
+// of the block's arithmetic.  (The three dependent operations of the
+// unfused form with a guarded load per level took 97 cycles a level.)
+// cs, zs: the strides, as constants (tri_tile_kernel) or values.
+template <int B, class SC, class SZ>
+__device__ __forceinline__ void tri_sweeps(double* c, const double* z, SC cs, SZ zs, int kmax, int e, double a) {
+  const int last = kmax - 1;
+  double r[B], w[B], rn[B], wn[B];
 #pragma unroll
-  for (int t = 0; t < kPre; ++t)
-    if (1 + t < kmax) {
-      ring[t] = c[(1 + t) * nm + m];
-      zring[t] = zt[(1 + t) * nm + m];
+  for (int t = 0; t < B; ++t) {
+    const int k = min(1 + t, last);
+    r[t] = c[k * cs];
+    w[t] = z[k * zs];
+  }
+  double p = c[0] * z[0];
+  c[0] = p;
+  int k = 1;
+  for (; k + B <= last; k += B) {
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+      const int q = min(k + B + t, last);
+      rn[t] = c[q * cs];
+      wn[t] = z[q * zs];
     }
-  double2 p = c[m];
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+      p = fma(-(a * w[t]), p, r[t] * w[t]);
+      c[(k + t) * cs] = p;
+    }
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+      r[t] = rn[t];
+      w[t] = wn[t];
+    }
+  }
+#pragma unroll
+  for (int t = 0; t < B; ++t)
+    if (k + t < last) {
+      p = fma(-(a * w[t]), p, r[t] * w[t]);
+      c[(k + t) * cs] = p;
+    }
   {
-    const double z = zt[m];
-    p.x = __dmul_rn(p.x, z);
-    p.y = __dmul_rn(p.y, z);
-    c[m] = p;
+    const double zk = z[last * zs], al = e == 3 ? 0.0 : a;  // e = 3: the identity row of w at the top
+    p = zk != 0.0 ? fma(-al, p, c[last * cs]) / zk : 0.0;
+    c[last * cs] = p;
   }
-  // forward sweep, rows 1 .. kmax-2
-  for (int k0 = 1; k0 < kmax - 1; k0 += kPre) {
 #pragma unroll
-    for (int t = 0; t < kPre; ++t) {
-      const int k = k0 + t;
-      if (k < kmax - 1) {
-        double2 q = ring[t];
-        const double z = zring[t];
-        if (k + kPre < kmax) {
-          ring[t] = c[(k + kPre) * nm + m];
-          zring[t] = zt[(k + kPre) * nm + m];
-        }
-        q.x = __dmul_rn(__dsub_rn(q.x, __dmul_rn(a, p.x)), z);
-        q.y = __dmul_rn(__dsub_rn(q.y, __dmul_rn(a, p.y)), z);
-        c[k * nm + m] = q;
-        p = q;
-      }
-    }
+  for (int t = 0; t < B; ++t) {
+    const int q = max(last - 1 - t, 0);
+    r[t] = c[q * cs];
+    w[t] = z[q * zs];
   }
-  {
-    const int k = kmax - 1;
-    const double z = zt[k * nm + m];
-    double2 q = c[k * nm + m];
-    if (z != 0.0) {
-      q.x = __ddiv_rn(__dsub_rn(q.x, __dmul_rn(a_last, p.x)), z);
-      q.y = __ddiv_rn(__dsub_rn(q.y, __dmul_rn(a_last, p.y)), z);
-    } else {
-      q.x = q.y = 0.0;
-    }
-    c[k * nm + m] = q;
-    p = q;
-  }
-  // back substitution, rows kmax-2 .. 0
+  k = last - 1;
+  for (; k - B >= -1; k -= B) {
 #pragma unroll
-  for (int t = 0; t < kPre; ++t) {
-    const int k = kmax - 2 - t;
-    if (k >= 0) {
-      ring[t] = c[k * nm + m];
-      zring[t] = dt[k * nm + m];
+    for (int t = 0; t < B; ++t) {
+      const int q = max(k - B - t, 0);
+      rn[t] = c[q * cs];
+      wn[t] = z[q * zs];
     }
-  }
-  for (int k0 = kmax - 2; k0 >= 0; k0 -= kPre) {
 #pragma unroll
-    for (int t = 0; t < kPre; ++t) {
-      const int k = k0 - t;
-      if (k >= 0) {
-        double2 q = ring[t];
-        const double dd = zring[t];
-        if (k - kPre >= 0) {
-          ring[t] = c[(k - kPre) * nm + m];
-          zring[t] = dt[(k - kPre) * nm + m];
-        }
-        q.x = __dsub_rn(q.x, __dmul_rn(dd, p.x));
-        q.y = __dsub_rn(q.y, __dmul_rn(dd, p.y));
-        c[k * nm + m] = q;
-        p = q;
-      }
+    for (int t = 0; t < B; ++t) {
+      p = fma(-(a * w[t]), p, r[t]);
+      c[(k - t) * cs] = p;
+    }
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+      r[t] = rn[t];
+      w[t] = wn[t];
     }
   }
+#pragma unroll
+  for (int t = 0; t < B; ++t)
+    if (k - t >= 0) {
+      p = fma(-(a * w[t]), p, r[t]);
+      c[(k - t) * cs] = p;
+    }
+}
+
+// C neighbouring columns of one x mode, all levels, per CTA: copied to shared
+// memory with their pivots, swept there by 2 C threads (real and imaginary
+// parts), written back: each mode is read and written once.  Bound by memory
+// (24 bytes in and 16 out per mode) with the sweeps' latency hidden by the
+// other CTAs on the SM: at 256 x 256 x 128, 40 us with C = 16 (4.4 TB/s)
+// against 46 us with C = 8, 69 us with C = 4 (short runs) and 41 us with
+// C = 32 (fewer CTAs); a thread per column on global memory with a register
+// ring, which stores and reloads the forward values, took 80 us.
+constexpr int kTriThreads = 64;
+
+template <int C>
+__global__ void __launch_bounds__(kTriThreads) tri_tile_kernel(int kmax, int jtot, int e, double a,
+                                                               const double* __restrict__ zt,
+                                                               double2* __restrict__ c) {
+  extern __shared__ __align__(16) double2 tsm[];  // [kmax][C] modes, then [kmax][C] pivots
+  double* zs = (double*)(tsm + kmax * C);
+  const int j0 = blockIdx.x * C, nj = min(C, jtot - j0);
+  const long o = (long)blockIdx.y * kmax * jtot + j0;
+  const int jl = threadIdx.x % C, k0 = threadIdx.x / C;
+  if (jl < nj)
+    for (int k = k0; k < kmax; k += kTriThreads / C) {
+      stage_async(&tsm[k * C + jl], &c[o + (long)k * jtot + jl]);
+      stage_async(&zs[k * C + jl], &zt[o + (long)k * jtot + jl]);
+    }
+  stage_wait();
+  __syncthreads();
+  if (threadIdx.x < 2 * nj)
+    tri_sweeps<8>((double*)tsm + threadIdx.x, zs + (threadIdx.x >> 1), Const<2 * C>{}, Const<C>{}, kmax, e, a);
+  __syncthreads();
+  if (jl < nj)
+    for (int k = k0; k < kmax; k += kTriThreads / C) c[o + (long)k * jtot + jl] = tsm[k * C + jl];
+}
+
+// Columns too long for a tile in shared memory: a thread per real column of
+// the modes in global memory.
+__global__ void __launch_bounds__(128) tri_apply_kernel(int kmax, int jtot, int nxm, int e, double a,
+                                                        const double* __restrict__ zt, double2* __restrict__ c) {
+  const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (q >= 2L * nxm * jtot) return;
+  const int part = (int)(q & 1), m = (int)((q >> 1) / jtot), j = (int)((q >> 1) % jtot);
+  const long o = (long)m * kmax * jtot + j;
+  tri_sweeps<16>((double*)(c + o) + part, zt + o, 2L * jtot, (long)jtot, kmax, e, a);
 }
 
 // ---------------------------------------------------------------- FFT ---
 constexpr int kMaxRadix = 61;
-constexpr int kMaxFactors = 16;
-constexpr int kFftThreads = 256;
-constexpr int kFftSmemComplex = 2048;  // complex values per buffer (two buffers: 64 KB)
-
-// Factorisation of a transform length (radices applied in this order) and its
-// twiddle table w[t] = exp(-2 pi i t / n), t < n.
-struct FftPlan {
-  int n, nf;
-  int radix[kMaxFactors];
-  const double2* w;
-};
+constexpr int kMaxPasses = 8;
+constexpr int kMaxLength = 2048;
 
 __device__ __forceinline__ double2 cmul(double2 a, double2 b) {
   return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
 }
 __device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
-
-// One radix-P butterfly of a self-sorting pass: v[r] = in[j + r n/P] times
-// exp(sign 2 pi i r k / (ns P)) (k = j mod ns), then the P-point DFT, V[q]
-// written to out[q ns] (out already offset to (j / ns) ns P + k).  The pass
-// twiddle index r k stride is below n (k < ns, r < P, stride = n / (ns P)).
-// Radices 2 and 4 apply their DFT with sign changes and swaps only; 3 and 5
-// take its roots from the table; all keep their values in registers.
-template <int P>
-__device__ __forceinline__ void butterfly(const double2* __restrict__ src, double2* __restrict__ dst, int j, int k,
-                                          int np, int ns, int stride, int wstep,
-                                          const double2* __restrict__ w, int sign) {
-  double2 v[P];
-#pragma unroll
-  for (int r = 0; r < P; ++r) {
-    double2 x = src[j + r * np];
-    if (r && k) {
-      double2 t = w[r * k * stride];
-      if (sign > 0) t = cconj(t);
-      x = cmul(x, t);
-    }
-    v[r] = x;
-  }
-  if constexpr (P == 2) {
-    dst[0] = make_double2(v[0].x + v[1].x, v[0].y + v[1].y);
-    dst[ns] = make_double2(v[0].x - v[1].x, v[0].y - v[1].y);
-  } else if constexpr (P == 4) {
-    // V_q = sum_r v_r exp(sign 2 pi i q r / 4): exp(sign i pi/2) = sign * i
-    const double2 s02 = make_double2(v[0].x + v[2].x, v[0].y + v[2].y);
-    const double2 d02 = make_double2(v[0].x - v[2].x, v[0].y - v[2].y);
-    const double2 s13 = make_double2(v[1].x + v[3].x, v[1].y + v[3].y);
-    const double2 d13 = make_double2(v[1].x - v[3].x, v[1].y - v[3].y);
-    // i * d13 = (-d13.y, d13.x)
-    const double sx = sign > 0 ? -d13.y : d13.y, sy = sign > 0 ? d13.x : -d13.x;  // sign * i * d13
-    dst[0] = make_double2(s02.x + s13.x, s02.y + s13.y);
-    dst[ns] = make_double2(d02.x + sx, d02.y + sy);
-    dst[2 * ns] = make_double2(s02.x - s13.x, s02.y - s13.y);
-    dst[3 * ns] = make_double2(d02.x - sx, d02.y - sy);
-  } else {
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      double2 acc = v[0];
-#pragma unroll
-      for (int r = 1; r < P; ++r) {
-        double2 t = w[((q * r) % P) * wstep];
-        if (sign > 0) t = cconj(t);
-        const double2 m = cmul(v[r], t);
-        acc.x += m.x;
-        acc.y += m.y;
-      }
-      dst[q * ns] = acc;
-    }
-  }
-}
-
-// The same for any radix p <= kMaxRadix: each output reads the p twiddled
-// inputs again from shared memory (no per-thread array).
-__device__ __forceinline__ void butterfly_any(const double2* __restrict__ src, double2* __restrict__ dst, int p,
-                                              int j, int k, int np, int ns, int stride, int wstep,
-                                              const double2* __restrict__ w, int sign) {
-#pragma unroll 1
-  for (int q = 0; q < p; ++q) {
-    double2 acc = make_double2(0.0, 0.0);
-#pragma unroll 1
-    for (int r = 0; r < p; ++r) {
-      double2 x = src[j + r * np];
-      if (r && k) {
-        double2 t = w[r * k * stride];
-        if (sign > 0) t = cconj(t);
-        x = cmul(x, t);
-      }
-      double2 t = w[((q * r) % p) * wstep];
-      if (sign > 0) t = cconj(t);
-      const double2 m = cmul(x, t);
-      acc.x += m.x;
-      acc.y += m.y;
-    }
-    dst[q * ns] = acc;
-  }
-}
-
-// nb sequences of length P.n in shared memory, sequence s at buf0 + s ld: self-sorting
-// mixed-radix passes (Stockham), ping-ponging between buf0 and buf1; returns
-// the buffer that holds the result.  sign = -1: forward (exp(-i..)), +1:
-// inverse, unnormalised.  For a pass of radix p after sub-transforms of
-// length ns: butterfly j < n/p takes v[r] = in[j + r n/p], twiddles it by
-// exp(sign 2 pi i r k / (ns p)) with k = j mod ns, forms the p-point DFT and
-// writes V[q] to out[(j / ns) ns p + k + q ns].
-__device__ double2* fft_smem(double2* buf0, double2* buf1, int nb, int ld, const FftPlan& P, int sign) {
-  const int n = P.n;
-  double2* in = buf0;
-  double2* out = buf1;
-  int ns = 1;
-  for (int f = 0; f < P.nf; ++f) {
-    const int p = P.radix[f], np = n / p, stride = n / (ns * p), wstep = n / p;
-    __syncthreads();
-    for (int idx = threadIdx.x; idx < nb * np; idx += blockDim.x) {
-      const int sq = idx / np, j = idx - sq * np, k = j % ns;
-      const double2* src = in + sq * ld;
-      double2* dst = out + sq * ld + (j / ns) * ns * p + k;
-      switch (p) {
-        case 2: butterfly<2>(src, dst, j, k, np, ns, stride, wstep, P.w, sign); break;
-        case 3: butterfly<3>(src, dst, j, k, np, ns, stride, wstep, P.w, sign); break;
-        case 4: butterfly<4>(src, dst, j, k, np, ns, stride, wstep, P.w, sign); break;
-        case 5: butterfly<5>(src, dst, j, k, np, ns, stride, wstep, P.w, sign); break;
-        default: butterfly_any(src, dst, p, j, k, np, ns, stride, wstep, P.w, sign); break;
-      }
-    }
-    ns *= p;
-    double2* t = in;
-    in = out;
-    out = t;
-  }
-  __syncthreads();
-  return in;
-}
-
-// Forward real-to-complex transform of rows of nx = 2 n reals (row r of the
-// block at src + r nx): z_m = x_2m + i x_2m+1, Z = FFT_n(z), then for
-// k = 0 .. n: X_k = (Z_k + conj Z_{n-k}) / 2 - (i/2) W^k (Z_k - conj Z_{n-k}),
-// W = exp(-2 pi i / nx), Z_n = Z_0; rows of n + 1 modes at dst + r ld.
-__global__ void __launch_bounds__(kFftThreads) fft_rows_r2c(long nrows, int rows_per_cta, int ld, FftPlan P,
-                                                            const double2* __restrict__ wpost,
-                                                            const double* __restrict__ src, double2* __restrict__ dst) {
-  extern __shared__ __align__(16) double2 fsm[];
-  const int n = P.n, nm = n + 1;
-  const long r0 = (long)blockIdx.x * rows_per_cta;
-  const int nb = (int)min((long)rows_per_cta, nrows - r0);
-  double2* b0 = fsm;
-  double2* b1 = fsm + rows_per_cta * n;
-  const double2* s2 = (const double2*)(src + r0 * 2 * n);
-  for (int t = threadIdx.x; t < nb * n; t += blockDim.x) b0[t] = s2[t];
-  const double2* Z = fft_smem(b0, b1, nb, n, P, -1);
-  for (int t = threadIdx.x; t < nb * nm; t += blockDim.x) {
-    const int r = t / nm, k = t - r * nm;
-    const double2 zk = Z[r * n + (k == n ? 0 : k)], zc = cconj(Z[r * n + (k == 0 ? 0 : n - k)]);
-    const double2 e = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y + zc.y));
-    const double2 o = make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y - zc.y));
-    const double2 wo = cmul(wpost[k], o);  // W^k o; times -i: (wo.y, -wo.x)
-    dst[(r0 + r) * ld + k] = make_double2(e.x + wo.y, e.y - wo.x);
-  }
-}
-
-// Inverse complex-to-real rows: from the n + 1 modes X_k of a row,
-// Z_k = (X_k + conj X_{n-k}) + i conj(W^k) (X_k - conj X_{n-k}), k < n,
-// z = unnormalised inverse FFT_n(Z), x_2m = Re z_m, x_2m+1 = Im z_m (nx x).
-__global__ void __launch_bounds__(kFftThreads) fft_rows_c2r(long nrows, int rows_per_cta, int ld, FftPlan P,
-                                                            const double2* __restrict__ wpost,
-                                                            const double2* __restrict__ src, double* __restrict__ dst) {
-  extern __shared__ __align__(16) double2 fsm[];
-  const int n = P.n, nm = n + 1;
-  const long r0 = (long)blockIdx.x * rows_per_cta;
-  const int nb = (int)min((long)rows_per_cta, nrows - r0);
-  double2* b0 = fsm;
-  double2* b1 = fsm + rows_per_cta * n;
-  double2* b2 = fsm + 2 * rows_per_cta * n;  // the modes, [nb][n + 1]
-  for (int t = threadIdx.x; t < nb * nm; t += blockDim.x) {
-    const int r = t / nm, k = t - r * nm;
-    b2[t] = src[(r0 + r) * ld + k];
-  }
-  __syncthreads();
-  for (int t = threadIdx.x; t < nb * n; t += blockDim.x) {
-    const int r = t / n, k = t - r * n;
-    const double2 xk = b2[r * nm + k], xc = cconj(b2[r * nm + n - k]);
-    const double2 sum = make_double2(xk.x + xc.x, xk.y + xc.y), dif = make_double2(xk.x - xc.x, xk.y - xc.y);
-    const double2 t2 = cmul(cconj(wpost[k]), dif);  // times i: (-t2.y, t2.x)
-    b0[t] = make_double2(sum.x - t2.y, sum.y + t2.x);
-  }
-  const double2* z = fft_smem(b0, b1, nb, n, P, +1);
-  double2* d2 = (double2*)(dst + r0 * 2 * n);
-  for (int t = threadIdx.x; t < nb * n; t += blockDim.x) d2[t] = z[t];
-}
-
-// Complex transforms of the columns of planes [nplanes][ny][ld] (ncols of
-// them valid): the CTA takes plane blockIdx.y and columns c0 .. c0 + cb - 1;
-// each warp loads runs of cb consecutive modes of a row.
-__global__ void __launch_bounds__(kFftThreads) fft_cols(int ncols, int ld, int cols_per_cta, FftPlan P, int sign,
-                                                        double2* __restrict__ data) {
-  extern __shared__ __align__(16) double2 fsm[];
-  const int ny = P.n, lds = ny + 1, c0 = blockIdx.x * cols_per_cta, cb = min(cols_per_cta, ncols - c0);
-  double2* plane = data + (long)blockIdx.y * ny * ld;
-  double2* b0 = fsm;
-  double2* b1 = fsm + cols_per_cta * lds;
-  // sequences at stride ny + 1: the transposing stores of neighbouring
-  // columns fall in different banks
-  for (int t = threadIdx.x; t < cb * ny; t += blockDim.x) {
-    const int j = t / cb, c = t - j * cb;
-    b0[c * lds + j] = plane[(long)j * ld + c0 + c];
-  }
-  const double2* Y = fft_smem(b0, b1, cb, lds, P, sign);
-  for (int t = threadIdx.x; t < cb * ny; t += blockDim.x) {
-    const int j = t / cb, c = t - j * cb;
-    plane[(long)j * ld + c0 + c] = Y[c * lds + j];
-  }
-}
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 cswap(double2 a) { return make_double2(a.y, a.x); }
 
 // ------------------------------------------------- power-of-two FFTs ---
 // Lengths N = 32, 64, 128, 256: a sequence belongs to TPS = N/8 consecutive
@@ -603,47 +447,230 @@ __device__ __forceinline__ void store_last(const double2 (&v)[8], double2* seq, 
   store_pass<N, LastPass<N>::R, LastPass<N>::NS>(v, seq, tau);
 }
 
-constexpr int kRegThreads = 256;
+// ------------------------------------------------- mixed-radix FFTs ---
+// Every other length: Stockham passes between two buffers in shared memory,
+// with radices up to 16 whose butterflies stay in registers (composite ones
+// built from their factors), so that most lengths take two passes: one pass
+// per prime factor spent its time in shared memory and in barriers (a 150-
+// point transform had four).  Forward transforms only: an inverse transform
+// swaps the real and imaginary parts of its input and of its output.
+//
+// x / d for x < 2^16 and 1 <= d <= 2^15 as a multiplication: m = floor(2^32 / d) + 1.
+struct FastDiv {
+  unsigned d, m;
+};
+__device__ __forceinline__ int fdiv_u(int x, FastDiv f) { return f.d == 1 ? x : (int)__umulhi((unsigned)x, f.m); }
 
-// Real-to-complex rows (complex length N = nx / 2), 256 / (N / 8) rows per
-// CTA, the post-processing split of fft_rows_r2c.  Loads go straight from
-// global memory into the first pass's registers (a half-row run of 16-byte
-// values per group of lanes); the modes are written with stride ld.
-template <int N>
-__global__ void __launch_bounds__(kRegThreads) rows_r2c_reg(long nrows, int ld, const double2* __restrict__ tw_g,
-                                                           const double2* __restrict__ wp_g,
-                                                           const double* __restrict__ src, double2* __restrict__ dst) {
-  constexpr int TPS = N / 8, SPC = kRegThreads / TPS, LD = N + 1;
-  __shared__ double2 tw[TwTab<N>::size], wp[N + 1];
-  __shared__ double2 buf[SPC * LD];
-  fill_tw<N>(tw, tw_g, threadIdx.x, kRegThreads);
-  for (int t = threadIdx.x; t <= N; t += kRegThreads) wp[t] = wp_g[t];
-  const int sq = threadIdx.x / TPS, tau = threadIdx.x % TPS;
-  const long row = (long)blockIdx.x * SPC + sq;
-  const bool ok = row < nrows;
-  const double2* s = (const double2*)src + row * N;
-  double2 v[8];
+// Pass of radix p after sub-transforms of length ns: np = n / p butterflies;
+// its twiddles tw[off + (r-1) ns + k] = exp(-2 pi i r k / (ns p)).
+struct FftPass {
+  int p, off;
+  FastDiv np, ns;
+};
+struct FftPlan {
+  int n, nf;
+  FftPass pass[kMaxPasses];
+  const double2* tw;
+};
+
+// buffer position of element e: one slot of padding after every eight, so
+// that the passes' strided writes (stride p) spread over the banks
+__host__ __device__ constexpr int fpad(int e) { return e + (e >> 3); }
+__host__ __device__ constexpr int fld(int n) { return fpad(n) + 1; }
+
+// forward DFTs of P values in registers, V_q = sum_r v_r exp(-2 pi i q r / P)
+template <int P>
+__device__ __forceinline__ void dft_fwd(double2* v);
+
+// coprime A, B (the prime-factor map: input n = B a + A b mod A B, output q
+// with q = qa mod A and q = qb mod B): no twiddles between the factors
+template <int A, int B>
+__device__ __forceinline__ void dft_coprime(double2* v) {
+  constexpr int N = A * B;
+  double2 t[N];
 #pragma unroll
-  for (int r = 0; r < 8; ++r) v[r] = ok ? s[tau + r * TPS] : make_double2(0.0, 0.0);
-  __syncthreads();  // the tables
-  double2* seq = buf + sq * LD;
-  fft_reg<N>(v, seq, tau, tw, -1);
-  __syncwarp();
-  store_last<N>(v, seq, tau);
-  __syncwarp();
-  if (!ok) return;
-  double2* o = dst + row * ld;
+  for (int b = 0; b < B; ++b) {
+    double2 u[A];
 #pragma unroll
-  for (int i = 0; i <= 8; ++i) {
-    const int k = tau + i * TPS;
-    if (k <= N) {
-      const double2 zk = seq[swz(k & (N - 1))], zc = cconj(seq[swz((N - k) & (N - 1))]);
-      const double2 e = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y + zc.y));
-      const double2 od = make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y - zc.y));
-      const double2 wo = cmul(wp[k], od);
-      o[k] = make_double2(e.x + wo.y, e.y - wo.x);
-    }
+    for (int a = 0; a < A; ++a) u[a] = v[(B * a + A * b) % N];
+    dft_fwd<A>(u);
+#pragma unroll
+    for (int a = 0; a < A; ++a) t[a * B + b] = u[a];
   }
+#pragma unroll
+  for (int a = 0; a < A; ++a) dft_fwd<B>(&t[a * B]);
+#pragma unroll
+  for (int q = 0; q < N; ++q) v[q] = t[(q % A) * B + q % B];
+}
+
+// odd prime P from the cosines and sines c[r], s[r] of 2 pi r / P: the sums
+// and differences of v_r and v_{P-r} take real factors
+template <int P>
+__device__ __forceinline__ void dft_odd(double2* v, const double (&c)[P / 2 + 1], const double (&s)[P / 2 + 1]) {
+  constexpr int H = P / 2;
+  double2 a[H], b[H];
+#pragma unroll
+  for (int r = 1; r <= H; ++r) {
+    a[r - 1] = cadd(v[r], v[P - r]);
+    b[r - 1] = csub(v[r], v[P - r]);
+  }
+  const double2 v0 = v[0];
+  double2 sum = v0;
+#pragma unroll
+  for (int r = 0; r < H; ++r) sum = cadd(sum, a[r]);
+  v[0] = sum;
+#pragma unroll
+  for (int q = 1; q <= H; ++q) {
+    double2 e = v0, o = make_double2(0.0, 0.0);
+#pragma unroll
+    for (int r = 1; r <= H; ++r) {
+      const int qr = (q * r) % P, i = qr <= H ? qr : P - qr;
+      const double sn = qr <= H ? s[i] : -s[i];
+      e.x += c[i] * a[r - 1].x;
+      e.y += c[i] * a[r - 1].y;
+      o.x += sn * b[r - 1].x;
+      o.y += sn * b[r - 1].y;
+    }
+    v[q] = make_double2(e.x + o.y, e.y - o.x);  // e - i o
+    v[P - q] = make_double2(e.x - o.y, e.y + o.x);
+  }
+}
+
+// A x B values with the twiddles exp(-2 pi i a b / (A B)) between the factors
+template <int A, int B>
+__device__ __forceinline__ void dft_square(double2* v, const double2 (&w)[A][B]) {
+  double2 t[A * B];
+#pragma unroll
+  for (int b = 0; b < B; ++b) {  // input n = B a + b
+    double2 u[A];
+#pragma unroll
+    for (int a = 0; a < A; ++a) u[a] = v[B * a + b];
+    dft_fwd<A>(u);
+#pragma unroll
+    for (int a = 0; a < A; ++a) t[a * B + b] = a && b ? cmul(u[a], w[a][b]) : u[a];
+  }
+#pragma unroll
+  for (int a = 0; a < A; ++a) {
+    dft_fwd<B>(&t[a * B]);
+#pragma unroll
+    for (int b = 0; b < B; ++b) v[a + A * b] = t[a * B + b];
+  }
+}
+
+template <> __device__ __forceinline__ void dft_fwd<2>(double2* v) { dft_reg<2>(v, -1); }
+template <> __device__ __forceinline__ void dft_fwd<4>(double2* v) { dft_reg<4>(v, -1); }
+template <> __device__ __forceinline__ void dft_fwd<8>(double2* v) { dft_reg<8>(v, -1); }
+template <> __device__ __forceinline__ void dft_fwd<3>(double2* v) {
+  const double c[2] = {1.0, -0.5}, s[2] = {0.0, 0.86602540378443864676};
+  dft_odd<3>(v, c, s);
+}
+template <> __device__ __forceinline__ void dft_fwd<5>(double2* v) {
+  const double c[3] = {1.0, 0.30901699437494742410, -0.80901699437494742410};
+  const double s[3] = {0.0, 0.95105651629515357212, 0.58778525229247312917};
+  dft_odd<5>(v, c, s);
+}
+template <> __device__ __forceinline__ void dft_fwd<7>(double2* v) {
+  const double c[4] = {1.0, 0.62348980185873353053, -0.22252093395631440429, -0.90096886790241912624};
+  const double s[4] = {0.0, 0.78183148246802980871, 0.97492791218182360702, 0.43388373911755812048};
+  dft_odd<7>(v, c, s);
+}
+template <> __device__ __forceinline__ void dft_fwd<6>(double2* v) { dft_coprime<2, 3>(v); }
+template <> __device__ __forceinline__ void dft_fwd<10>(double2* v) { dft_coprime<2, 5>(v); }
+template <> __device__ __forceinline__ void dft_fwd<12>(double2* v) { dft_coprime<4, 3>(v); }
+template <> __device__ __forceinline__ void dft_fwd<14>(double2* v) { dft_coprime<2, 7>(v); }
+template <> __device__ __forceinline__ void dft_fwd<15>(double2* v) { dft_coprime<3, 5>(v); }
+template <> __device__ __forceinline__ void dft_fwd<9>(double2* v) {
+  constexpr double c1 = 0.76604444311897803520, s1 = 0.64278760968653932632;  // 2 pi / 9
+  constexpr double c2 = 0.17364817766693034885, s2 = 0.98480775301220805937;
+  constexpr double c4 = -0.93969262078590838405, s4 = 0.34202014332566873304;
+  const double2 w[3][3] = {{{1, 0}, {1, 0}, {1, 0}}, {{1, 0}, {c1, -s1}, {c2, -s2}}, {{1, 0}, {c2, -s2}, {c4, -s4}}};
+  dft_square<3, 3>(v, w);
+}
+template <> __device__ __forceinline__ void dft_fwd<16>(double2* v) {
+  constexpr double c1 = 0.92387953251128675613, s1 = 0.38268343236508977173, h = 0.70710678118654752440;
+  const double2 w[4][4] = {{{1, 0}, {1, 0}, {1, 0}, {1, 0}},
+                           {{1, 0}, {c1, -s1}, {h, -h}, {s1, -c1}},
+                           {{1, 0}, {h, -h}, {0, -1}, {-h, -h}},
+                           {{1, 0}, {s1, -c1}, {-h, -h}, {-c1, s1}}};
+  dft_square<4, 4>(v, w);
+}
+
+template <int P>
+__device__ __forceinline__ void any_pass(const double2* in, double2* out, int nb, int ld, const FftPass& F,
+                                         const double2* __restrict__ tw) {
+  const int np = (int)F.np.d, ns = (int)F.ns.d;
+  const double2* t = tw + F.off;
+  for (int idx = threadIdx.x; idx < nb * np; idx += blockDim.x) {
+    const int sq = fdiv_u(idx, F.np), j = idx - sq * np, k = j - fdiv_u(j, F.ns) * ns;
+    const double2* src = in + sq * ld;
+    double2 v[P];
+#pragma unroll
+    for (int r = 0; r < P; ++r) v[r] = src[fpad(j + r * np)];
+    if (ns > 1)
+#pragma unroll
+      for (int r = 1; r < P; ++r) v[r] = cmul(v[r], t[(r - 1) * ns + k]);
+    dft_fwd<P>(v);
+    double2* dst = out + sq * ld;
+    const int o = (j - k) * P + k;
+#pragma unroll
+    for (int q = 0; q < P; ++q) dst[fpad(o + q * ns)] = v[q];
+  }
+}
+
+// any prime radix up to kMaxRadix, straight from its definition: a thread per
+// output; the P-point roots are twiddles too (wroot[t] = exp(-2 pi i t / p))
+__device__ __forceinline__ void prime_pass(const double2* in, double2* out, int nb, int ld, const FftPass& F,
+                                           const double2* __restrict__ tw) {
+  const int p = F.p, np = (int)F.np.d, ns = (int)F.ns.d, n = np * p;
+  const double2* t = tw + F.off;
+  const double2* root = t + (p - 1) * ns;
+  for (int idx = threadIdx.x; idx < nb * n; idx += blockDim.x) {
+    const int bq = fdiv_u(idx, F.np), j = idx - bq * np, sq = bq / p, q = bq - sq * p;
+    const int k = j - fdiv_u(j, F.ns) * ns;
+    const double2* src = in + sq * ld;
+    double2 acc = src[fpad(j)];
+    int qr = 0;
+    for (int r = 1; r < p; ++r) {
+      qr += q;
+      if (qr >= p) qr -= p;
+      const double2 x = cmul(src[fpad(j + r * np)], cmul(t[(r - 1) * ns + k], root[qr]));
+      acc = cadd(acc, x);
+    }
+    out[sq * ld + fpad((j - k) * p + k + q * ns)] = acc;
+  }
+}
+
+// nb sequences of length P.n in shared memory, sequence s at b0 + s ld
+// (element e at fpad(e)), transformed forward between b0 and b1; returns the
+// buffer that holds the result.  Begins and ends with a block barrier.
+__device__ __forceinline__ double2* fft_any(double2* b0, double2* b1, int nb, int ld, const FftPlan& P) {
+  double2* in = b0;
+  double2* out = b1;
+  for (int f = 0; f < P.nf; ++f) {
+    const FftPass& F = P.pass[f];
+    __syncthreads();
+    switch (F.p) {
+      case 2: any_pass<2>(in, out, nb, ld, F, P.tw); break;
+      case 3: any_pass<3>(in, out, nb, ld, F, P.tw); break;
+      case 4: any_pass<4>(in, out, nb, ld, F, P.tw); break;
+      case 5: any_pass<5>(in, out, nb, ld, F, P.tw); break;
+      case 6: any_pass<6>(in, out, nb, ld, F, P.tw); break;
+      case 7: any_pass<7>(in, out, nb, ld, F, P.tw); break;
+      case 8: any_pass<8>(in, out, nb, ld, F, P.tw); break;
+      case 9: any_pass<9>(in, out, nb, ld, F, P.tw); break;
+      case 10: any_pass<10>(in, out, nb, ld, F, P.tw); break;
+      case 12: any_pass<12>(in, out, nb, ld, F, P.tw); break;
+      case 14: any_pass<14>(in, out, nb, ld, F, P.tw); break;
+      case 15: any_pass<15>(in, out, nb, ld, F, P.tw); break;
+      case 16: any_pass<16>(in, out, nb, ld, F, P.tw); break;
+      default: prime_pass(in, out, nb, ld, F, P.tw); break;
+    }
+    double2* t = in;
+    in = out;
+    out = t;
+  }
+  __syncthreads();
+  return in;
 }
 
 // Where the inverse rows put the solution: dense (f == nullptr: into the
@@ -656,13 +683,156 @@ struct RowsOut {
   int jtot;
 };
 
-// Complex-to-real rows, the pre-processing of fft_rows_c2r: the modes of the
-// CTA's rows go through shared memory (row pairs X_k, X_{n-k}), the first
-// pass's inputs are formed in registers, the last pass writes the reals
-// straight to global memory (16-byte runs, or pairs of 8-byte values into a
-// halo field).
+// Forward real-to-complex transform of nb rows of nx = 2 n reals per CTA:
+// z_m = x_2m + i x_2m+1, Z = FFT_n(z), then for k = 0 .. n:
+// X_k = (Z_k + conj Z_{n-k}) / 2 - (i/2) W^k (Z_k - conj Z_{n-k}),
+// W = exp(-2 pi i / nx), Z_n = Z_0; mode k of row r at dst[k nrows + r].
+constexpr int kAnyThreads = 128;
+
+__global__ void __launch_bounds__(kAnyThreads, 4) rows_r2c_any(long nrows, FastDiv nb, FftPlan P,
+                                                            const double2* __restrict__ wpost,
+                                                            const double* __restrict__ src, double2* __restrict__ dst) {
+  extern __shared__ __align__(16) double2 fsm[];
+  const int n = P.n, ld = fld(n);
+  const long r0 = (long)blockIdx.x * nb.d;
+  const int rows = (int)min((long)nb.d, nrows - r0);
+  double2* b0 = fsm;
+  double2* b1 = fsm + nb.d * ld;
+  const double2* s2 = (const double2*)src + r0 * n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r = warp; r < rows; r += kAnyThreads / 32)
+    for (int t = lane; t < n; t += 32) b0[r * ld + fpad(t)] = s2[(long)r * n + t];
+  const double2* Z = fft_any(b0, b1, rows, ld, P);
+  for (int t = threadIdx.x; t < (n + 1) * (int)nb.d; t += kAnyThreads) {
+    const int k = fdiv_u(t, nb), r = t - k * nb.d;
+    if (r >= rows) continue;
+    const double2 zk = Z[r * ld + fpad(k == n ? 0 : k)], zc = cconj(Z[r * ld + fpad(k == 0 ? 0 : n - k)]);
+    const double2 e = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y + zc.y));
+    const double2 o = make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y - zc.y));
+    const double2 wo = cmul(wpost[k], o);  // W^k o; times -i: (wo.y, -wo.x)
+    dst[(long)k * nrows + r0 + r] = make_double2(e.x + wo.y, e.y - wo.x);
+  }
+}
+
+// Inverse complex-to-real rows: from the n + 1 modes X_k of a row,
+// Z_k = (X_k + conj X_{n-k}) + i conj(W^k) (X_k - conj X_{n-k}), k < n,
+// z = unnormalised inverse FFT_n(Z), x_2m = Re z_m, x_2m+1 = Im z_m (nx x).
+__global__ void __launch_bounds__(kAnyThreads, 4) rows_c2r_any(long nrows, FastDiv nb, FftPlan P,
+                                                            const double2* __restrict__ wpost,
+                                                            const double2* __restrict__ src, double* __restrict__ dst,
+                                                            RowsOut out) {
+  extern __shared__ __align__(16) double2 fsm[];
+  const int n = P.n, ld = fld(n);
+  const long r0 = (long)blockIdx.x * nb.d;
+  const int rows = (int)min((long)nb.d, nrows - r0);
+  double2* b0 = fsm;
+  double2* b1 = fsm + nb.d * ld;
+  for (int t = threadIdx.x; t < (n / 2 + 1) * (int)nb.d; t += kAnyThreads) {
+    const int k = fdiv_u(t, nb), r = t - k * nb.d;
+    if (r >= rows) continue;
+    const double2 a = src[(long)k * nrows + r0 + r], b = src[(long)(n - k) * nrows + r0 + r];
+    auto z = [&](double2 x, double2 y, int q) {  // Z_q from X_q = x and X_{n-q} = y
+      const double2 yc = cconj(y);
+      const double2 sum = cadd(x, yc), t2 = cmul(cconj(wpost[q]), csub(x, yc));  // times i: (-t2.y, t2.x)
+      return make_double2(sum.x - t2.y, sum.y + t2.x);
+    };
+    b0[r * ld + fpad(k)] = cswap(z(a, b, k));
+    if (k > 0) b0[r * ld + fpad(n - k)] = cswap(z(b, a, n - k));
+  }
+  const double2* z = fft_any(b0, b1, rows, ld, P);  // swapped: (Im, Re)
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r = warp; r < rows; r += kAnyThreads / 32) {
+    const long row = r0 + r;
+    if (!out.f) {
+      double2* d2 = (double2*)dst + row * n;
+      for (int t = lane; t < n; t += 32) d2[t] = cswap(z[r * ld + fpad(t)]);
+    } else {
+      const int j = (int)(row % out.jtot);
+      const long k = row / out.jtot;
+      double* f = out.f + (k + 1) * out.plane + (j + 1) * out.ldi + 1;
+      for (int i = lane; i < 2 * n; i += 32) {
+        const double2 v = z[r * ld + fpad(i >> 1)];
+        f[i] = (i & 1 ? v.x : v.y) * out.scale;
+      }
+    }
+  }
+}
+
+// y transforms: nseq contiguous sequences, nb per CTA, in place; an inverse by
+// swapping parts
+__global__ void __launch_bounds__(kAnyThreads, 4) cols_any(long nseq, int nb, FftPlan P, bool inv,
+                                                        double2* __restrict__ data) {
+  extern __shared__ __align__(16) double2 fsm[];
+  const int n = P.n, ld = fld(n);
+  const long s0 = (long)blockIdx.x * nb;
+  const int ns = (int)min((long)nb, nseq - s0);
+  double2* d = data + s0 * n;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int r = warp; r < ns; r += kAnyThreads / 32)
+    for (int t = lane; t < n; t += 32) {
+      const double2 x = d[(long)r * n + t];
+      fsm[r * ld + fpad(t)] = inv ? cswap(x) : x;
+    }
+  const double2* y = fft_any(fsm, fsm + nb * ld, ns, ld, P);
+  for (int r = warp; r < ns; r += kAnyThreads / 32)
+    for (int t = lane; t < n; t += 32) {
+      const double2 x = y[r * ld + fpad(t)];
+      d[(long)r * n + t] = inv ? cswap(x) : x;
+    }
+}
+
+constexpr int kRegThreads = 256;
+
+// Real-to-complex rows (complex length N = nx / 2), 256 / (N / 8) rows per
+// CTA, the post-processing split of rows_r2c_any.  Loads go straight from
+// global memory into the first pass's registers (a half-row run of 16-byte
+// values per group of lanes); the modes are written transposed, a run of the
+// CTA's rows per mode (128 to 1024 bytes).
 template <int N>
-__global__ void __launch_bounds__(kRegThreads) rows_c2r_reg(long nrows, int ld, const double2* __restrict__ tw_g,
+__global__ void __launch_bounds__(kRegThreads) rows_r2c_reg(long nrows, const double2* __restrict__ tw_g,
+                                                           const double2* __restrict__ wp_g,
+                                                           const double* __restrict__ src, double2* __restrict__ dst) {
+  constexpr int TPS = N / 8, SPC = kRegThreads / TPS, LD = N + 1;
+  __shared__ double2 tw[TwTab<N>::size], wp[N + 1];
+  __shared__ double2 buf[SPC * LD];
+  fill_tw<N>(tw, tw_g, threadIdx.x, kRegThreads);
+  for (int t = threadIdx.x; t <= N; t += kRegThreads) wp[t] = wp_g[t];
+  const int sq = threadIdx.x / TPS, tau = threadIdx.x % TPS;
+  const long row0 = (long)blockIdx.x * SPC, row = row0 + sq;
+  const bool ok = row < nrows;
+  const double2* s = (const double2*)src + row * N;
+  double2 v[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) v[r] = ok ? s[tau + r * TPS] : make_double2(0.0, 0.0);
+  __syncthreads();  // the tables
+  double2* seq = buf + sq * LD;
+  fft_reg<N>(v, seq, tau, tw, -1);
+  __syncwarp();
+  store_last<N>(v, seq, tau);
+  __syncthreads();
+  const int rr = threadIdx.x % SPC, k0 = threadIdx.x / SPC;
+  if (row0 + rr >= nrows) return;
+  const double2* q = buf + rr * LD;
+#pragma unroll
+  for (int i = 0; i <= 8; ++i) {
+    const int k = k0 + i * TPS;
+    if (k <= N) {
+      const double2 zk = q[swz(k & (N - 1))], zc = cconj(q[swz((N - k) & (N - 1))]);
+      const double2 e = make_double2(0.5 * (zk.x + zc.x), 0.5 * (zk.y + zc.y));
+      const double2 od = make_double2(0.5 * (zk.x - zc.x), 0.5 * (zk.y - zc.y));
+      const double2 wo = cmul(wp[k], od);
+      dst[(long)k * nrows + row0 + rr] = make_double2(e.x + wo.y, e.y - wo.x);
+    }
+  }
+}
+
+// Complex-to-real rows, the pre-processing of rows_c2r_any: the modes of the
+// CTA's rows come in transposed through shared memory (row pairs X_k,
+// X_{n-k}), the first pass's inputs are formed in registers, the last pass
+// writes the reals straight to global memory (16-byte runs, or pairs of
+// 8-byte values into a halo field).
+template <int N>
+__global__ void __launch_bounds__(kRegThreads) rows_c2r_reg(long nrows, const double2* __restrict__ tw_g,
                                                            const double2* __restrict__ wp_g,
                                                            const double2* __restrict__ src, double* __restrict__ dst,
                                                            RowsOut out) {
@@ -672,15 +842,18 @@ __global__ void __launch_bounds__(kRegThreads) rows_c2r_reg(long nrows, int ld, 
   fill_tw<N>(tw, tw_g, threadIdx.x, kRegThreads);
   for (int t = threadIdx.x; t <= N; t += kRegThreads) wp[t] = wp_g[t];
   const int sq = threadIdx.x / TPS, tau = threadIdx.x % TPS;
-  const long row = (long)blockIdx.x * SPC + sq;
+  const long row0 = (long)blockIdx.x * SPC, row = row0 + sq;
   const bool ok = row < nrows;
-  double2* seq = buf + sq * LD;  // first the row's N + 1 modes (linear), then the FFT slot
-  const double2* s = src + row * ld;
+  {
+    const int rr = threadIdx.x % SPC, k0 = threadIdx.x / SPC;
+    const bool in = row0 + rr < nrows;
 #pragma unroll
-  for (int i = 0; i <= 8; ++i) {
-    const int k = tau + i * TPS;
-    if (k <= N) seq[k] = ok ? s[k] : make_double2(0.0, 0.0);
+    for (int i = 0; i <= 8; ++i) {
+      const int k = k0 + i * TPS;
+      if (k <= N) buf[rr * LD + k] = in ? src[(long)k * nrows + row0 + rr] : make_double2(0.0, 0.0);
+    }
   }
+  double2* seq = buf + sq * LD;  // first the row's N + 1 modes (linear), then the FFT slot
   __syncthreads();  // the tables and the modes
   double2 v[8];
 #pragma unroll
@@ -714,64 +887,89 @@ __global__ void __launch_bounds__(kRegThreads) rows_c2r_reg(long nrows, int ld, 
   }
 }
 
-// Column transforms (length N = ny) of planes [nplanes][N][ld], ncols valid
-// columns: 256 / (N / 8) columns per CTA, loaded row by row (runs of
-// consecutive modes) into per-column slots of shared memory, transformed by
-// a lane group each, and written back the same way.
+// y transforms: contiguous sequences of length N in place, 256 / (N / 8) per
+// CTA, registers to registers
 template <int N>
-__global__ void __launch_bounds__(kRegThreads) cols_reg(int ncols, int ld, const double2* __restrict__ tw_g, int sign,
+__global__ void __launch_bounds__(kRegThreads) cols_reg(long nseq, const double2* __restrict__ tw_g, int sign,
                                                        double2* __restrict__ data) {
-  constexpr int TPS = N / 8, CB = kRegThreads / TPS, LD = N + 1, YS = kRegThreads / CB;
+  constexpr int TPS = N / 8, SPC = kRegThreads / TPS, LD = N + 1;
   __shared__ double2 tw[TwTab<N>::size];
-  __shared__ double2 buf[CB * LD];
+  __shared__ double2 buf[SPC * LD];
   fill_tw<N>(tw, tw_g, threadIdx.x, kRegThreads);
-  double2* plane = data + (long)blockIdx.y * N * ld;
-  const int c0 = blockIdx.x * CB;
-  {
-    const int c = threadIdx.x % CB, y0 = threadIdx.x / CB;
-    const bool in = c0 + c < ncols;
-#pragma unroll 4
-    for (int y = y0; y < N; y += YS) buf[c * LD + swz(y)] = in ? plane[(long)y * ld + c0 + c] : make_double2(0., 0.);
-  }
-  __syncthreads();
   const int sq = threadIdx.x / TPS, tau = threadIdx.x % TPS;
-  double2* seq = buf + sq * LD;
+  const long s = (long)blockIdx.x * SPC + sq;
+  const bool ok = s < nseq;
+  double2* d = data + s * N;
   double2 v[8];
-  load_pass<N, 8>(v, seq, tau);
-  fft_reg<N>(v, seq, tau, tw, sign);
-  __syncwarp();
-  store_last<N>(v, seq, tau);
+#pragma unroll
+  for (int r = 0; r < 8; ++r) v[r] = ok ? d[tau + r * TPS] : make_double2(0.0, 0.0);
   __syncthreads();
-  {
-    const int c = threadIdx.x % CB, y0 = threadIdx.x / CB;
-    if (c0 + c < ncols)
-#pragma unroll 4
-      for (int y = y0; y < N; y += YS) plane[(long)y * ld + c0 + c] = buf[c * LD + swz(y)];
-  }
-}
-
-// dense solution -> scaled halo field (the generic inverse rows' epilogue)
-__global__ void scatter_out_kernel(long n, int itot, const double* __restrict__ r, RowsOut out) {
-  const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  const long i = q % itot, row = q / itot, j = row % out.jtot, k = row / out.jtot;
-  out.f[(k + 1) * out.plane + (j + 1) * out.ldi + i + 1] = r[q] * out.scale;
+  fft_reg<N>(v, buf + sq * LD, tau, tw, sign);
+  if (!ok) return;
+  constexpr int R = LastPass<N>::R, NS = LastPass<N>::NS;
+#pragma unroll
+  for (int b = 0; b < 8 / R; ++b)
+#pragma unroll
+    for (int q = 0; q < R; ++q) d[out_pos<N, R, NS>(tau, b, q)] = v[b * R + q];
 }
 
 }  // namespace
 
 namespace {
 
-// radices of n (4s first, then the other primes up to kMaxRadix); false when
-// a prime factor is larger or there are too many factors
-bool factor(int n, FftPlan& P) {
-  P.n = n;
-  P.nf = 0;
+FastDiv fast_div(int d) { return FastDiv{(unsigned)d, (unsigned)((1ull << 32) / (unsigned)d) + 1u}; }
+
+// The fewest radices whose product is n, and among those the smallest largest
+// one; prime factors above 7 are passes of their own.
+void best_radices(int n, std::vector<int>& cur, std::vector<int>& best) {
+  static const int radices[] = {16, 15, 14, 12, 10, 9, 8, 7, 6, 5, 4, 3, 2};
+  if (n == 1) {
+    auto key = [](const std::vector<int>& v) { return v.empty() ? 0 : *std::max_element(v.begin(), v.end()); };
+    if (best.empty() || cur.size() < best.size() || (cur.size() == best.size() && key(cur) < key(best))) best = cur;
+    return;
+  }
+  if (!best.empty() && cur.size() + 1 > best.size()) return;
+  for (int r : radices)
+    if (n % r == 0 && (cur.empty() || r <= cur.back())) {
+      cur.push_back(r);
+      best_radices(n / r, cur, best);
+      cur.pop_back();
+    }
+}
+
+// passes of length n and their twiddles (appended to tw as (re, im) pairs);
+// false when a prime factor is above kMaxRadix or there are too many passes
+bool make_plan(int n, FftPlan& P, std::vector<double>& tw) {
+  std::vector<int> rad, primes;
   int m = n;
-  while (m % 4 == 0 && P.nf < kMaxFactors) { P.radix[P.nf++] = 4; m /= 4; }
-  for (int p = 2; p <= kMaxRadix && m > 1; ++p)
-    while (m % p == 0 && P.nf < kMaxFactors) { P.radix[P.nf++] = p; m /= p; }
-  return m == 1 && n >= 1;
+  for (int p = 11; p <= m; p += 2)
+    while (m % p == 0) {
+      if (p > kMaxRadix) return false;
+      primes.push_back(p);
+      m /= p;
+    }
+  std::vector<int> cur;
+  if (m > 1) best_radices(m, cur, rad);
+  rad.insert(rad.end(), primes.begin(), primes.end());
+  if ((int)rad.size() > kMaxPasses) return false;
+  P.n = n;
+  P.nf = (int)rad.size();
+  int ns = 1;
+  auto put = [&](double t) {  // exp(-2 pi i t)
+    tw.push_back(std::cos(2.0 * kPi * t));
+    tw.push_back(-std::sin(2.0 * kPi * t));
+  };
+  const int base = (int)(tw.size() / 2);
+  for (int f = 0; f < P.nf; ++f) {
+    const int p = rad[f];
+    P.pass[f] = FftPass{p, (int)(tw.size() / 2) - base, fast_div(n / p), fast_div(ns)};
+    for (int r = 1; r < p; ++r)
+      for (int k = 0; k < ns; ++k) put((double)(r * k) / (double)(ns * p));
+    if (p > 16 || p == 11 || p == 13)
+      for (int t = 0; t < p; ++t) put((double)t / (double)p);
+    ns *= p;
+  }
+  return true;
 }
 
 std::vector<double> twiddles(int n) {  // exp(-2 pi i t / n) as (re, im) pairs
@@ -783,41 +981,50 @@ std::vector<double> twiddles(int n) {  // exp(-2 pi i t / n) as (re, im) pairs
   return w;
 }
 
-}  // namespace
-
-namespace {
 bool pow2_fast(int n) { return n == 32 || n == 64 || n == 128 || n == 256; }
-int mode_stride(int itot) { return (itot / 2 + 1 + 7) / 8 * 8; }  // nxm rounded up to 8 slots (128 B)
+
+size_t tri_tile_smem(int kmax, int C) { return (sizeof(double2) + sizeof(double)) * (size_t)kmax * C; }
+
+// sequences per CTA of the mixed-radix row and column kernels: about 1280
+// values (two padded buffers: 46 KB, four CTAs of 128 threads on an SM)
+int any_rows(int n) { return std::max(1, std::min(16, 1280 / n)); }
+size_t any_smem(int n) { return sizeof(double2) * 2 * any_rows(n) * fld(n); }
+
+#define SG_POW2_DISPATCH(n, call) \
+  switch (n) {                    \
+    case 32: call(32); break;     \
+    case 64: call(64); break;     \
+    case 128: call(128); break;   \
+    default: call(256); break;    \
+  }
+
+struct Plans {
+  FftPlan x, y;
+};
+
 }  // namespace
 
 int poisson_setup(sg_ctx* c, unsigned types) {
   auto& s = c->pois;
   const sg_config& f = c->cfg;
-  const long nslots = (long)mode_stride(f.itot) * f.jtot;
+  const long nxm = f.itot / 2 + 1, nslots = nxm * f.jtot;
   void* p = nullptr;
-  if (s.ready) {
+  auto tables = [&]() -> int {
     for (int e = 0; e < 4; ++e)
       if ((types >> e & 1u) && !s.zt[e]) {
         SG_TRY(dalloc(c, p, sizeof(double) * nslots * f.ktot), "alloc");
         s.zt[e] = (double*)p;
-        SG_TRY(dalloc(c, p, sizeof(double) * nslots * f.ktot), "alloc");
-        s.dt[e] = (double*)p;
       }
     return SG_OK;
-  }
+  };
+  if (s.ready) return tables();
   if (f.itot % 2 != 0 || f.ktot < 4) return fail(c, SG_ERR_CONFIG, "solver1d here needs an even itot and ktot >= 4");
-  const long nreal = (long)f.itot * f.jtot * f.ktot, nxm = f.itot / 2 + 1;
+  const long nreal = (long)f.itot * f.jtot * f.ktot;
   SG_TRY(dalloc(c, p, sizeof(double) * nreal), "alloc");
   s.r = (double*)p;
   SG_TRY(dalloc(c, p, sizeof(double2) * nslots * f.ktot), "alloc");
   s.c = p;
-  for (int e = 0; e < 4; ++e)
-    if (types >> e & 1u) {
-      SG_TRY(dalloc(c, p, sizeof(double) * nslots * f.ktot), "alloc");
-      s.zt[e] = (double*)p;
-      SG_TRY(dalloc(c, p, sizeof(double) * nslots * f.ktot), "alloc");
-      s.dt[e] = (double*)p;
-    }
+  SG_RET(tables());
   // initsolver.f90:111-130: xrt(2m) = xrt(2m+1) = -4 dxi^2 sin(2m pi / (2 itot))^2, the
   // modes of a real transform in x; in y the complex modes j and jtot - j share yrt
   std::vector<double> tab(nxm + f.jtot);
@@ -831,28 +1038,32 @@ int poisson_setup(sg_ctx* c, unsigned types) {
   s.tab = (double*)p;
   SG_TRY(cudaMemcpy(s.tab, tab.data(), sizeof(double) * tab.size(), cudaMemcpyHostToDevice), "upload");
   // FFT plans: complex length itot/2 for the rows (real length itot), jtot
-  // for the columns; twiddle tables exp(-2 pi i t / n) and the row split's
-  // W^k = exp(-2 pi i k / itot), k <= itot/2
-  FftPlan px{}, py{};
-  if (!factor(f.itot / 2, px) || !factor(f.jtot, py) || f.itot / 2 > kFftSmemComplex || f.jtot > kFftSmemComplex)
+  // for the y transforms.  Tables, one after the other: the register
+  // transforms' exp(-2 pi i t / n) of both lengths, the row split's
+  // W^k = exp(-2 pi i k / itot), k <= itot/2, then the mixed-radix passes' own.
+  Plans pl{};
+  const int n = f.itot / 2;
+  std::vector<double> w = twiddles(n), wy = twiddles(f.jtot), wp(2 * (size_t)nxm), px, py;
+  if (n > kMaxLength || f.jtot > kMaxLength || !make_plan(n, pl.x, px) || !make_plan(f.jtot, pl.y, py))
     return fail(c, SG_ERR_CONFIG, "solver1d here needs itot/2 and jtot of at most 2048 whose prime factors are "
                                   "at most 61");
-  std::vector<double> w = twiddles(f.itot / 2), wy = twiddles(f.jtot), wp(2 * (size_t)nxm);
   for (long k = 0; k < nxm; ++k) {
     wp[2 * k] = std::cos(2.0 * kPi * k / f.itot);
     wp[2 * k + 1] = -std::sin(2.0 * kPi * k / f.itot);
   }
+  const size_t opx = w.size() / 2 + wy.size() / 2 + wp.size() / 2, opy = opx + px.size() / 2;
   w.insert(w.end(), wy.begin(), wy.end());
   w.insert(w.end(), wp.begin(), wp.end());
+  w.insert(w.end(), px.begin(), px.end());
+  w.insert(w.end(), py.begin(), py.end());
   SG_TRY(dalloc(c, p, sizeof(double) * w.size()), "alloc");
   SG_TRY(cudaMemcpy(p, w.data(), sizeof(double) * w.size(), cudaMemcpyHostToDevice), "upload");
   s.w = (double2*)p;
-  px.w = s.w;
-  py.w = s.w + f.itot / 2;
-  s.wpost = s.w + f.itot / 2 + f.jtot;
-  static_assert(sizeof(FftPlan) <= sizeof(s.plan_x), "plan storage");
-  std::memcpy(s.plan_x, &px, sizeof(px));
-  std::memcpy(s.plan_y, &py, sizeof(py));
+  pl.x.tw = s.w + opx;
+  pl.y.tw = s.w + opy;
+  s.wpost = s.w + n + f.jtot;
+  static_assert(sizeof(Plans) <= sizeof(s.plans), "plan storage");
+  std::memcpy(s.plans, &pl, sizeof(pl));
   s.ready = true;
   return SG_OK;
 }
@@ -862,74 +1073,58 @@ void poisson_free(sg_ctx* c) { (void)c; }
 namespace {
 
 template <int N>
-void launch_r2c(long nrows, int ld, const double2* tw, const double2* wp, const double* r, double2* m,
+void launch_r2c(long nrows, const double2* tw, const double2* wp, const double* r, double2* m, cudaStream_t st) {
+  constexpr int SPC = kRegThreads / (N / 8);
+  rows_r2c_reg<N><<<(unsigned)((nrows + SPC - 1) / SPC), kRegThreads, 0, st>>>(nrows, tw, wp, r, m);
+}
+template <int N>
+void launch_c2r(long nrows, const double2* tw, const double2* wp, const double2* m, double* r, const RowsOut& o,
                 cudaStream_t st) {
   constexpr int SPC = kRegThreads / (N / 8);
-  rows_r2c_reg<N><<<(unsigned)((nrows + SPC - 1) / SPC), kRegThreads, 0, st>>>(nrows, ld, tw, wp, r, m);
+  rows_c2r_reg<N><<<(unsigned)((nrows + SPC - 1) / SPC), kRegThreads, 0, st>>>(nrows, tw, wp, m, r, o);
 }
 template <int N>
-void launch_c2r(long nrows, int ld, const double2* tw, const double2* wp, const double2* m, double* r,
-                const RowsOut& o, cudaStream_t st) {
+void launch_cols(long nseq, const double2* tw, int sign, double2* m, cudaStream_t st) {
   constexpr int SPC = kRegThreads / (N / 8);
-  rows_c2r_reg<N><<<(unsigned)((nrows + SPC - 1) / SPC), kRegThreads, 0, st>>>(nrows, ld, tw, wp, m, r, o);
+  cols_reg<N><<<(unsigned)((nseq + SPC - 1) / SPC), kRegThreads, 0, st>>>(nseq, tw, sign, m);
 }
-template <int N>
-void launch_cols(int ncols, int ld, int planes, const double2* tw, int sign, double2* m, cudaStream_t st) {
-  constexpr int CB = kRegThreads / (N / 8);
-  cols_reg<N><<<dim3((unsigned)((ncols + CB - 1) / CB), (unsigned)planes), kRegThreads, 0, st>>>(ncols, ld, tw, sign,
-                                                                                                 m);
+
+template <int C>
+cudaError_t launch_tri_tile(int kmax, int jtot, int nxm, int e, double a, const double* zt, double2* c,
+                            cudaStream_t st) {
+  const size_t smem = tri_tile_smem(kmax, C);
+  cudaError_t err = smem_limit(tri_tile_kernel<C>, smem);
+  if (err != cudaSuccess) return err;
+  tri_tile_kernel<C><<<dim3((unsigned)((jtot + C - 1) / C), (unsigned)nxm), kTriThreads, smem, st>>>(kmax, jtot, e, a,
+                                                                                                   zt, c);
+  return cudaGetLastError();
 }
-#define SG_POW2_DISPATCH(n, call) \
-  switch (n) {                    \
-    case 32: call(32); break;     \
-    case 64: call(64); break;     \
-    case 128: call(128); break;   \
-    default: call(256); break;    \
-  }
+
+// The widest tile of which at least three fit an SM (runs of 256, 128 or 64
+// bytes); tiles of four columns as long as one fits, then global memory.
+cudaError_t launch_tri(int kmax, int jtot, int nxm, int e, double a, const double* zt, double2* c, cudaStream_t st) {
+  constexpr size_t third = 72 * 1024, most = 220 * 1024;
+  if (tri_tile_smem(kmax, 16) <= third) return launch_tri_tile<16>(kmax, jtot, nxm, e, a, zt, c, st);
+  if (tri_tile_smem(kmax, 8) <= third) return launch_tri_tile<8>(kmax, jtot, nxm, e, a, zt, c, st);
+  if (tri_tile_smem(kmax, 4) <= most) return launch_tri_tile<4>(kmax, jtot, nxm, e, a, zt, c, st);
+  tri_apply_kernel<<<(unsigned)((2L * nxm * jtot + 127) / 128), 128, 0, st>>>(kmax, jtot, nxm, e, a, zt, c);
+  return cudaGetLastError();
+}
 
 }  // namespace
 
 int poisson_solve(sg_ctx* c, double* r, int e, double shift, cudaStream_t st, const PoisOut* out) {
   auto& s = c->pois;
   const sg_config& f = c->cfg;
-  FftPlan px, py;
-  std::memcpy(&px, s.plan_x, sizeof(px));
-  std::memcpy(&py, s.plan_y, sizeof(py));
-  const int n = f.itot / 2, nxm = n + 1, ld = mode_stride(f.itot);
-  const long nrows = (long)f.jtot * f.ktot, nslots = (long)ld * f.jtot;
-  const bool rows_fast = pow2_fast(n), cols_fast = pow2_fast(f.jtot);
+  Plans pl;
+  std::memcpy(&pl, s.plans, sizeof(pl));
+  const int n = f.itot / 2, nxm = n + 1;
+  const long nrows = (long)f.jtot * f.ktot;
   const RowsOut ro{out ? out->f : nullptr, out ? out->ldi : 0, out ? out->plane : 0, out ? out->scale : 0.0, f.jtot};
-  // generic passes: rows per CTA in two (forward) or three (inverse) buffers
-  // of at most kFftSmemComplex values; columns per CTA likewise
-  const int rpc = std::max(1, kFftSmemComplex / n), cpc = std::max(1, kFftSmemComplex / f.jtot);
-  const size_t sm_f = sizeof(double2) * 2 * rpc * n, sm_i = sizeof(double2) * rpc * (2 * n + nxm);
-  const size_t sm_c = sizeof(double2) * 2 * cpc * (f.jtot + 1);
-  if (!rows_fast) {
-    SG_TRY(smem_limit(fft_rows_r2c, sm_f), "fft");
-    SG_TRY(smem_limit(fft_rows_c2r, sm_i), "fft");
-  }
-  if (!cols_fast) SG_TRY(smem_limit(fft_cols, sm_c), "fft");
-  const unsigned gr = (unsigned)((nrows + rpc - 1) / rpc);
-  const dim3 gc((unsigned)((nxm + cpc - 1) / cpc), (unsigned)f.ktot);
+  const double dzi = 1.0 / (f.lz / f.ktot);
   double2* modes = (double2*)s.c;
   const double2* twx = s.w;
   const double2* twy = s.w + n;
-#define SG_R2C(N) launch_r2c<N>(nrows, ld, twx, s.wpost, r, modes, st)
-#define SG_COLS_F(N) launch_cols<N>(nxm, ld, f.ktot, twy, -1, modes, st)
-#define SG_COLS_I(N) launch_cols<N>(nxm, ld, f.ktot, twy, +1, modes, st)
-#define SG_C2R(N) launch_c2r<N>(nrows, ld, twx, s.wpost, modes, r, ro, st)
-  if (rows_fast) {
-    SG_POW2_DISPATCH(n, SG_R2C)
-  } else {
-    fft_rows_r2c<<<gr, kFftThreads, sm_f, st>>>(nrows, rpc, ld, px, s.wpost, r, modes);
-  }
-  if (cols_fast) {
-    SG_POW2_DISPATCH(f.jtot, SG_COLS_F)
-  } else {
-    fft_cols<<<gc, kFftThreads, sm_c, st>>>(nxm, ld, cpc, py, -1, modes);
-  }
-  const double dzi = 1.0 / (f.lz / f.ktot);
-  const unsigned gt = (unsigned)((nslots + 127) / 128);
   int launches = 5;
   if (e < 0 || e > 3 || !s.zt[e]) return fail(c, SG_ERR_STATE, "solver1d: tables of this row type were not set up");
   if (!s.tvalid[e] || s.tshift[e] != shift) {
@@ -938,31 +1133,49 @@ int poisson_solve(sg_ctx* c, double* r, int e, double shift, cudaStream_t st, co
     // direct calls that may come before the graph's first launch
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     SG_TRY(cudaStreamIsCapturing(st, &cap), "solver1d");
-    tri_coeff_kernel<<<gt, 128, 0, st>>>(f.ktot, f.jtot, ld, nxm, e, dzi, shift, s.tab, s.tab + nxm, s.zt[e], s.dt[e]);
+    tri_coeff_kernel<<<(unsigned)((nxm * f.jtot + 127) / 128), 128, 0, st>>>(f.ktot, f.jtot, nxm, e, dzi, shift, s.tab,
+                                                                             s.tab + nxm, s.zt[e]);
     s.tvalid[e] = cap == cudaStreamCaptureStatusNone;
     s.tshift[e] = shift;
     launches += 1;
   }
-  tri_apply_kernel<<<gt, 128, 0, st>>>(f.ktot, f.jtot, ld, nxm, e, dzi, s.zt[e], s.dt[e], modes);
-  if (cols_fast) {
-    SG_POW2_DISPATCH(f.jtot, SG_COLS_I)
-  } else {
-    fft_cols<<<gc, kFftThreads, sm_c, st>>>(nxm, ld, cpc, py, +1, modes);
-  }
-  if (rows_fast) {
-    SG_POW2_DISPATCH(n, SG_C2R)
-  } else {
-    fft_rows_c2r<<<gr, kFftThreads, sm_i, st>>>(nrows, rpc, ld, px, s.wpost, modes, r);
-    if (out) {
-      const long nreal = nrows * f.itot;
-      scatter_out_kernel<<<(unsigned)((nreal + 255) / 256), 256, 0, st>>>(nreal, f.itot, r, ro);
-      launches += 1;
-    }
-  }
+  // x rows to modes
+  const int rx = any_rows(n);
+  const unsigned gx = (unsigned)((nrows + rx - 1) / rx);
+  if (pow2_fast(n)) {
+#define SG_R2C(N) launch_r2c<N>(nrows, twx, s.wpost, r, modes, st)
+    SG_POW2_DISPATCH(n, SG_R2C)
 #undef SG_R2C
-#undef SG_COLS_F
-#undef SG_COLS_I
+  } else {
+    SG_TRY(smem_limit(rows_r2c_any, any_smem(n)), "fft");
+    rows_r2c_any<<<gx, kAnyThreads, any_smem(n), st>>>(nrows, fast_div(rx), pl.x, s.wpost, r, modes);
+  }
+  // y transforms, elimination, inverse y transforms
+  const long nseq = (long)nxm * f.ktot;
+  const int ry = any_rows(f.jtot);
+  auto cols = [&](int sign) -> int {
+    if (pow2_fast(f.jtot)) {
+#define SG_COLS(N) launch_cols<N>(nseq, twy, sign, modes, st)
+      SG_POW2_DISPATCH(f.jtot, SG_COLS)
+#undef SG_COLS
+    } else {
+      SG_TRY(smem_limit(cols_any, any_smem(f.jtot)), "fft");
+      cols_any<<<(unsigned)((nseq + ry - 1) / ry), kAnyThreads, any_smem(f.jtot), st>>>(nseq, ry, pl.y, sign > 0, modes);
+    }
+    return SG_OK;
+  };
+  SG_RET(cols(-1));
+  SG_TRY(launch_tri(f.ktot, f.jtot, nxm, e, dzi * dzi, s.zt[e], modes, st), "solver1d");
+  SG_RET(cols(+1));
+  // modes to x rows
+  if (pow2_fast(n)) {
+#define SG_C2R(N) launch_c2r<N>(nrows, twx, s.wpost, modes, r, ro, st)
+    SG_POW2_DISPATCH(n, SG_C2R)
 #undef SG_C2R
+  } else {
+    SG_TRY(smem_limit(rows_c2r_any, any_smem(n)), "fft");
+    rows_c2r_any<<<gx, kAnyThreads, any_smem(n), st>>>(nrows, fast_div(rx), pl.x, s.wpost, modes, r, ro);
+  }
   SG_TRY(cudaGetLastError(), "solver1d");
   c->launches += launches;
   return SG_OK;
