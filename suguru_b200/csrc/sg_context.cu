@@ -898,7 +898,6 @@ void sg_destroy(sg_ctx* c) {
   if (c->st) cudaStreamSynchronize(c->st);
   if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
   if (c->graph) cudaGraphDestroy(c->graph);
-  poisson_free(c);
   for (void* p : c->allocs) cudaFree(p);
   for (int k = 0; k <= sg_ctx::kMarkStages; ++k)
     if (c->ev[k]) cudaEventDestroy(c->ev[k]);

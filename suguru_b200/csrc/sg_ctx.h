@@ -153,8 +153,9 @@ struct sg_ctx {
   // solver1d on the GPU (sg_poisson.cu), shared by the indicator and the flow solver
   struct PoissonState {
     bool ready = false;
-    double* r = nullptr;     // real FFT input / output [ktot][jtot][itot]
-    void* c = nullptr;       // modes [itot/2 + 1][ktot][jtot] (double2)
+    int nfields = 0;         // fields the arrays below hold (1: indicator alone, 4: flow solver)
+    double* r = nullptr;     // real FFT input / output [min(nfields, 3)][ktot][jtot][itot]
+    void* c = nullptr;       // modes [nfields][itot/2 + 1][ktot][jtot] (double2)
     // elimination pivots per row type e = 0..3 (sg_poisson.cu), laid out as
     // the modes, for the shift they were made with
     double* zt[4] = {nullptr, nullptr, nullptr, nullptr};
@@ -178,9 +179,6 @@ struct sg_ctx {
   struct FlowState {
     bool ready = false;
     double rep = 1, vb2 = 0, vt2 = 0;
-    double* ru = nullptr;    // right-hand sides of u and v, [ktot][jtot][itot]
-    double* rv = nullptr;
-    double* p = nullptr;     // pressure correction with halos
     void* stage[13] = {};    // device copies of the fields in host memory mode
   } flow;
 };
@@ -218,21 +216,20 @@ const int* sur_flags(sg_ctx* c);
 // force pipeline only, outputs into device arrays lag[0..6] (sg_context.cu)
 int run_forces_only(sg_ctx* c, const double* X, const double* Y, const double* Z, void* const* lag);
 
-// solver1d (sg_poisson.cu): FFT buffers and plans made once per context;
+// solver1d (sg_poisson.cu): FFT buffers and plans made once per context, for
+// `nfields` fields at once (1, or 4 for poisson_project).
 // poisson_solve replaces r ([ktot][jtot][itot], interior values) with
 // itot * jtot times the solution of the rows of initsolver(e) (shift = Rep/dt
-// for e = 2, 3): the FFT pair is left unnormalised.  With out, the solution
-// times out->scale goes to the interior of a field with a one-cell halo
-// instead (value (i, j, k), 0-based, at f[(k+1) plane + (j+1) ldi + i+1]),
-// and r is left holding intermediate values.
-struct PoisOut {
-  double* f;
-  long ldi, plane;
-  double scale;
-};
-int poisson_setup(sg_ctx* c, unsigned types);  // types: bit e for each row type e the caller solves
-void poisson_free(sg_ctx* c);
-int poisson_solve(sg_ctx* c, double* r, int e, double shift, cudaStream_t st, const PoisOut* out = nullptr);
+// for e = 2, 3): the FFT pair is left unnormalised.
+// poisson_project runs the flow step from its right-hand sides r3
+// ([3][ktot][jtot][itot]: u, v, w) on: the solves of w (initsolver(3)), u and
+// v (initsolver(2)), fillps, the solve after initsolver(1), correc, and p +=
+// the correction; u, v, w and p (fields with a one-cell halo) get their
+// halos as bounduvw (wall values vb2, vt2 of v) and boundp leave them.
+int poisson_setup(sg_ctx* c, unsigned types, int nfields);  // types: bit e for each row type e the caller solves
+int poisson_solve(sg_ctx* c, double* r, int e, double shift, cudaStream_t st);
+int poisson_project(sg_ctx* c, const double* r3, double dt, double shift, double* u, double* v, double* w, double* p,
+                    double vb2, double vt2, cudaStream_t st);
 // indicator function (sg_indicator.cu)
 int indicator_setup(sg_ctx* c, double visc0, double lambda, double thetainc, double ta, double rep);
 template <class T>

@@ -14,9 +14,8 @@
 //  correc (correc.f90): the velocity minus dt times the pressure gradient,
 //      bounduvw; pnew += p, boundp.
 //
-// One thread per cell; every field is (0:i1,0:j1,0:k1) with x fastest.  A
-// halo kernel computes each halo cell from the interior cell it copies, so
-// that it reads nothing another thread writes.
+// Two parts: the right-hand sides here, then everything from the solves to
+// the updated pressure in mode space (poisson_project, sg_poisson.cu).
 #include <cmath>
 
 #include "sg_common.cuh"
@@ -35,182 +34,125 @@ __device__ __forceinline__ long at(const FGrid& g, int i, int j, int k) {
   return (long)k * g.plane + (long)j * g.ldi + i;
 }
 
-// interior cell q (x fastest) -> (i, j, k), 1-based
-__device__ __forceinline__ void cell_of(const FGrid& g, long q, int& i, int& j, int& k) {
-  i = (int)(q % g.itot) + 1;
-  j = (int)((q / g.itot) % g.jtot) + 1;
-  k = (int)(q / ((long)g.itot * g.jtot)) + 1;
-}
-
-struct Flux {
-  double x, y, z;  // -p + m of each direction
-};
-
-// the face fluxes of momxad / momyad / momzad for component C at one level
-template <int C>
-__device__ __forceinline__ Flux fluxes(const FGrid& g, const double* __restrict__ U, const double* __restrict__ V,
-                                       const double* __restrict__ W, int i, int j, int k) {
-  const long o = at(g, i, j, k), ox = 1, oy = g.ldi, oz = g.plane;
-  double xp, xm, yp, ym, zp, zm;
-  if (C == 0) {
-    xp = 0.25 * (U[o + ox] + U[o]) * (U[o + ox] + U[o]);
-    xm = 0.25 * (U[o - ox] + U[o]) * (U[o - ox] + U[o]);
-    yp = 0.25 * (U[o + oy] + U[o]) * (V[o + ox] + V[o]);
-    ym = 0.25 * (U[o - oy] + U[o]) * (V[o + ox - oy] + V[o - oy]);
-    zp = 0.25 * (U[o + oz] + U[o]) * (W[o + ox] + W[o]);
-    zm = 0.25 * (U[o - oz] + U[o]) * (W[o + ox - oz] + W[o - oz]);
-  } else if (C == 1) {
-    xp = 0.25 * (U[o] + U[o + oy]) * (V[o] + V[o + ox]);
-    xm = 0.25 * (U[o - ox] + U[o - ox + oy]) * (V[o] + V[o - ox]);
-    yp = 0.25 * (V[o] + V[o + oy]) * (V[o] + V[o + oy]);
-    ym = 0.25 * (V[o] + V[o - oy]) * (V[o] + V[o - oy]);
-    zp = 0.25 * (W[o] + W[o + oy]) * (V[o + oz] + V[o]);
-    zm = 0.25 * (W[o - oz] + W[o - oz + oy]) * (V[o - oz] + V[o]);
-  } else {
-    xp = 0.25 * (W[o] + W[o + ox]) * (U[o] + U[o + oz]);
-    xm = 0.25 * (W[o] + W[o - ox]) * (U[o - ox] + U[o - ox + oz]);
-    yp = 0.25 * (W[o] + W[o + oy]) * (V[o] + V[o + oz]);
-    ym = 0.25 * (W[o] + W[o - oy]) * (V[o - oy] + V[o - oy + oz]);
-    zp = 0.25 * (W[o] + W[o + oz]) * (W[o] + W[o + oz]);
-    zm = 0.25 * (W[o] + W[o - oz]) * (W[o] + W[o - oz]);
-  }
-  return Flux{-xp + xm, -yp + ym, -zp + zm};
-}
-
 struct Fields {
-  const double *uo, *vo, *wo, *uoo, *voo, *woo, *p, *fx, *fy, *fz;
+  const double* f[7];   // u, v, w of level n, of level n-1, p
+  const double* fb[3];  // IB force
 };
 
 // fftuvw's right-hand sides of u, v and w into the solver's layout
-// [k-1][j-1][i-1], one thread per interior cell for all three (the stencils
-// share most of their loads)
-template <int C>
-__device__ __forceinline__ double momentum_rhs(const FGrid& g, const Fields& F, double dt, double rep, int i, int j,
-                                               int k) {
-  const long o = at(g, i, j, k);
-  const long step = C == 0 ? 1 : (C == 1 ? g.ldi : g.plane);
-  const double dd = C == 0 ? g.dxi : (C == 1 ? g.dyi : g.dzi);
-  const double* f = C == 0 ? F.fx : (C == 1 ? F.fy : F.fz);
-  const double* vo = C == 0 ? F.uo : (C == 1 ? F.vo : F.wo);
-  const double durk = (-dd * ((F.p[o + step] - F.p[o]))) + f[o];
-  const Flux a = fluxes<C>(g, F.uo, F.vo, F.wo, i, j, k);
-  const Flux b = fluxes<C>(g, F.uoo, F.voo, F.woo, i, j, k);
-  const double ad = g.dxi * ((1.5 * a.x) - (.5 * b.x)) + g.dyi * ((1.5 * a.y) - (.5 * b.y)) +
-                    g.dzi * ((1.5 * a.z) - (.5 * b.z));
-  double d = -durk;
-  d = d - ad;
-  d = d - (vo[o] / dt);
-  return d * rep;
-}
+// [field][k-1][j-1][i-1].
+//
+// The convection of the three components shares six products per grid point
+// and level: with the sums U_x = u(i) + u(i+1) and so on, the fluxes through
+// the faces between the point and its upper neighbours are (times 1/4)
+//   U_x U_x,  U_y V_x,  U_z W_x,  V_y V_y,  V_z W_y,  W_z W_z,
+// and every component's face flux is one of them, here or at the lower
+// neighbour.  A thread per point forms them for both levels, combined as
+// 1.5 (n) - 0.5 (n-1) at once, and takes the lower neighbours' in x and y
+// from shared memory and in z from its own previous step: about 80 FP64
+// operations a cell instead of 270 when each component's stencil was
+// evaluated by itself.  Blocks of 32 x 8 cells march up kMomZ levels, the
+// first step for the z fluxes below only; the threads hold the block's points
+// with one more column and row on either side, each loads its point of every
+// field once per level, one level ahead of its use, and the upper neighbours
+// in x and y come through shared memory too (loading them from global memory
+// kept 24 loads a cell in the way of the arithmetic: 250 us at
+// 256 x 256 x 128; the arrays' 870 MB take 134 us).
+constexpr int kMomX = 32, kMomY = 8, kMomZ = 16;
+constexpr int kMomW = kMomX + 2, kMomPts = kMomW * (kMomY + 2), kMomThreads = (kMomPts + 31) / 32 * 32;
 
-// Blocks of 32 x 8 cells in (x, y) that march up kMomZ consecutive z levels,
-// so that the stencil's y neighbours of a warp are mostly the block's own
-// loads and its z neighbours the block's loads of the levels just before
-// and after (L1), not L2's.
-constexpr int kMomZ = 8;
+constexpr int kMomRow = kMomPts + kMomW;  // slots per array, the last row's upper neighbours included
+constexpr size_t kMomSmem = sizeof(double) * 2 * (7 + 5) * kMomRow;
 
-__global__ void __launch_bounds__(256) momentum_rhs_kernel(FGrid g, Fields F, double dt, double rep,
-                                                           double* __restrict__ ru, double* __restrict__ rv,
-                                                           double* __restrict__ rw) {
-  const int nbx = (g.itot + 31) / 32;
-  const int i = (int)(blockIdx.x % nbx) * 32 + (int)(threadIdx.x & 31) + 1;
-  const int j = (int)(blockIdx.x / nbx) * 8 + (int)(threadIdx.x >> 5) + 1;
-  if (i > g.itot || j > g.jtot) return;
+__global__ void __launch_bounds__(kMomThreads, 2) momentum_rhs_kernel(FGrid g, Fields F, double dt, double rep,
+                                                                   double* __restrict__ r) {
+  // two levels of: the seven fields, then XX, XY, XZ, YY, YZ of the points
+  extern __shared__ __align__(16) double smom[];
+  const int nbx = (g.itot + kMomX - 1) / kMomX, t = threadIdx.x;
+  const int fx = t % kMomW, fy = t / kMomW;
+  const int i = (int)(blockIdx.x % nbx) * kMomX + fx, j = (int)(blockIdx.x / nbx) * kMomY + fy;
+  const bool cell = t < kMomPts && fx > 0 && fy > 0 && fx <= kMomX && fy <= kMomY && i <= g.itot && j <= g.jtot;
   const int k0 = (int)blockIdx.y * kMomZ + 1, k1 = min(k0 + kMomZ, g.ktot + 1);
-  for (int k = k0; k < k1; ++k) {
-    const long q = ((long)(k - 1) * g.jtot + (j - 1)) * g.itot + (i - 1);
-    ru[q] = momentum_rhs<0>(g, F, dt, rep, i, j, k);
-    rv[q] = momentum_rhs<1>(g, F, dt, rep, i, j, k);
-    rw[q] = k == g.ktot ? 0.0 : momentum_rhs<2>(g, F, dt, rep, i, j, k);  // dwdt(i,j,kmax) = 0 (fftuvw.f90:86-92)
-  }
-}
-
-// bounduvw (mode 0: u; 1: v with wall values vb2, vt2; 2: w) or boundp (mode
-// 3) on the cells outside the interior, from the rule of bound.f90:7-139 at
-// the interior column each copies.  One thread per halo cell: the two z
-// planes (all i, j), then the two y rows (k = 1..kmax, all i), then the two
-// x columns (k = 1..kmax, j = 1..jmax).  The w row kmax of the interior is
-// already zero: its right-hand side is zero and its row the identity.
-__global__ void halo_kernel(FGrid g, int mode, double vb2, double vt2, double* __restrict__ f) {
-  const long nz = 2L * g.ldi * g.ldj, ny = 2L * g.ldi * g.ktot, nx = 2L * g.jtot * g.ktot;
-  long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  int i, j, k;
-  if (q < nz) {
-    k = q < g.plane ? 0 : g.ktot + 1;
-    q %= g.plane;
-    j = (int)(q / g.ldi);
-    i = (int)(q % g.ldi);
-  } else if ((q -= nz) < ny) {
-    const long side = (long)g.ldi * g.ktot;
-    j = q < side ? 0 : g.jtot + 1;
-    q %= side;
-    k = 1 + (int)(q / g.ldi);
-    i = (int)(q % g.ldi);
-  } else if ((q -= ny) < nx) {
-    const long side = (long)g.jtot * g.ktot;
-    i = q < side ? 0 : g.itot + 1;
-    q %= side;
-    k = 1 + (int)(q / g.jtot);
-    j = 1 + (int)(q % g.jtot);
-  } else {
-    return;
-  }
-  const long o = at(g, i, j, k);
-  const int is = i == 0 ? g.itot : (i == g.itot + 1 ? 1 : i);
-  const int js = j == 0 ? g.jtot : (j == g.jtot + 1 ? 1 : j);
-  double v;
-  if (mode == 2 && k == g.ktot) {  // w(i,j,kmax) = 0 in the halos too
-    v = 0.0;
-  } else if (k >= 1 && k <= g.ktot) {
-    v = f[at(g, is, js, k)];
-  } else if (k == 0) {
-    const double f1 = f[at(g, is, js, 1)];
-    v = mode == 0 ? -f1 : (mode == 1 ? vb2 - f1 : (mode == 2 ? 0.0 : f1));
-  } else {
-    const double fk = f[at(g, is, js, g.ktot)];
-    v = mode == 0 ? -fk : (mode == 1 ? vt2 - fk : (mode == 2 ? f[at(g, is, js, g.ktot - 1)] : fk));
-  }
-  f[o] = v;
-}
-
-// fillps: the divergence of the predicted velocity over dt
-__global__ void fillps_kernel(FGrid g, double dti, const double* __restrict__ u, const double* __restrict__ v,
-                              const double* __restrict__ w, double* __restrict__ rhs) {
+  const int plane = (int)g.plane;  // a field has less than 2^31 values
+  int o = (int)at(g, min(i, g.itot + 1), min(j, g.jtot + 1), k0 - 1);
   const long n = (long)g.itot * g.jtot * g.ktot;
-  const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  int i, j, k;
-  cell_of(g, q, i, j, k);
-  const long o = at(g, i, j, k);
-  rhs[q] = ((w[o] - w[o - g.plane]) * (dti * g.dzi) + (v[o] - v[o - g.ldi]) * (dti * g.dyi)) +
-           (u[o] - u[o - 1]) * (dti * g.dxi);
+  double* q = r + ((long)(k0 - 1) * g.jtot + (j - 1)) * g.itot + (i - 1);
+  const double dti = 1.0 / dt;
+  double cur[7], nx[7], zprev[3] = {0.0, 0.0, 0.0};  // XZ, YZ, ZZ of the level below
+  double fo[3] = {0.0, 0.0, 0.0};
+  double part[3] = {0.0, 0.0, 0.0};  // the previous level's right-hand sides but for its lower neighbours' fluxes
+#pragma unroll
+  for (int c = 0; c < 7; ++c) {
+    cur[c] = F.f[c][o];
+    nx[c] = F.f[c][o + plane];
+  }
+  // the level's fluxes at the lower neighbours complete its right-hand sides
+  auto finish = [&](int k) {
+    const double* se = smom + (14 + 5 * (k & 1)) * kMomRow + t;
+    auto at = [&](int h, int d) { return se[h * kMomRow - d]; };
+    q[0] = (part[0] - (g.dxi * at(0, 1) + g.dyi * at(1, kMomW))) * rep;
+    q[n] = (part[1] - (g.dxi * at(1, 1) + g.dyi * at(3, kMomW))) * rep;
+    // dwdt(i,j,kmax) = 0 (fftuvw.f90:86-92)
+    q[2 * n] = k == g.ktot ? 0.0 : (part[2] - (g.dxi * at(2, 1) + g.dyi * at(4, kMomW))) * rep;
+    q += (long)g.jtot * g.itot;
+  };
+  for (int k = k0 - 1; k < k1; ++k) {
+    // the level after the next, and the next level's forces, ahead of their use
+    double nn[7], fn[3];
+    const bool more = k + 1 < k1;
+    o += plane;
+#pragma unroll
+    for (int c = 0; c < 7; ++c) nn[c] = more ? F.f[c][o + plane] : 0.0;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) fn[c] = more && cell ? F.fb[c][o] : 0.0;
+    double* s = smom + 7 * (k & 1) * kMomRow + t;
+    double* se = smom + (14 + 5 * (k & 1)) * kMomRow + t;
+    if (t < kMomPts)
+#pragma unroll
+      for (int c = 0; c < 7; ++c) s[c * kMomRow] = cur[c];
+    __syncthreads();  // this level's fields and the previous level's fluxes
+    if (cell && k > k0) finish(k - 1);
+    if (t < kMomPts) {
+      // XX, XY, XZ, YY, YZ, ZZ of both levels, 1/4 (1.5 (n) - 0.5 (n-1))
+      double e[6];
+#pragma unroll
+      for (int l = 0; l < 2; ++l) {
+        const int a = 3 * l, b = a + 1, c = a + 2;
+        const double ux = cur[a] + s[a * kMomRow + 1], uy = cur[a] + s[a * kMomRow + kMomW], uz = cur[a] + nx[a];
+        const double vx = cur[b] + s[b * kMomRow + 1], vy = cur[b] + s[b * kMomRow + kMomW], vz = cur[b] + nx[b];
+        const double wx = cur[c] + s[c * kMomRow + 1], wy = cur[c] + s[c * kMomRow + kMomW], wz = cur[c] + nx[c];
+        const double m[6] = {ux * ux, uy * vx, uz * wx, vy * vy, vz * wy, wz * wz};
+#pragma unroll
+        for (int h = 0; h < 6; ++h) e[h] = l == 0 ? 0.375 * m[h] : e[h] - 0.125 * m[h];
+      }
+#pragma unroll
+      for (int h = 0; h < 5; ++h) se[h * kMomRow] = e[h];
+      const double dp[3] = {s[6 * kMomRow + 1] - cur[6], s[6 * kMomRow + kMomW] - cur[6], nx[6] - cur[6]};
+      const double dd[3] = {g.dxi, g.dyi, g.dzi};
+      const double up[3] = {g.dxi * e[0] + g.dyi * e[1] + g.dzi * (e[2] - zprev[0]),
+                            g.dxi * e[1] + g.dyi * e[3] + g.dzi * (e[4] - zprev[1]),
+                            g.dxi * e[2] + g.dyi * e[4] + g.dzi * (e[5] - zprev[2])};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        double v = cur[c] * dti;
+        v = fma(fma(-v, dt, cur[c]), dti, v);  // cur / dt: the product and one residual correction
+        part[c] = dd[c] * dp[c] - fo[c] + up[c] - v;
+      }
+      zprev[0] = e[2];
+      zprev[1] = e[4];
+      zprev[2] = e[5];
+    }
+#pragma unroll
+    for (int c = 0; c < 7; ++c) {
+      cur[c] = nx[c];
+      nx[c] = nn[c];
+    }
+#pragma unroll
+    for (int c = 0; c < 3; ++c) fo[c] = fn[c];
+  }
+  __syncthreads();
+  if (cell) finish(k1 - 1);
 }
-
-// correc
-__global__ void correc_kernel(FGrid g, double dt, const double* __restrict__ p, double* __restrict__ u,
-                              double* __restrict__ v, double* __restrict__ w) {
-  const long n = (long)g.itot * g.jtot * g.ktot;
-  const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  int i, j, k;
-  cell_of(g, q, i, j, k);
-  const long o = at(g, i, j, k);
-  u[o] = u[o] - (dt * g.dxi) * (p[o + 1] - p[o]);
-  v[o] = v[o] - (dt * g.dyi) * (p[o + g.ldi] - p[o]);
-  w[o] = w[o] - (dt * g.dzi) * (p[o + g.plane] - p[o]);
-}
-
-__global__ void add_interior_kernel(FGrid g, const double* __restrict__ p, double* __restrict__ pn) {
-  const long n = (long)g.itot * g.jtot * g.ktot;
-  const long q = (long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (q >= n) return;
-  int i, j, k;
-  cell_of(g, q, i, j, k);
-  const long o = at(g, i, j, k);
-  pn[o] = pn[o] + p[o];
-}
-
-unsigned blocks(long n) { return (unsigned)((n + 255) / 256); }
 
 }  // namespace
 
@@ -218,17 +160,13 @@ int flow_setup(sg_ctx* c, double rep, double vb2, double vt2) {
   if (c->mixed) return fail(c, SG_ERR_CONFIG, "the flow solver runs on FP64 contexts");
   if (!(rep > 0.0) || !std::isfinite(rep) || !std::isfinite(vb2) || !std::isfinite(vt2))
     return fail(c, SG_ERR_ARG, "rep must be positive and finite, the wall values finite");
-  SG_RET(poisson_setup(c, (1u << 1) | (1u << 2) | (1u << 3)));
+  SG_RET(poisson_setup(c, (1u << 1) | (1u << 2) | (1u << 3), 4));
   auto& s = c->flow;
   s.rep = rep;
   s.vb2 = vb2;
   s.vt2 = vt2;
   if (s.ready) return SG_OK;
   const sg_config& f = c->cfg;
-  const long nreal = (long)f.itot * f.jtot * f.ktot;
-  SG_TRY(dalloc(c, s.ru, sizeof(double) * nreal), "alloc");
-  SG_TRY(dalloc(c, s.rv, sizeof(double) * nreal), "alloc");
-  SG_TRY(dalloc(c, s.p, sizeof(double) * c->nfield), "alloc");
   if (f.mem == SG_MEM_HOST)
     for (int q = 0; q < 13; ++q) SG_TRY(dalloc(c, s.stage[q], sizeof(double) * c->nfield), "alloc");
   s.ready = true;
@@ -244,36 +182,14 @@ int flow_run(sg_ctx* c, double dt, const double* uo, const double* vo, const dou
   const IBGrid& ib = c->grid;
   FGrid g{f.itot, f.jtot, f.ktot, ib.ldi, ib.ldj, (long)ib.ldi * ib.ldj, 1.0 / (f.lx / f.itot),
           1.0 / (f.ly / f.jtot), 1.0 / (f.lz / f.ktot)};
-  const long nreal = (long)f.itot * f.jtot * f.ktot, nf = c->nfield - nreal;  // halo cells
-  const double inv_n = 1.0 / ((double)f.itot * f.jtot), shift = s.rep / dt;
-  double* rw = c->pois.r;
-  Fields F{uo, vo, wo, uoo, voo, woo, p, fx, fy, fz};
-  // fftuvw: right-hand sides, then w (initsolver(3)) and u, v (initsolver(2))
-  const dim3 mgrid((unsigned)(((f.itot + 31) / 32) * ((f.jtot + 7) / 8)), (unsigned)((f.ktot + kMomZ - 1) / kMomZ));
-  momentum_rhs_kernel<<<mgrid, 256, 0, st>>>(g, F, dt, s.rep, s.ru, s.rv, rw);
+  const Fields F{{uo, vo, wo, uoo, voo, woo, p}, {fx, fy, fz}};
+  const dim3 mgrid((unsigned)(((f.itot + kMomX - 1) / kMomX) * ((f.jtot + kMomY - 1) / kMomY)),
+                   (unsigned)((f.ktot + kMomZ - 1) / kMomZ));
+  SG_TRY(smem_limit(momentum_rhs_kernel, kMomSmem), "momentum");
+  momentum_rhs_kernel<<<mgrid, kMomThreads, kMomSmem, st>>>(g, F, dt, s.rep, c->pois.r);
   SG_TRY(cudaGetLastError(), "momentum");
-  // each solution goes, times 1 / (itot jtot), straight into its field
-  const PoisOut ow{w, g.ldi, g.plane, inv_n}, ou{u, g.ldi, g.plane, inv_n}, ov{v, g.ldi, g.plane, inv_n},
-      op{s.p, g.ldi, g.plane, inv_n};
-  SG_RET(poisson_solve(c, rw, 3, shift, st, &ow));
-  SG_RET(poisson_solve(c, s.ru, 2, shift, st, &ou));
-  SG_RET(poisson_solve(c, s.rv, 2, shift, st, &ov));
-  halo_kernel<<<blocks(nf), 256, 0, st>>>(g, 0, s.vb2, s.vt2, u);
-  halo_kernel<<<blocks(nf), 256, 0, st>>>(g, 1, s.vb2, s.vt2, v);
-  halo_kernel<<<blocks(nf), 256, 0, st>>>(g, 2, s.vb2, s.vt2, w);
-  // projection: fillps, solver1d after initsolver(1), boundp, correc, bounduvw
-  fillps_kernel<<<blocks(nreal), 256, 0, st>>>(g, 1.0 / dt, u, v, w, rw);
-  SG_RET(poisson_solve(c, rw, 1, 0.0, st, &op));
-  halo_kernel<<<blocks(nf), 256, 0, st>>>(g, 3, 0.0, 0.0, s.p);
-  correc_kernel<<<blocks(nreal), 256, 0, st>>>(g, dt, s.p, u, v, w);
-  halo_kernel<<<blocks(nf), 256, 0, st>>>(g, 0, s.vb2, s.vt2, u);
-  halo_kernel<<<blocks(nf), 256, 0, st>>>(g, 1, s.vb2, s.vt2, v);
-  halo_kernel<<<blocks(nf), 256, 0, st>>>(g, 2, s.vb2, s.vt2, w);
-  // pnew += p, boundp
-  add_interior_kernel<<<blocks(nreal), 256, 0, st>>>(g, s.p, p);
-  halo_kernel<<<blocks(nf), 256, 0, st>>>(g, 3, 0.0, 0.0, p);
-  SG_TRY(cudaGetLastError(), "flow step");
-  c->launches += 12;
+  c->launches += 1;
+  SG_RET(poisson_project(c, c->pois.r, dt, s.rep / dt, u, v, w, p, s.vb2, s.vt2, st));
   return SG_OK;
 }
 

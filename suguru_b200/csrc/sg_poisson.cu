@@ -13,7 +13,12 @@
 // Modes lie [m][k][j] (x mode, level, y): the rows' kernels transpose as they
 // write and read (runs of the CTA's rows), so that the y transforms run on
 // contiguous sequences and the elimination on tiles of neighbouring columns.
-// A solve is five launches: rows_r2c, cols, tri_tile, cols, rows_c2r.
+// A solve is five launches: rows_r2c, cols, tri_tile, cols, rows_c2r.  The
+// flow step's four solves and its projection run together in mode space
+// (poisson_project): the three right-hand sides are transformed in one launch
+// per direction, tri_flow_tile solves u, v, w, takes their divergence, solves
+// the pressure correction and corrects the three on chip, and the inverse
+// rows write the fields with their halos.
 // (A cluster of eight CTAs holding one x mode's whole plane over distributed
 // shared memory, for cols, tri_tile, cols in one launch, moves a third of
 // the bytes but took 119 us against 89 us at 256 x 256 x 128: 33 clusters
@@ -34,7 +39,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <type_traits>
 #include <vector>
 
 #include "sg_common.cuh"
@@ -117,124 +121,194 @@ __global__ void __launch_bounds__(128) tri_coeff_kernel(int kmax, int jtot, int 
   zm[(long)(kmax - 1) * jtot] = __dsub_rn(bb, __dmul_rn(r.a, dk));
 }
 
-template <int V>
-using Const = std::integral_constant<int, V>;
+__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
+  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
+}
+__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
+__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
+__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
+__device__ __forceinline__ double2 cswap(double2 a) { return make_double2(a.y, a.x); }
 
-// The two sweeps of one real column (the real or the imaginary parts of a
-// mode's levels: the elimination's coefficients are real) at c[k cs], its
-// pivots at z[k zs]; a = dzi^2 is both a_k (k = 1 .. kmax-2) and c_k.  Bound
-// by the chain from level to level, so each sweep is one fused multiply-add
-// per level on it (8 cycles; the products r_k z_k and a z_k are off it) and
-// runs in blocks of B levels without branches, the next block's loads ahead
-// of the block's arithmetic.  (The three dependent operations of the
-// unfused form with a guarded load per level took 97 cycles a level.)
-// cs, zs: the strides, as constants (tri_tile_kernel) or values.
-template <int B, class SC, class SZ>
-__device__ __forceinline__ void tri_sweeps(double* c, const double* z, SC cs, SZ zs, int kmax, int e, double a) {
-  const int last = kmax - 1;
-  double r[B], w[B], rn[B], wn[B];
-#pragma unroll
-  for (int t = 0; t < B; ++t) {
-    const int k = min(1 + t, last);
-    r[t] = c[k * cs];
-    w[t] = z[k * zs];
+// x / d for x < 2^16 and 1 <= d <= 2^15 as a multiplication: m = floor(2^32 / d) + 1.
+struct FastDiv {
+  unsigned d, m;
+};
+__device__ __forceinline__ int fdiv_u(int x, FastDiv f) { return f.d == 1 ? x : (int)__umulhi((unsigned)x, f.m); }
+
+// A tile of C neighbouring columns of one x mode in shared memory, and the
+// elimination on it.  The sweeps are first-order recurrences
+//   q_k = al_k q_{k-1} + z_k r_k,  x_k = q_k + al_k x_{k+1},  al_k = -a z_k
+// (a = dzi^2 is both a_k, k >= 1, and c_k), the same for the real and the
+// imaginary parts.  A chain of all levels takes 34 cycles a level, 8,700 for
+// 128 levels up and down, with two warps busy; so the levels are cut into
+// eight segments, and a warp sweeps four real columns, lane = 4 segment +
+// column: from a zero start for the segment's end value and the product of
+// its al, which shuffles compose into the true starts, then from those.
+// |al| <= 1, so the composition loses nothing.  Rows of a segment are shifted
+// by 32 bytes per segment (pivots: 16), so that the warp's lanes fall on
+// different banks.
+constexpr int kSegs = 8;
+
+template <int C>
+struct Tile {
+  FastDiv len;  // levels per segment
+  __device__ __forceinline__ int at(int k, int jl) const { return k * C + jl + 2 * fdiv_u(k, len); }
+};
+__host__ __device__ constexpr int tile_size(int kmax, int C) { return kmax * C + 2 * kSegs; }
+
+// Columns 4 col4 .. 4 col4 + 3 of the tile's 2 C real ones; whole warps.
+template <int C>
+__device__ __forceinline__ void tri_tile_sweeps(double2* tile, const double* zs, int col4, int kmax, int len, int e,
+                                                double a) {
+  const int lane = threadIdx.x & 31, seg = lane >> 2, cl = lane & 3, col = 4 * col4 + cl;
+  const int k0 = seg * len, n = min(len, kmax - k0), nu = min(n, kmax - 1 - k0);
+  double* c = (double*)(tile + k0 * C + 2 * seg) + col;
+  const double* z = zs + k0 * C + 2 * seg + (col >> 1);
+  double f = 1.0, p = 0.0, in = 0.0;
+#pragma unroll 4
+  for (int t = 0; t < nu; ++t) {
+    const double w = z[t * C], al = -(a * w);
+    p = fma(al, p, c[2 * t * C] * w);
+    f *= al;
   }
-  double p = c[0] * z[0];
-  c[0] = p;
+  __syncwarp();
+#pragma unroll
+  for (int t = 0; t < kSegs - 1; ++t) {
+    const double ft = __shfl_sync(0xffffffffu, f, 4 * t + cl), pt = __shfl_sync(0xffffffffu, p, 4 * t + cl);
+    if (t < seg) in = fma(ft, in, pt);
+  }
+  p = in;
+#pragma unroll 4
+  for (int t = 0; t < nu; ++t) {
+    const double w = z[t * C];
+    p = fma(-(a * w), p, c[2 * t * C] * w);
+    c[2 * t * C] = p;
+  }
+  if (n > 0 && k0 + n == kmax) {  // the top row: its pivot itself is tabulated; e = 3: the identity row of w
+    const double w = z[nu * C];
+    c[2 * nu * C] = w != 0.0 ? fma(e == 3 ? 0.0 : -a, p, c[2 * nu * C]) / w : 0.0;
+  }
+  f = 1.0;
+  p = 0.0;
+#pragma unroll 4
+  for (int t = n - 1; t >= 0; --t) {  // (the top row's al only meets zeros)
+    const double al = -(a * z[t * C]);
+    p = fma(al, p, c[2 * t * C]);
+    f *= al;
+  }
+  __syncwarp();
+  in = 0.0;
+#pragma unroll
+  for (int t = kSegs - 1; t > 0; --t) {
+    const double ft = __shfl_sync(0xffffffffu, f, 4 * t + cl), pt = __shfl_sync(0xffffffffu, p, 4 * t + cl);
+    if (t > seg) in = fma(ft, in, pt);
+  }
+  p = in;
+#pragma unroll 4
+  for (int t = n - 1; t >= 0; --t) {
+    p = fma(-(a * z[t * C]), p, c[2 * t * C]);
+    c[2 * t * C] = p;
+  }
+}
+
+// C columns, all levels, per CTA: copied to shared memory with their pivots,
+// solved there, written back; each mode is read and written once.  Memory-
+// bound (24 bytes in and 16 out per mode, 176 MB at 256 x 256 x 128); runs of
+// 256 bytes (C = 16) beat 128 and 64.
+template <int C>
+__global__ void __launch_bounds__(16 * C) tri_tile_kernel(int kmax, int jtot, FastDiv len, int e, double a,
+                                                          const double* __restrict__ zt, double2* __restrict__ c) {
+  extern __shared__ __align__(16) double2 tsm[];  // modes, then pivots
+  const Tile<C> T{len};
+  double* zs = (double*)(tsm + tile_size(kmax, C));
+  const int j0 = blockIdx.x * C, nj = min(C, jtot - j0);
+  const long o = (long)blockIdx.y * kmax * jtot + j0;
+  const int jl = threadIdx.x % C, k0 = threadIdx.x / C;
+  if (jl < nj)
+    for (int k = k0; k < kmax; k += 16) {
+      stage_async(&tsm[T.at(k, jl)], &c[o + (long)k * jtot + jl]);
+      stage_async(&zs[T.at(k, jl)], &zt[o + (long)k * jtot + jl]);
+    }
+  stage_wait();
+  __syncthreads();
+  tri_tile_sweeps<C>(tsm, zs, threadIdx.x >> 5, kmax, len.d, e, a);
+  __syncthreads();
+  if (jl < nj)
+    for (int k = k0; k < kmax; k += 16) c[o + (long)k * jtot + jl] = tsm[T.at(k, jl)];
+}
+
+// The two sweeps of one real column in global memory, at c[k cs] with its
+// pivots at z[k zs], in blocks of B levels, the next block's loads ahead of
+// the block's arithmetic in the other of two register sets.
+template <int B>
+__device__ __forceinline__ void tri_sweeps(double* c, const double* z, long cs, long zs, int kmax, int e, double a) {
+  const int last = kmax - 1, nb = (last - 1) / B;  // full blocks of rows 1 .. last - 1
+  double r0[B], w0[B], r1[B], w1[B], p;
+  auto load = [&](double(&r)[B], double(&w)[B], int k, int dir) {
+    const double *ck = c + k * cs, *zk = z + k * zs;
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+      r[t] = ck[dir * t * cs];
+      w[t] = zk[dir * t * zs];
+    }
+  };
+  auto up = [&](const double(&r)[B], const double(&w)[B], int k) {
+    double* ck = c + k * cs;
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+      p = fma(-(a * w[t]), p, r[t] * w[t]);
+      ck[t * cs] = p;
+    }
+  };
+  auto down = [&](const double(&r)[B], const double(&w)[B], int k) {
+    double* ck = c + k * cs;
+#pragma unroll
+    for (int t = 0; t < B; ++t) {
+      p = fma(-(a * w[t]), p, r[t]);
+      ck[-t * cs] = p;
+    }
+  };
   int k = 1;
-  for (; k + B <= last; k += B) {
-#pragma unroll
-    for (int t = 0; t < B; ++t) {
-      const int q = min(k + B + t, last);
-      rn[t] = c[q * cs];
-      wn[t] = z[q * zs];
-    }
-#pragma unroll
-    for (int t = 0; t < B; ++t) {
-      p = fma(-(a * w[t]), p, r[t] * w[t]);
-      c[(k + t) * cs] = p;
-    }
-#pragma unroll
-    for (int t = 0; t < B; ++t) {
-      r[t] = rn[t];
-      w[t] = wn[t];
+  if (nb > 0) load(r0, w0, k, 1);
+  p = c[0] * z[0];
+  c[0] = p;
+  for (int b = 0; b < nb; b += 2) {
+    if (b + 1 < nb) load(r1, w1, k + B, 1);
+    up(r0, w0, k);
+    k += B;
+    if (b + 1 < nb) {
+      if (b + 2 < nb) load(r0, w0, k + B, 1);
+      up(r1, w1, k);
+      k += B;
     }
   }
-#pragma unroll
-  for (int t = 0; t < B; ++t)
-    if (k + t < last) {
-      p = fma(-(a * w[t]), p, r[t] * w[t]);
-      c[(k + t) * cs] = p;
-    }
+  for (; k < last; ++k) {
+    const double w = z[k * zs];
+    p = fma(-(a * w), p, c[k * cs] * w);
+    c[k * cs] = p;
+  }
   {
     const double zk = z[last * zs], al = e == 3 ? 0.0 : a;  // e = 3: the identity row of w at the top
     p = zk != 0.0 ? fma(-al, p, c[last * cs]) / zk : 0.0;
     c[last * cs] = p;
   }
-#pragma unroll
-  for (int t = 0; t < B; ++t) {
-    const int q = max(last - 1 - t, 0);
-    r[t] = c[q * cs];
-    w[t] = z[q * zs];
-  }
   k = last - 1;
-  for (; k - B >= -1; k -= B) {
-#pragma unroll
-    for (int t = 0; t < B; ++t) {
-      const int q = max(k - B - t, 0);
-      rn[t] = c[q * cs];
-      wn[t] = z[q * zs];
-    }
-#pragma unroll
-    for (int t = 0; t < B; ++t) {
-      p = fma(-(a * w[t]), p, r[t]);
-      c[(k - t) * cs] = p;
-    }
-#pragma unroll
-    for (int t = 0; t < B; ++t) {
-      r[t] = rn[t];
-      w[t] = wn[t];
+  for (int t = (last - 1) - nb * B; t > 0; --t, --k) {
+    p = fma(-(a * z[k * zs]), p, c[k * cs]);
+    c[k * cs] = p;
+  }
+  if (nb > 0) load(r0, w0, k, -1);
+  for (int b = 0; b < nb; b += 2) {
+    if (b + 1 < nb) load(r1, w1, k - B, -1);
+    down(r0, w0, k);
+    k -= B;
+    if (b + 1 < nb) {
+      if (b + 2 < nb) load(r0, w0, k - B, -1);
+      down(r1, w1, k);
+      k -= B;
     }
   }
-#pragma unroll
-  for (int t = 0; t < B; ++t)
-    if (k - t >= 0) {
-      p = fma(-(a * w[t]), p, r[t]);
-      c[(k - t) * cs] = p;
-    }
-}
-
-// C neighbouring columns of one x mode, all levels, per CTA: copied to shared
-// memory with their pivots, swept there by 2 C threads (real and imaginary
-// parts), written back: each mode is read and written once.  Bound by memory
-// (24 bytes in and 16 out per mode) with the sweeps' latency hidden by the
-// other CTAs on the SM: at 256 x 256 x 128, 40 us with C = 16 (4.4 TB/s)
-// against 46 us with C = 8, 69 us with C = 4 (short runs) and 41 us with
-// C = 32 (fewer CTAs); a thread per column on global memory with a register
-// ring, which stores and reloads the forward values, took 80 us.
-constexpr int kTriThreads = 64;
-
-template <int C>
-__global__ void __launch_bounds__(kTriThreads) tri_tile_kernel(int kmax, int jtot, int e, double a,
-                                                               const double* __restrict__ zt,
-                                                               double2* __restrict__ c) {
-  extern __shared__ __align__(16) double2 tsm[];  // [kmax][C] modes, then [kmax][C] pivots
-  double* zs = (double*)(tsm + kmax * C);
-  const int j0 = blockIdx.x * C, nj = min(C, jtot - j0);
-  const long o = (long)blockIdx.y * kmax * jtot + j0;
-  const int jl = threadIdx.x % C, k0 = threadIdx.x / C;
-  if (jl < nj)
-    for (int k = k0; k < kmax; k += kTriThreads / C) {
-      stage_async(&tsm[k * C + jl], &c[o + (long)k * jtot + jl]);
-      stage_async(&zs[k * C + jl], &zt[o + (long)k * jtot + jl]);
-    }
-  stage_wait();
-  __syncthreads();
-  if (threadIdx.x < 2 * nj)
-    tri_sweeps<8>((double*)tsm + threadIdx.x, zs + (threadIdx.x >> 1), Const<2 * C>{}, Const<C>{}, kmax, e, a);
-  __syncthreads();
-  if (jl < nj)
-    for (int k = k0; k < kmax; k += kTriThreads / C) c[o + (long)k * jtot + jl] = tsm[k * C + jl];
+  c[0] = fma(-(a * z[0]), p, c[0]);
 }
 
 // Columns too long for a tile in shared memory: a thread per real column of
@@ -248,18 +322,113 @@ __global__ void __launch_bounds__(128) tri_apply_kernel(int kmax, int jtot, int 
   tri_sweeps<16>((double*)(c + o) + part, zt + o, 2L * jtot, (long)jtot, kmax, e, a);
 }
 
+// The flow step's solves and projection for C columns of one x mode, all
+// levels: u and v (e = 2), w (e = 3), the divergence over dt (fillps), the
+// pressure correction (e = 1) and the corrected velocities (correc), on the
+// modes in shared memory.  A difference along x or y is a factor per mode,
+// with ex = exp(-2 pi i m / itot) and ey = exp(-2 pi i j / jtot):
+//   u(i) - u(i-1) -> (1 - ex) u,   p(i+1) - p(i) -> (conj(ex) - 1) p;
+// w(0) = 0 in the divergence, and the top row of w, zero, takes no
+// correction (p(k1) = p(kmax)).  Memory-bound (72 bytes in and 64 out per
+// mode, 590 MB at 256 x 256 x 128); in physical space the same steps moved
+// the modes of all four fields twice more, and u, v, w and p once each
+// through fillps and correc.
+struct FlowModes {
+  double2 *u, *v, *w, *p;                      // [m][k][j]
+  const double *z2, *z3, *z1;                  // pivots of e = 2, 3, 1
+  const double2 *ex, *ey;
+  double sx, sy, sz;                           // dxi / dt, dyi / dt, dzi / dt
+  double gx, gy, gz;                           // dt dxi, dt dyi, dt dzi
+};
+
+__device__ __forceinline__ double2 mode_divergence(const FlowModes& F, double2 dx, double2 dy, double2 u, double2 v,
+                                                   double2 w, double2 wl) {
+  const double2 a = cmul(dx, u), b = cmul(dy, v);
+  return make_double2((w.x - wl.x) * F.sz + b.x * F.sy + a.x * F.sx, (w.y - wl.y) * F.sz + b.y * F.sy + a.y * F.sx);
+}
+
+// u -= dt dxi (conj(ex) - 1) p, with dx = 1 - ex: conj(ex) - 1 = -conj(dx)
+__device__ __forceinline__ double2 mode_corrected(double2 u, double2 dx, double2 p, double g) {
+  const double2 q = cmul(cconj(dx), p);
+  return make_double2(u.x + g * q.x, u.y + g * q.y);
+}
+
+template <int C>
+__global__ void __launch_bounds__(48 * C) tri_flow_tile_kernel(int kmax, int jtot, FastDiv len, double a, FlowModes F) {
+  extern __shared__ __align__(16) double2 tsm[];  // u, v, w, then the pivots z2, z3, z1
+  const Tile<C> T{len};
+  const int n = tile_size(kmax, C);
+  double2 *su = tsm, *sv = su + n, *sw = sv + n;
+  double *z2 = (double*)(sw + n), *z3 = z2 + n, *z1 = z3 + n;
+  double2* sp = (double2*)z2;  // the pressure correction takes the place of z2, z3 after their use
+  const int j0 = blockIdx.x * C, nj = min(C, jtot - j0), m = blockIdx.y;
+  const long o = (long)m * kmax * jtot + j0;
+  const int jl = threadIdx.x % C, k0 = threadIdx.x / C, warp = threadIdx.x >> 5;
+  if (jl < nj)
+    for (int k = k0; k < kmax; k += 48) {
+      const int q = T.at(k, jl);
+      const long g = o + (long)k * jtot + jl;
+      stage_async(&su[q], &F.u[g]);
+      stage_async(&sv[q], &F.v[g]);
+      stage_async(&sw[q], &F.w[g]);
+      stage_async(&z2[q], &F.z2[g]);
+      stage_async(&z3[q], &F.z3[g]);
+      stage_async(&z1[q], &F.z1[g]);
+    }
+  stage_wait();
+  __syncthreads();
+  {  // C / 2 warps for each of u, v, w
+    const int f = warp / (C / 2), c4 = warp - f * (C / 2);
+    tri_tile_sweeps<C>(f == 0 ? su : f == 1 ? sv : sw, f == 2 ? z3 : z2, c4, kmax, len.d, f == 2 ? 3 : 2, a);
+  }
+  __syncthreads();
+  const double2 ex = F.ex[m], ey = F.ey[min(j0 + jl, jtot - 1)];
+  const double2 dx = make_double2(1.0 - ex.x, -ex.y), dy = make_double2(1.0 - ey.x, -ey.y);
+  if (jl < nj)
+    for (int k = k0; k < kmax; k += 48) {
+      const int q = T.at(k, jl);
+      sp[q] = mode_divergence(F, dx, dy, su[q], sv[q], sw[q], k ? sw[T.at(k - 1, jl)] : make_double2(0.0, 0.0));
+    }
+  __syncthreads();
+  if (warp < C / 2) tri_tile_sweeps<C>(sp, z1, warp, kmax, len.d, 1, a);
+  __syncthreads();
+  if (jl < nj)
+    for (int k = k0; k < kmax; k += 48) {
+      const int q = T.at(k, jl);
+      const long g = o + (long)k * jtot + jl;
+      const double2 p = sp[q], pu = k + 1 < kmax ? sp[T.at(k + 1, jl)] : p;
+      F.u[g] = mode_corrected(su[q], dx, p, F.gx);
+      F.v[g] = mode_corrected(sv[q], dy, p, F.gy);
+      F.w[g] = make_double2(sw[q].x - F.gz * (pu.x - p.x), sw[q].y - F.gz * (pu.y - p.y));
+      F.p[g] = p;
+    }
+}
+
+// The same on global memory, for columns too long for a tile: the divergence
+// of the solved velocities, and after the pressure solve their correction
+__global__ void mode_divergence_kernel(int kmax, int jtot, long n, FlowModes F) {
+  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= n) return;
+  const int j = (int)(g % jtot), k = (int)(g / jtot % kmax), m = (int)(g / ((long)jtot * kmax));
+  const double2 ex = F.ex[m], ey = F.ey[j];
+  F.p[g] = mode_divergence(F, make_double2(1.0 - ex.x, -ex.y), make_double2(1.0 - ey.x, -ey.y), F.u[g], F.v[g], F.w[g],
+                           k ? F.w[g - jtot] : make_double2(0.0, 0.0));
+}
+__global__ void mode_correct_kernel(int kmax, int jtot, long n, FlowModes F) {
+  const long g = (long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (g >= n) return;
+  const int j = (int)(g % jtot), k = (int)(g / jtot % kmax), m = (int)(g / ((long)jtot * kmax));
+  const double2 ex = F.ex[m], ey = F.ey[j], p = F.p[g], pu = k + 1 < kmax ? F.p[g + jtot] : p;
+  F.u[g] = mode_corrected(F.u[g], make_double2(1.0 - ex.x, -ex.y), p, F.gx);
+  F.v[g] = mode_corrected(F.v[g], make_double2(1.0 - ey.x, -ey.y), p, F.gy);
+  const double2 w = F.w[g];
+  F.w[g] = make_double2(w.x - F.gz * (pu.x - p.x), w.y - F.gz * (pu.y - p.y));
+}
+
 // ---------------------------------------------------------------- FFT ---
 constexpr int kMaxRadix = 61;
 constexpr int kMaxPasses = 8;
 constexpr int kMaxLength = 2048;
-
-__device__ __forceinline__ double2 cmul(double2 a, double2 b) {
-  return make_double2(a.x * b.x - a.y * b.y, a.x * b.y + a.y * b.x);
-}
-__device__ __forceinline__ double2 cconj(double2 a) { return make_double2(a.x, -a.y); }
-__device__ __forceinline__ double2 cadd(double2 a, double2 b) { return make_double2(a.x + b.x, a.y + b.y); }
-__device__ __forceinline__ double2 csub(double2 a, double2 b) { return make_double2(a.x - b.x, a.y - b.y); }
-__device__ __forceinline__ double2 cswap(double2 a) { return make_double2(a.y, a.x); }
 
 // ------------------------------------------------- power-of-two FFTs ---
 // Lengths N = 32, 64, 128, 256: a sequence belongs to TPS = N/8 consecutive
@@ -454,12 +623,6 @@ __device__ __forceinline__ void store_last(const double2 (&v)[8], double2* seq, 
 // per prime factor spent its time in shared memory and in barriers (a 150-
 // point transform had four).  Forward transforms only: an inverse transform
 // swaps the real and imaginary parts of its input and of its output.
-//
-// x / d for x < 2^16 and 1 <= d <= 2^15 as a multiplication: m = floor(2^32 / d) + 1.
-struct FastDiv {
-  unsigned d, m;
-};
-__device__ __forceinline__ int fdiv_u(int x, FastDiv f) { return f.d == 1 ? x : (int)__umulhi((unsigned)x, f.m); }
 
 // Pass of radix p after sub-transforms of length ns: np = n / p butterflies;
 // its twiddles tw[off + (r-1) ns + k] = exp(-2 pi i r k / (ns p)).
@@ -674,13 +837,70 @@ __device__ __forceinline__ double2* fft_any(double2* b0, double2* b1, int nb, in
 }
 
 // Where the inverse rows put the solution: dense (f == nullptr: into the
-// transform's own real array), or scaled into the interior of a field with a
-// one-cell halo, value (i, j, k) (0-based) at f[(k+1) plane + (j+1) ldi + i+1].
+// transform's own real array), or scaled into a field with a one-cell halo,
+// halo cells included: the periodic images in x and y, and the wall planes by
+// bounduvw's and boundp's rules (bound.f90:7-139).
 struct RowsOut {
   double* f;
   long ldi, plane;
-  double scale;
-  int jtot;
+  double scale, lo, hi;  // wall values: f(0) = lo - f(1), f(k1) = hi - f(kmax) (u, v)
+  int itot, jtot, ktot;
+  int kind;              // 0: u or v; 1: w (zero at the bottom, f(k1) = f(kmax-1)); 2: pressure, added to f
+};
+struct RowsOuts {
+  RowsOut o[4];
+};
+
+// Row (j, k) (0-based) of a field and the rows it is copied to: its periodic
+// image in y, and beside a wall the halo plane's row and that row's image.
+// Consecutive lanes put consecutive cells (a thread that stored its own pairs
+// of cells filled half of each sector it touched: 161 against 127 us for the
+// four fields of a flow step at 256 x 256 x 128).
+struct RowTarget {
+  double *f, *img, *wall, *wall_img;
+  double scale, wa, wc;  // wall value: wc + wa x
+  int nx;
+  bool add;
+  __device__ __forceinline__ RowTarget(const RowsOut& o, int j, int k) {
+    const int jh = j == 0 ? o.jtot + 1 : (j == o.jtot - 1 ? 0 : -1);
+    int kh = -1;
+    wa = 1.0;
+    wc = 0.0;
+    if (o.kind == 1) {
+      if (k == 0) { kh = 0; wa = 0.0; }
+      if (k == o.ktot - 2) kh = o.ktot + 1;
+    } else if (k == 0 || k == o.ktot - 1) {
+      kh = k == 0 ? 0 : o.ktot + 1;
+      if (o.kind == 0) { wa = -1.0; wc = k == 0 ? o.lo : o.hi; }
+    }
+    auto row = [&](int jj, int kk) { return o.f + kk * o.plane + jj * o.ldi; };
+    f = row(j + 1, k + 1);
+    img = jh >= 0 ? row(jh, k + 1) : nullptr;
+    wall = kh >= 0 ? row(j + 1, kh) : nullptr;
+    wall_img = kh >= 0 && jh >= 0 ? row(jh, kh) : nullptr;
+    scale = o.scale;
+    nx = o.itot;
+    add = o.kind == 2;
+  }
+  __device__ __forceinline__ void store(double* r, int i, double x) const {
+    r[i] = x;
+    if (i == 1) r[nx + 1] = x;
+    if (i == nx) r[0] = x;
+  }
+  __device__ __forceinline__ void put(int i, double x) const {  // cell i of 1 .. itot
+    x *= scale;
+    if (add) x = f[i] + x;
+    store(f, i, x);
+    copies(i, x);
+  }
+  __device__ __forceinline__ void copies(int i, double x) const {
+    if (img) store(img, i, x);
+    if (wall) {
+      x = wa == 0.0 ? 0.0 : wc + wa * x;
+      store(wall, i, x);
+      if (wall_img) store(wall_img, i, x);
+    }
+  }
 };
 
 // Forward real-to-complex transform of nb rows of nx = 2 n reals per CTA:
@@ -694,6 +914,8 @@ __global__ void __launch_bounds__(kAnyThreads, 4) rows_r2c_any(long nrows, FastD
                                                             const double* __restrict__ src, double2* __restrict__ dst) {
   extern __shared__ __align__(16) double2 fsm[];
   const int n = P.n, ld = fld(n);
+  src += (long)blockIdx.y * nrows * 2 * n;  // field
+  dst += (long)blockIdx.y * nrows * (n + 1);
   const long r0 = (long)blockIdx.x * nb.d;
   const int rows = (int)min((long)nb.d, nrows - r0);
   double2* b0 = fsm;
@@ -720,9 +942,11 @@ __global__ void __launch_bounds__(kAnyThreads, 4) rows_r2c_any(long nrows, FastD
 __global__ void __launch_bounds__(kAnyThreads, 4) rows_c2r_any(long nrows, FastDiv nb, FftPlan P,
                                                             const double2* __restrict__ wpost,
                                                             const double2* __restrict__ src, double* __restrict__ dst,
-                                                            RowsOut out) {
+                                                            RowsOuts outs) {
   extern __shared__ __align__(16) double2 fsm[];
   const int n = P.n, ld = fld(n);
+  const RowsOut& out = outs.o[blockIdx.y];  // field
+  src += (long)blockIdx.y * nrows * (n + 1);
   const long r0 = (long)blockIdx.x * nb.d;
   const int rows = (int)min((long)nb.d, nrows - r0);
   double2* b0 = fsm;
@@ -747,12 +971,10 @@ __global__ void __launch_bounds__(kAnyThreads, 4) rows_c2r_any(long nrows, FastD
       double2* d2 = (double2*)dst + row * n;
       for (int t = lane; t < n; t += 32) d2[t] = cswap(z[r * ld + fpad(t)]);
     } else {
-      const int j = (int)(row % out.jtot);
-      const long k = row / out.jtot;
-      double* f = out.f + (k + 1) * out.plane + (j + 1) * out.ldi + 1;
+      const RowTarget t(out, (int)(row % out.jtot), (int)(row / out.jtot));
       for (int i = lane; i < 2 * n; i += 32) {
         const double2 v = z[r * ld + fpad(i >> 1)];
-        f[i] = (i & 1 ? v.x : v.y) * out.scale;
+        t.put(i + 1, i & 1 ? v.x : v.y);
       }
     }
   }
@@ -793,6 +1015,8 @@ __global__ void __launch_bounds__(kRegThreads) rows_r2c_reg(long nrows, const do
                                                            const double2* __restrict__ wp_g,
                                                            const double* __restrict__ src, double2* __restrict__ dst) {
   constexpr int TPS = N / 8, SPC = kRegThreads / TPS, LD = N + 1;
+  src += (long)blockIdx.y * nrows * 2 * N;  // field
+  dst += (long)blockIdx.y * nrows * (N + 1);
   __shared__ double2 tw[TwTab<N>::size], wp[N + 1];
   __shared__ double2 buf[SPC * LD];
   fill_tw<N>(tw, tw_g, threadIdx.x, kRegThreads);
@@ -829,14 +1053,16 @@ __global__ void __launch_bounds__(kRegThreads) rows_r2c_reg(long nrows, const do
 // Complex-to-real rows, the pre-processing of rows_c2r_any: the modes of the
 // CTA's rows come in transposed through shared memory (row pairs X_k,
 // X_{n-k}), the first pass's inputs are formed in registers, the last pass
-// writes the reals straight to global memory (16-byte runs, or pairs of
-// 8-byte values into a halo field).
+// writes the reals straight to global memory in 16-byte runs, or through the
+// slot into a field and its halo (RowTarget).
 template <int N>
 __global__ void __launch_bounds__(kRegThreads) rows_c2r_reg(long nrows, const double2* __restrict__ tw_g,
                                                            const double2* __restrict__ wp_g,
                                                            const double2* __restrict__ src, double* __restrict__ dst,
-                                                           RowsOut out) {
+                                                           RowsOuts outs) {
   constexpr int TPS = N / 8, SPC = kRegThreads / TPS, LD = N + 1;
+  const RowsOut& out = outs.o[blockIdx.y];  // field
+  src += (long)blockIdx.y * nrows * (N + 1);
   __shared__ double2 tw[TwTab<N>::size], wp[N + 1];
   __shared__ double2 buf[SPC * LD];
   fill_tw<N>(tw, tw_g, threadIdx.x, kRegThreads);
@@ -865,26 +1091,39 @@ __global__ void __launch_bounds__(kRegThreads) rows_c2r_reg(long nrows, const do
     v[r] = make_double2(sum.x - t2.y, sum.y + t2.x);
   }
   fft_reg<N>(v, seq, tau, tw, +1);
-  if (!ok) return;
-  constexpr int R = LastPass<N>::R, NS = LastPass<N>::NS;
   if (!out.f) {
+    if (!ok) return;
+    constexpr int R = LastPass<N>::R, NS = LastPass<N>::NS;
     double2* d2 = (double2*)dst + row * N;
 #pragma unroll
     for (int b = 0; b < 8 / R; ++b)
 #pragma unroll
       for (int q = 0; q < R; ++q) d2[out_pos<N, R, NS>(tau, b, q)] = v[b * R + q];
-  } else {
-    const long j = row % out.jtot, k = row / out.jtot;
-    double* f = out.f + (k + 1) * out.plane + (j + 1) * out.ldi + 1;
-#pragma unroll
-    for (int b = 0; b < 8 / R; ++b)
-#pragma unroll
-      for (int q = 0; q < R; ++q) {
-        const int m = out_pos<N, R, NS>(tau, b, q);
-        f[2 * m] = v[b * R + q].x * out.scale;
-        f[2 * m + 1] = v[b * R + q].y * out.scale;
-      }
+    return;
   }
+  __syncwarp();
+  store_last<N>(v, seq, tau);
+  __syncwarp();
+  if (!ok) return;
+  const RowTarget t(out, (int)(row % out.jtot), (int)(row / out.jtot));
+  const double* xs = (const double*)seq;
+  double x[16];  // cells tau + q TPS + 1
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const int i = tau + q * TPS;
+    x[q] = t.scale * xs[2 * swz(i >> 1) + (i & 1)];
+  }
+  double* f = t.f + 1 + tau;
+  if (t.add)
+#pragma unroll
+    for (int q = 0; q < 16; ++q) x[q] = f[q * TPS] + x[q];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) f[q * TPS] = x[q];
+  if (tau == 0) t.f[2 * N + 1] = x[0];
+  if (tau == TPS - 1) t.f[0] = x[15];
+  if (t.img || t.wall)
+#pragma unroll
+    for (int q = 0; q < 16; ++q) t.copies(tau + q * TPS + 1, x[q]);
 }
 
 // y transforms: contiguous sequences of length N in place, 256 / (N / 8) per
@@ -983,7 +1222,8 @@ std::vector<double> twiddles(int n) {  // exp(-2 pi i t / n) as (re, im) pairs
 
 bool pow2_fast(int n) { return n == 32 || n == 64 || n == 128 || n == 256; }
 
-size_t tri_tile_smem(int kmax, int C) { return (sizeof(double2) + sizeof(double)) * (size_t)kmax * C; }
+size_t tri_tile_smem(int kmax, int C) { return (sizeof(double2) + sizeof(double)) * (size_t)tile_size(kmax, C); }
+FastDiv segment_length(int kmax) { return fast_div((kmax + kSegs - 1) / kSegs); }
 
 // sequences per CTA of the mixed-radix row and column kernels: about 1280
 // values (two padded buffers: 46 KB, four CTAs of 128 threads on an SM)
@@ -1004,7 +1244,7 @@ struct Plans {
 
 }  // namespace
 
-int poisson_setup(sg_ctx* c, unsigned types) {
+int poisson_setup(sg_ctx* c, unsigned types, int nfields) {
   auto& s = c->pois;
   const sg_config& f = c->cfg;
   const long nxm = f.itot / 2 + 1, nslots = nxm * f.jtot;
@@ -1017,13 +1257,22 @@ int poisson_setup(sg_ctx* c, unsigned types) {
       }
     return SG_OK;
   };
-  if (s.ready) return tables();
-  if (f.itot % 2 != 0 || f.ktot < 4) return fail(c, SG_ERR_CONFIG, "solver1d here needs an even itot and ktot >= 4");
   const long nreal = (long)f.itot * f.jtot * f.ktot;
-  SG_TRY(dalloc(c, p, sizeof(double) * nreal), "alloc");
-  s.r = (double*)p;
-  SG_TRY(dalloc(c, p, sizeof(double2) * nslots * f.ktot), "alloc");
-  s.c = p;
+  auto fields = [&]() -> int {  // real and mode arrays for nfields fields at once
+    if (s.nfields >= nfields) return SG_OK;
+    SG_TRY(dalloc(c, p, sizeof(double) * nreal * std::min(nfields, 3)), "alloc");
+    s.r = (double*)p;
+    SG_TRY(dalloc(c, p, sizeof(double2) * nslots * f.ktot * nfields), "alloc");
+    s.c = p;
+    s.nfields = nfields;
+    return SG_OK;
+  };
+  if (s.ready) {
+    SG_RET(fields());
+    return tables();
+  }
+  if (f.itot % 2 != 0 || f.ktot < 4) return fail(c, SG_ERR_CONFIG, "solver1d here needs an even itot and ktot >= 4");
+  SG_RET(fields());
   SG_RET(tables());
   // initsolver.f90:111-130: xrt(2m) = xrt(2m+1) = -4 dxi^2 sin(2m pi / (2 itot))^2, the
   // modes of a real transform in x; in y the complex modes j and jtot - j share yrt
@@ -1068,20 +1317,21 @@ int poisson_setup(sg_ctx* c, unsigned types) {
   return SG_OK;
 }
 
-void poisson_free(sg_ctx* c) { (void)c; }
+
 
 namespace {
 
 template <int N>
-void launch_r2c(long nrows, const double2* tw, const double2* wp, const double* r, double2* m, cudaStream_t st) {
-  constexpr int SPC = kRegThreads / (N / 8);
-  rows_r2c_reg<N><<<(unsigned)((nrows + SPC - 1) / SPC), kRegThreads, 0, st>>>(nrows, tw, wp, r, m);
-}
-template <int N>
-void launch_c2r(long nrows, const double2* tw, const double2* wp, const double2* m, double* r, const RowsOut& o,
+void launch_r2c(long nrows, int nf, const double2* tw, const double2* wp, const double* r, double2* m,
                 cudaStream_t st) {
   constexpr int SPC = kRegThreads / (N / 8);
-  rows_c2r_reg<N><<<(unsigned)((nrows + SPC - 1) / SPC), kRegThreads, 0, st>>>(nrows, tw, wp, m, r, o);
+  rows_r2c_reg<N><<<dim3((unsigned)((nrows + SPC - 1) / SPC), nf), kRegThreads, 0, st>>>(nrows, tw, wp, r, m);
+}
+template <int N>
+void launch_c2r(long nrows, int nf, const double2* tw, const double2* wp, const double2* m, double* r,
+                const RowsOuts& o, cudaStream_t st) {
+  constexpr int SPC = kRegThreads / (N / 8);
+  rows_c2r_reg<N><<<dim3((unsigned)((nrows + SPC - 1) / SPC), nf), kRegThreads, 0, st>>>(nrows, tw, wp, m, r, o);
 }
 template <int N>
 void launch_cols(long nseq, const double2* tw, int sign, double2* m, cudaStream_t st) {
@@ -1095,90 +1345,185 @@ cudaError_t launch_tri_tile(int kmax, int jtot, int nxm, int e, double a, const 
   const size_t smem = tri_tile_smem(kmax, C);
   cudaError_t err = smem_limit(tri_tile_kernel<C>, smem);
   if (err != cudaSuccess) return err;
-  tri_tile_kernel<C><<<dim3((unsigned)((jtot + C - 1) / C), (unsigned)nxm), kTriThreads, smem, st>>>(kmax, jtot, e, a,
-                                                                                                   zt, c);
+  tri_tile_kernel<C><<<dim3((unsigned)((jtot + C - 1) / C), (unsigned)nxm), 16 * C, smem, st>>>(
+      kmax, jtot, segment_length(kmax), e, a, zt, c);
+  return cudaGetLastError();
+}
+
+constexpr size_t kThirdOfSm = 75 * 1024, kTileMost = 220 * 1024;
+
+cudaError_t launch_tri_apply(int kmax, int jtot, int nxm, int e, double a, const double* zt, double2* c,
+                             cudaStream_t st) {
+  tri_apply_kernel<<<(unsigned)((2L * nxm * jtot + 127) / 128), 128, 0, st>>>(kmax, jtot, nxm, e, a, zt, c);
   return cudaGetLastError();
 }
 
 // The widest tile of which at least three fit an SM (runs of 256, 128 or 64
 // bytes); tiles of four columns as long as one fits, then global memory.
 cudaError_t launch_tri(int kmax, int jtot, int nxm, int e, double a, const double* zt, double2* c, cudaStream_t st) {
-  constexpr size_t third = 72 * 1024, most = 220 * 1024;
-  if (tri_tile_smem(kmax, 16) <= third) return launch_tri_tile<16>(kmax, jtot, nxm, e, a, zt, c, st);
-  if (tri_tile_smem(kmax, 8) <= third) return launch_tri_tile<8>(kmax, jtot, nxm, e, a, zt, c, st);
-  if (tri_tile_smem(kmax, 4) <= most) return launch_tri_tile<4>(kmax, jtot, nxm, e, a, zt, c, st);
-  tri_apply_kernel<<<(unsigned)((2L * nxm * jtot + 127) / 128), 128, 0, st>>>(kmax, jtot, nxm, e, a, zt, c);
+  if (tri_tile_smem(kmax, 16) <= kThirdOfSm) return launch_tri_tile<16>(kmax, jtot, nxm, e, a, zt, c, st);
+  if (tri_tile_smem(kmax, 8) <= kThirdOfSm) return launch_tri_tile<8>(kmax, jtot, nxm, e, a, zt, c, st);
+  if (tri_tile_smem(kmax, 4) <= kTileMost) return launch_tri_tile<4>(kmax, jtot, nxm, e, a, zt, c, st);
+  return launch_tri_apply(kmax, jtot, nxm, e, a, zt, c, st);
+}
+
+template <int C>
+cudaError_t launch_flow_tile(int kmax, int jtot, int nxm, double a, const FlowModes& F, cudaStream_t st) {
+  const size_t smem = 3 * tri_tile_smem(kmax, C);
+  cudaError_t err = smem_limit(tri_flow_tile_kernel<C>, smem);
+  if (err != cudaSuccess) return err;
+  tri_flow_tile_kernel<C><<<dim3((unsigned)((jtot + C - 1) / C), (unsigned)nxm), 48 * C, smem, st>>>(
+      kmax, jtot, segment_length(kmax), a, F);
   return cudaGetLastError();
 }
 
-}  // namespace
+// Likewise for the flow step's four solves, three times the tile's memory.
+cudaError_t launch_flow_tri(int kmax, int jtot, int nxm, double a, const FlowModes& F, cudaStream_t st, int& launches) {
+  launches += 1;
+  if (3 * tri_tile_smem(kmax, 8) <= kThirdOfSm) return launch_flow_tile<8>(kmax, jtot, nxm, a, F, st);
+  if (3 * tri_tile_smem(kmax, 4) <= kTileMost) return launch_flow_tile<4>(kmax, jtot, nxm, a, F, st);
+  const long n = (long)nxm * kmax * jtot;
+  const unsigned nb = (unsigned)((n + 255) / 256);
+  cudaError_t e = launch_tri(kmax, jtot, nxm, 2, a, F.z2, F.u, st);
+  if (e == cudaSuccess) e = launch_tri(kmax, jtot, nxm, 2, a, F.z2, F.v, st);
+  if (e == cudaSuccess) e = launch_tri(kmax, jtot, nxm, 3, a, F.z3, F.w, st);
+  if (e != cudaSuccess) return e;
+  mode_divergence_kernel<<<nb, 256, 0, st>>>(kmax, jtot, n, F);
+  e = launch_tri(kmax, jtot, nxm, 1, a, F.z1, F.p, st);
+  if (e != cudaSuccess) return e;
+  mode_correct_kernel<<<nb, 256, 0, st>>>(kmax, jtot, n, F);
+  launches += 5;
+  return cudaGetLastError();
+}
 
-int poisson_solve(sg_ctx* c, double* r, int e, double shift, cudaStream_t st, const PoisOut* out) {
+// The pivots of row type e for this shift, (re)built if they were made for
+// another; inside a stream capture the build is recorded but has not run, so
+// they are not marked valid for the direct calls that may come before the
+// graph's first launch.
+int poisson_tables(sg_ctx* c, int e, double shift, cudaStream_t st) {
+  auto& s = c->pois;
+  const sg_config& f = c->cfg;
+  const int nxm = f.itot / 2 + 1;
+  if (e < 0 || e > 3 || !s.zt[e]) return fail(c, SG_ERR_STATE, "solver1d: tables of this row type were not set up");
+  if (s.tvalid[e] && s.tshift[e] == shift) return SG_OK;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  SG_TRY(cudaStreamIsCapturing(st, &cap), "solver1d");
+  tri_coeff_kernel<<<(unsigned)((nxm * f.jtot + 127) / 128), 128, 0, st>>>(
+      f.ktot, f.jtot, nxm, e, 1.0 / (f.lz / f.ktot), shift, s.tab, s.tab + nxm, s.zt[e]);
+  SG_TRY(cudaGetLastError(), "solver1d");
+  s.tvalid[e] = cap == cudaStreamCaptureStatusNone;
+  s.tshift[e] = shift;
+  c->launches += 1;
+  return SG_OK;
+}
+
+// nf real fields [nf][ktot][jtot][itot] to their modes [nf][m][k][j]
+int rows_forward(sg_ctx* c, int nf, const double* r, double2* modes, cudaStream_t st) {
   auto& s = c->pois;
   const sg_config& f = c->cfg;
   Plans pl;
   std::memcpy(&pl, s.plans, sizeof(pl));
-  const int n = f.itot / 2, nxm = n + 1;
+  const int n = f.itot / 2, nb = any_rows(n);
   const long nrows = (long)f.jtot * f.ktot;
-  const RowsOut ro{out ? out->f : nullptr, out ? out->ldi : 0, out ? out->plane : 0, out ? out->scale : 0.0, f.jtot};
-  const double dzi = 1.0 / (f.lz / f.ktot);
-  double2* modes = (double2*)s.c;
-  const double2* twx = s.w;
-  const double2* twy = s.w + n;
-  int launches = 5;
-  if (e < 0 || e > 3 || !s.zt[e]) return fail(c, SG_ERR_STATE, "solver1d: tables of this row type were not set up");
-  if (!s.tvalid[e] || s.tshift[e] != shift) {
-    // (re)build the tables for this shift; inside a stream capture the build
-    // is recorded but has not run, so they are not marked valid for the
-    // direct calls that may come before the graph's first launch
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    SG_TRY(cudaStreamIsCapturing(st, &cap), "solver1d");
-    tri_coeff_kernel<<<(unsigned)((nxm * f.jtot + 127) / 128), 128, 0, st>>>(f.ktot, f.jtot, nxm, e, dzi, shift, s.tab,
-                                                                             s.tab + nxm, s.zt[e]);
-    s.tvalid[e] = cap == cudaStreamCaptureStatusNone;
-    s.tshift[e] = shift;
-    launches += 1;
-  }
-  // x rows to modes
-  const int rx = any_rows(n);
-  const unsigned gx = (unsigned)((nrows + rx - 1) / rx);
   if (pow2_fast(n)) {
-#define SG_R2C(N) launch_r2c<N>(nrows, twx, s.wpost, r, modes, st)
+#define SG_R2C(N) launch_r2c<N>(nrows, nf, s.w, s.wpost, r, modes, st)
     SG_POW2_DISPATCH(n, SG_R2C)
 #undef SG_R2C
   } else {
     SG_TRY(smem_limit(rows_r2c_any, any_smem(n)), "fft");
-    rows_r2c_any<<<gx, kAnyThreads, any_smem(n), st>>>(nrows, fast_div(rx), pl.x, s.wpost, r, modes);
+    rows_r2c_any<<<dim3((unsigned)((nrows + nb - 1) / nb), nf), kAnyThreads, any_smem(n), st>>>(nrows, fast_div(nb), pl.x,
+                                                                                              s.wpost, r, modes);
   }
-  // y transforms, elimination, inverse y transforms
-  const long nseq = (long)nxm * f.ktot;
-  const int ry = any_rows(f.jtot);
-  auto cols = [&](int sign) -> int {
-    if (pow2_fast(f.jtot)) {
-#define SG_COLS(N) launch_cols<N>(nseq, twy, sign, modes, st)
-      SG_POW2_DISPATCH(f.jtot, SG_COLS)
-#undef SG_COLS
-    } else {
-      SG_TRY(smem_limit(cols_any, any_smem(f.jtot)), "fft");
-      cols_any<<<(unsigned)((nseq + ry - 1) / ry), kAnyThreads, any_smem(f.jtot), st>>>(nseq, ry, pl.y, sign > 0, modes);
-    }
-    return SG_OK;
-  };
-  SG_RET(cols(-1));
-  SG_TRY(launch_tri(f.ktot, f.jtot, nxm, e, dzi * dzi, s.zt[e], modes, st), "solver1d");
-  SG_RET(cols(+1));
-  // modes to x rows
+  SG_TRY(cudaGetLastError(), "solver1d");
+  c->launches += 1;
+  return SG_OK;
+}
+
+int rows_inverse(sg_ctx* c, int nf, const double2* modes, double* r, const RowsOuts& out, cudaStream_t st) {
+  auto& s = c->pois;
+  const sg_config& f = c->cfg;
+  Plans pl;
+  std::memcpy(&pl, s.plans, sizeof(pl));
+  const int n = f.itot / 2, nb = any_rows(n);
+  const long nrows = (long)f.jtot * f.ktot;
   if (pow2_fast(n)) {
-#define SG_C2R(N) launch_c2r<N>(nrows, twx, s.wpost, modes, r, ro, st)
+#define SG_C2R(N) launch_c2r<N>(nrows, nf, s.w, s.wpost, modes, r, out, st)
     SG_POW2_DISPATCH(n, SG_C2R)
 #undef SG_C2R
   } else {
     SG_TRY(smem_limit(rows_c2r_any, any_smem(n)), "fft");
-    rows_c2r_any<<<gx, kAnyThreads, any_smem(n), st>>>(nrows, fast_div(rx), pl.x, s.wpost, modes, r, ro);
+    rows_c2r_any<<<dim3((unsigned)((nrows + nb - 1) / nb), nf), kAnyThreads, any_smem(n), st>>>(nrows, fast_div(nb), pl.x,
+                                                                                              s.wpost, modes, r, out);
   }
   SG_TRY(cudaGetLastError(), "solver1d");
-  c->launches += launches;
+  c->launches += 1;
   return SG_OK;
+}
+
+// y transforms of the modes of nf fields, in place
+int cols_transform(sg_ctx* c, int nf, int sign, double2* modes, cudaStream_t st) {
+  auto& s = c->pois;
+  const sg_config& f = c->cfg;
+  Plans pl;
+  std::memcpy(&pl, s.plans, sizeof(pl));
+  const int n = f.itot / 2, nb = any_rows(f.jtot);
+  const long nseq = (long)nf * (n + 1) * f.ktot;
+  if (pow2_fast(f.jtot)) {
+#define SG_COLS(N) launch_cols<N>(nseq, s.w + n, sign, modes, st)
+    SG_POW2_DISPATCH(f.jtot, SG_COLS)
+#undef SG_COLS
+  } else {
+    SG_TRY(smem_limit(cols_any, any_smem(f.jtot)), "fft");
+    cols_any<<<(unsigned)((nseq + nb - 1) / nb), kAnyThreads, any_smem(f.jtot), st>>>(nseq, nb, pl.y, sign > 0, modes);
+  }
+  SG_TRY(cudaGetLastError(), "solver1d");
+  c->launches += 1;
+  return SG_OK;
+}
+
+}  // namespace
+
+int poisson_solve(sg_ctx* c, double* r, int e, double shift, cudaStream_t st) {
+  auto& s = c->pois;
+  const sg_config& f = c->cfg;
+  const double dzi = 1.0 / (f.lz / f.ktot);
+  double2* modes = (double2*)s.c;
+  SG_RET(poisson_tables(c, e, shift, st));
+  SG_RET(rows_forward(c, 1, r, modes, st));
+  SG_RET(cols_transform(c, 1, -1, modes, st));
+  SG_TRY(launch_tri(f.ktot, f.jtot, f.itot / 2 + 1, e, dzi * dzi, s.zt[e], modes, st), "solver1d");
+  c->launches += 1;
+  SG_RET(cols_transform(c, 1, +1, modes, st));
+  return rows_inverse(c, 1, modes, r, RowsOuts{}, st);
+}
+
+int poisson_project(sg_ctx* c, const double* r3, double dt, double shift, double* u, double* v, double* w, double* p,
+                    double vb2, double vt2, cudaStream_t st) {
+  auto& s = c->pois;
+  const sg_config& f = c->cfg;
+  const int nxm = f.itot / 2 + 1;
+  const double dxi = 1.0 / (f.lx / f.itot), dyi = 1.0 / (f.ly / f.jtot), dzi = 1.0 / (f.lz / f.ktot), dti = 1.0 / dt;
+  const long nm = (long)nxm * f.ktot * f.jtot;
+  double2* M = (double2*)s.c;
+  SG_RET(poisson_tables(c, 2, shift, st));
+  SG_RET(poisson_tables(c, 3, shift, st));
+  SG_RET(poisson_tables(c, 1, 0.0, st));
+  SG_RET(rows_forward(c, 3, r3, M, st));
+  SG_RET(cols_transform(c, 3, -1, M, st));
+  const FlowModes F{M,        M + nm,   M + 2 * nm, M + 3 * nm,   s.zt[2],  s.zt[3],  s.zt[1], s.wpost,
+                    s.w + f.itot / 2, dti * dxi, dti * dyi, dti * dzi, dt * dxi, dt * dyi, dt * dzi};
+  int launches = 0;
+  SG_TRY(launch_flow_tri(f.ktot, f.jtot, nxm, dzi * dzi, F, st, launches), "solver1d");
+  c->launches += launches;
+  SG_RET(cols_transform(c, 4, +1, M, st));
+  const IBGrid& g = c->grid;
+  const long plane = (long)g.ldi * g.ldj;
+  const double scale = 1.0 / ((double)f.itot * f.jtot);
+  const RowsOuts o{{{u, g.ldi, plane, scale, 0.0, 0.0, f.itot, f.jtot, f.ktot, 0},
+                    {v, g.ldi, plane, scale, vb2, vt2, f.itot, f.jtot, f.ktot, 0},
+                    {w, g.ldi, plane, scale, 0.0, 0.0, f.itot, f.jtot, f.ktot, 1},
+                    {p, g.ldi, plane, scale, 0.0, 0.0, f.itot, f.jtot, f.ktot, 2}}};
+  return rows_inverse(c, 4, M, nullptr, o, st);
 }
 
 }  // namespace sg
