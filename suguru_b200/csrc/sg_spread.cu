@@ -32,12 +32,21 @@
 //    minus that of 1.5 * 2^23 -- no conversion instruction per contribution.
 //    The fixed-point step is 2^-22 of 0.3 times the component's largest
 //    contribution, below FP32 rounding of a typical cell value.
-//  - FP64: 64-bit fixed point (|sum| < 2^56 from the component's largest
-//    contribution in the tile times its entry count, or above 4096 entries
-//    from 0.3 * the same exact integer sum of m_c as FP32 takes) kept as three limbs of 19 bits, the
-//    lower two unsigned, so that the atomics stay native 32-bit adds; with at
-//    most 4096 contributions per pass no limb can overflow, and between passes
-//    the limbs are folded into 64-bit registers.
+//  - FP64: fixed point in two signed 32-bit limbs, in passes of at most 255
+//    entries whose limbs are then added into 64-bit registers.  With K entries
+//    in a pass and h the bit length of K, a contribution v, |v| < 2^(63-2h), is
+//    split as hi 2^p + lo, p = 32 - h: one FMA against 1.5 * 2^(52+p) rounds v
+//    to a multiple of 2^p whose integer is the low word of the sum, a second
+//    one forms the exact rest, |lo| <= 2^(p-1), and an addition of 1.5 * 2^52
+//    rounds it, so that K contributions overflow neither limb and no
+//    conversion or 64-bit shift is needed.  The step is 0.3 times the largest
+//    m_c over 2^(63-2h): 2^-47 of the largest contribution with 128 or more
+//    entries, finer with fewer.  Bound by the shared-memory atomics: three
+//    limbs of 19 bits in passes of 4096, split with a 64-bit integer
+//    conversion (step 2^-56 of the entry count times the largest m_c, coarser
+//    but for tiles of over 4096 very uneven entries), took 251 us at 524,288
+//    points on 256 x 256 x 128, these two take 208 us; leaving out the
+//    contributions that fall outside the tile by a predicate took 270 us.
 // Entries go to threads in blocks of 256: the lowest ceil(k/32) warps take the
 // k entries of a block, interleaved, so that no warp idles on a short list and
 // neighbouring points (adjacent entries) land in different warps, where they
@@ -51,45 +60,42 @@ namespace {
 
 constexpr float kMagic = 12582912.0f;          // 1.5 * 2^23
 constexpr int kMagicBits = 0x4B400000;          // its bit pattern
-constexpr int LB = 19;      // FP64 limb width
+constexpr double kMagic64 = 6755399441055744.0;  // 1.5 * 2^52
 constexpr int kOut = -(1 << 24);  // offset of a stencil node outside the tile
-constexpr int MAXC = 4096;  // FP64 contributions per pass: 19 + 12 <= 31 bits per limb
 
 template <class T>
 struct Fixed;
 template <>
 struct Fixed<float> {
   static constexpr int NW = 1;
-  static constexpr int QB = 30;
   static constexpr int PASS = 1 << 30;
 };
 template <>
 struct Fixed<double> {
-  static constexpr int NW = 3;
-  static constexpr int QB = 3 * LB - 1;
-  static constexpr int PASS = MAXC;
-  __device__ static __forceinline__ void add(unsigned int* base, int stride, double v) {
-    long long q = __double2ll_rn(v);  // q = sum_w limb_w 2^(LB w)
-    atomicAdd(base, (unsigned int)(q & ((1ll << LB) - 1)));
-    q >>= LB;
-    atomicAdd(base + stride, (unsigned int)(q & ((1ll << LB) - 1)));
-    q >>= LB;
-    atomicAdd(base + 2 * stride, (unsigned int)(int)q);
+  static constexpr int NW = 2;
+  static constexpr int PASS = 255;
+  // low limb width for `n` entries in a pass: 32 - the bit length of n
+  __device__ static __forceinline__ int low_bits(int n) { return __clz(n); }
+  // adds pyz * wx (in units of the step); mh = 1.5 * 2^(52+p)
+  __device__ static __forceinline__ void add(unsigned int* base, int stride, double pyz, double wx, double mh) {
+    const double t = fma(pyz, wx, mh);
+    const double l = fma(pyz, wx, -(t - mh)) + kMagic64;
+    atomicAdd(base + stride, (unsigned int)__double2loint(t));
+    atomicAdd(base, (unsigned int)__double2loint(l));
   }
-  __device__ static __forceinline__ long long fold(const unsigned int* base, int stride) {
-    long long v = (long long)(int)base[2 * stride];
-    v = (v << LB) + (long long)base[stride];
-    return (v << LB) + (long long)base[0];
+  __device__ static __forceinline__ long long fold(const unsigned int* base, int stride, int p) {
+    return ((long long)(int)base[stride] << p) + (long long)(int)base[0];
   }
 };
 
-// The smallest e with b < 2^e (0 for b <= 0), at least -60 so that the
-// scales stay finite in float: the exponent field of b read directly (these
-// run once per thread and tile, so no library frexp/ldexp calls).
-__device__ __forceinline__ int exp_above(double b) {
+// The smallest e with b < 2^e (0 for b <= 0), at least `least` so that the
+// scales stay finite (-60 in float, -900 in double): the exponent field of b
+// read directly (these run once per thread and tile, so no library
+// frexp/ldexp calls).
+__device__ __forceinline__ int exp_above(double b, int least = -60) {
   if (!(b > 0.0)) return 0;
   const int e = (int)((__double_as_longlong(b) >> 52) & 0x7ff) - 1022;
-  return e < -60 ? -60 : e;
+  return e < least ? least : e;
 }
 
 // exact 2^e, built from its exponent field inside the normal range
@@ -118,7 +124,7 @@ __device__ __forceinline__ void tile_scales(int e0, int e1, const int* __restric
                                             const ForceRec<T>* __restrict__ frc, T (*s_red)[8],
                                             unsigned long long (*s_sum)[8], T* scale, T* iscale) {
   constexpr bool F32 = sizeof(T) == 4;
-  constexpr int QB = Fixed<T>::QB;
+  constexpr int QB = 30;  // FP32 sums stay below 2^QB
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   {
     T rmax[3] = {T(0), T(0), T(0)};
@@ -142,24 +148,28 @@ __device__ __forceinline__ void tile_scales(int e0, int e1, const int* __restric
       for (int q = 1; q < 8; ++q) rmax[c] = fmax(rmax[c], s_red[c][q]);
     }
     const int cnt = e1 - e0;
-    // FP64: |sum| < 2^QB from the largest m_c times the entry count
     int sh[3];
+    if constexpr (!F32) {
+      // FP64: every contribution below 2^(63-2h) for a pass's entries, and the
+      // tile's sum below 2^62 (more than 2^15 entries)
+      const int h = 32 - Fixed<double>::low_bits(min(cnt, Fixed<double>::PASS));
 #pragma unroll
-    for (int c = 0; c < 3; ++c) sh[c] = QB - exp_above((double)rmax[c] * (double)(F32 ? 0.3 * cnt : cnt));
-    // FP32: every single contribution below 2^22 ...
-    int sh1[3] = {QB, QB, QB};
-    bool need[3] = {false, false, false}, dense = false;
+      for (int c = 0; c < 3; ++c) {
+        const double m = 0.3 * (double)rmax[c];
+        sh[c] = min(63 - 2 * h - exp_above(m, -900), 62 - exp_above(m * (double)cnt, -900));
+      }
+    } else {
 #pragma unroll
-    for (int c = 0; c < 3; ++c) {
-      if constexpr (F32) {
+      for (int c = 0; c < 3; ++c) sh[c] = QB - exp_above((double)rmax[c] * (0.3 * cnt));
+      // FP32: every single contribution below 2^22 ...
+      int sh1[3] = {QB, QB, QB};
+      bool need[3] = {false, false, false}, dense = false;
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
         sh1[c] = 22 - exp_above(0.3 * (double)rmax[c]);
         need[c] = sh[c] < sh1[c];
-      } else {
-        need[c] = cnt > MAXC;  // FP64: the count bound costs precision above one pass of entries
+        dense = dense || need[c];
       }
-      dense = dense || need[c];
-    }
-    {
       if (dense) {  // uniform across the CTA: computed from the block-wide maxima
         // ... and, where the count bound would cost precision (more than 2^8
         // entries), |sum| < 2^QB from 0.3 * sum of m_c, taken as an exact
@@ -197,9 +207,8 @@ __device__ __forceinline__ void tile_scales(int e0, int e1, const int* __restric
           if (need[c]) sh[c] = QB - exp_above(0.3 * ((double)t * pow2<double>(exr[c] - 12)));
         }
       }
-      if constexpr (F32)
 #pragma unroll
-        for (int c = 0; c < 3; ++c) sh[c] = min(sh[c], sh1[c]);
+      for (int c = 0; c < 3; ++c) sh[c] = min(sh[c], sh1[c]);
     }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
@@ -230,7 +239,7 @@ __global__ void pack_forces_kernel(long n, double dvi, const T* __restrict__ FX,
 // indicator's lagr2eulrind, interp_spread.f90:1319-1343) instead of the
 // staggered ones.
 template <class T, int TX, int TY, int TZ, bool CTR>
-__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) spread_kernel(IBGrid g, const int* __restrict__ entries,
+__global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) spread_kernel(IBGrid g, const int* __restrict__ entries,
                                                      const int* __restrict__ starts,
                                                      const PosRec<T>* __restrict__ pos,
                                                      const ForceRec<T>* __restrict__ frc, T* __restrict__ ox,
@@ -269,6 +278,12 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) spread_kernel(IBG
     tile_scales<T>(e0, e1, entries, frc, s_red, s_sum, scale, iscale);
 
     // ---- one point per thread, in passes of at most PASS entries
+    int lowb = 0;    // FP64: width of the low limb
+    double mh = 0.0;  // and 1.5 * 2^(52 + lowb)
+    if constexpr (!F32) {
+      lowb = Fixed<double>::low_bits(min(e1 - e0, Fixed<double>::PASS));
+      mh = kMagic64 * pow2<double>(lowb);
+    }
     for (int c0 = e0; c0 < e1; c0 += Fixed<T>::PASS) {
       const int c1 = min(e1, c0 + Fixed<T>::PASS);
       for (int eb = c0; eb < c1; eb += 256) {
@@ -347,7 +362,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) spread_kernel(IBG
                   const float t = fmaf(pyz, wx, kMagic);  // round(pyz * wx) in the low mantissa bits
                   atomicAdd(&acc[0][c][slot], (unsigned int)(__float_as_int(t) - kMagicBits));
                 } else {
-                  Fixed<T>::add(&acc[0][c][slot], 3 * NCP, pyz * wx);
+                  Fixed<T>::add(&acc[0][c][slot], 3 * NCP, pyz, wx, mh);
                 }
               }
             }
@@ -356,7 +371,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) spread_kernel(IBG
       }
       __syncthreads();
       if constexpr (!F32) {
-        // fold this pass's limbs into 64-bit totals and clear them
+        // fold this pass's limbs into 64-bit totals, and clear them for another
+        const bool more = c1 < e1;
 #pragma unroll
         for (int r = 0; r < NT; ++r) {
           const int q = tid + 256 * r;
@@ -364,13 +380,14 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 2) spread_kernel(IBG
             const int sq = q % TX + RS * ((q / TX) % TY) + PS * (q / (TX * TY));  // padded slot
 #pragma unroll
             for (int c = 0; c < 3; ++c) {
-              tot[r][c] += Fixed<double>::fold(&acc[0][c][sq], 3 * NCP);
+              tot[r][c] += Fixed<double>::fold(&acc[0][c][sq], 3 * NCP, lowb);
+              if (more)
 #pragma unroll
-              for (int w = 0; w < NW; ++w) acc[w][c][sq] = 0u;
+                for (int w = 0; w < NW; ++w) acc[w][c][sq] = 0u;
             }
           }
         }
-        __syncthreads();
+        if (more) __syncthreads();
       }
     }
   }
