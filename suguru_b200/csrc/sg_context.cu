@@ -130,13 +130,12 @@ cudaError_t build_tables(sg_ctx* c, Group& g) {
   return cudaSuccess;
 }
 
-void add_problem(std::vector<LegProblem>& P, std::vector<LegWork>& W, const LegProblem& p, int& maxJ, int& maxK) {
+void add_problem(std::vector<LegProblem>& P, std::vector<LegWork>& W, const LegProblem& p, size_t& elems) {
   const int id = (int)P.size();
   P.push_back(p);
   for (int m = 0; m < p.M; ++m)
     for (int q0 = 0; q0 < p.Q; q0 += 32) W.push_back(LegWork{id, m, q0});
-  maxJ = std::max(maxJ, p.J);
-  maxK = std::max(maxK, p.K);
+  elems = std::max(elems, legendre_elems(p.J, p.K, 0, 0));
 }
 
 LegProblem prob(const void* A, long long sAc, long long sAr, long long sAm, const void* B, long long sBm, void* D,
@@ -182,7 +181,7 @@ int bend_setup(sg_ctx* c) {
   const int pi = c->mixed ? 1 : 0;
   std::vector<LegProblem> P = c->h_probs;
   std::vector<LegWork> W, WT;
-  int maxJ = 0, maxK = 0;
+  size_t elems = 0;
   std::vector<int> ids;
   for (size_t gi = 0; gi < c->groups.size(); ++gi) {
     Group& gr = c->groups[gi];
@@ -207,7 +206,7 @@ int bend_setup(sg_ctx* c) {
     ids.push_back((int)P.size());
     add_problem(P, W, prob(gr.buf.Cpos, 6 * LN * LN, LN * LN, LN, gr.tab.syn_B[pi], 2 * LD * LN, gr.buf.GB,
                            6 * LN * 2 * LD, LN * 2 * LD, 2 * LD, 6, n, N, 2 * nD, N, 1, (int)gi, 4),
-                maxJ, maxK);
+                elems);
   }
   if (c->mixed) {
     std::vector<uint16_t> img;
@@ -244,8 +243,7 @@ int bend_setup(sg_ctx* c) {
   SG_TRY(upload(c, tmp, W), "work");
   c->d_lwB = (LegWork*)tmp;
   c->nlwB = (int)W.size();
-  c->maxJB = maxJ;
-  c->maxKB = maxK;
+  c->leg_elemsB = elems;
   c->h_probs = P;
   assign_terms(c, c->h_probs);
   SG_TRY(upload(c, tmp, c->h_probs), "problems");
@@ -392,32 +390,33 @@ int setup(sg_ctx* c) {
     const int G = (int)gi;
     // S0: analysis of the displacement (force grid, truncated to degree < N)
     add_problem(P, W[0], prob(b.Fpos, 6 * N * nD, N * nD, nD, gr.tab.ana_D[pi], N * nD, b.Cpos, 6 * N * N, N * N, N,
-                              6, n, N, N, nD, 0, G, 1), c->maxJ[0], c->maxK[0]);
+                              6, n, N, N, nD, 0, G, 1), c->leg_elems[0]);
     // S1: synthesis of P, dP, d2P series on the dealias grid
     add_problem(P, W[1], prob(b.Cpos, 6 * N * N, N * N, N, gr.tab.syn_D[pi], 3 * nD * N, b.G, 6 * N * 3 * nD,
-                              N * 3 * nD, 3 * nD, 6, n, N, 3 * nD, N, 1, G, 0), c->maxJ[1], c->maxK[1]);
+                              N * 3 * nD, 3 * nD, 6, n, N, 3 * nD, N, 1, G, 0), c->leg_elems[1]);
     // S2: analysis of force and normals (dealias grid, truncated)
     add_problem(P, W[2], prob(b.Fout, 12 * N * nD, N * nD, nD, gr.tab.ana_D[pi], N * nD, b.Cout, 12 * N * N, N * N, N,
-                              12, n, N, N, nD, 0, G, 1), c->maxJ[2], c->maxK[2]);
+                              12, n, N, N, nD, 0, G, 1), c->leg_elems[2]);
     // S3: synthesis on the SH grid: normals (rows 0-5) and shape (rows 6-11)
     add_problem(P, W[3], prob((const char*)b.Cout + E * 6 * N * N, 12 * N * N, N * N, N, gr.tab.syn_O[pi],
                               2 * nO * N, b.GO, 12 * N * 2 * nO, N * 2 * nO, 2 * nO, 6, n, N, 2 * nO, N, 1, G, 2),
-                c->maxJ[3], c->maxK[3]);
+                c->leg_elems[3]);
     add_problem(P, W[3], prob(b.Cpos, 6 * N * N, N * N, N, gr.tab.syn_O[pi], 2 * nO * N,
                               (char*)b.GO + E * 6 * N * 2 * nO, 12 * N * 2 * nO, N * 2 * nO, 2 * nO, 6, n, N, 2 * nO,
                               N, 1, G, 2),
-                c->maxJ[3], c->maxK[3]);
+                c->leg_elems[3]);
     // S4: analysis on the SH grid of renormalised normals and surface metric
     add_problem(P, W[4], prob(b.Fsh, 8 * N * nO, N * nO, nO, gr.tab.ana_O[pi], N * nO, b.Csh, 8 * N * N, N * N, N, 8,
-                              n, N, N, nO, 0, G, 3), c->maxJ[4], c->maxK[4]);
+                              n, N, N, nO, 0, G, 3), c->leg_elems[4]);
     // S5: synthesis on the force grid (P only): force rows 0-5, normals+surfmet rows 6-13
     add_problem(P, W[5], prob(b.Cout, 12 * N * N, N * N, N, gr.tab.syn_D[pi], 3 * nD * N, b.GF, 14 * N * nD, N * nD,
-                              nD, 6, n, N, nD, N, 1, G, 0), c->maxJ[5], c->maxK[5]);
+                              nD, 6, n, N, nD, N, 1, G, 0), c->leg_elems[5]);
     add_problem(P, W[5], prob(b.Csh, 8 * N * N, N * N, N, gr.tab.syn_D[pi], 3 * nD * N,
                               (char*)b.GF + E * 6 * N * nD, 14 * N * nD, N * nD, nD, 8, n, N, nD, N, 1, G, 0),
-                c->maxJ[5], c->maxK[5]);
+                c->leg_elems[5]);
   }
-  // tensor-core path (FP32 data): three launches of chained contractions.
+  // chained contractions in three launches (tensor cores in the mixed path,
+  // CUDA cores in FP64).
   // Per group the problems above are, in order, S0 S1 S2 S3a S3b S4 S5a S5b;
   // S2 is split into its force rows (S2f) and normal rows (S2n) so that each
   // half chains into the synthesis that consumes it:
@@ -426,7 +425,7 @@ int setup(sg_ctx* c) {
   // With the surrogate on, S5a runs in launch 2 instead, after the surrogate
   // force has replaced the analysed force rows.
   std::vector<int> roots[3];
-  if (c->mixed) {
+  {
     const size_t ng = c->groups.size();
     for (size_t gi = 0; gi < ng; ++gi) {
       const Group& gr = c->groups[gi];
@@ -455,6 +454,21 @@ int setup(sg_ctx* c) {
     }
     for (int f = 0; f < 3; ++f) c->leg_roots[f] = roots[f];
   }
+  if (!c->mixed)
+    for (int f = 0; f < 3; ++f) {
+      std::vector<LegWork> WF;
+      for (int r : roots[f]) {
+        const LegProblem& p = P[r];
+        const int n0 = p.next[0], n1 = n0 >= 0 ? p.next[1] : -1;
+        c->leg_elemsF[f] = std::max(
+            c->leg_elemsF[f], legendre_elems(p.J, p.K, n0 >= 0 ? P[n0].J : 0, n1 >= 0 ? P[n1].J : 0));
+        for (int m = 0; m < p.M; ++m)
+          for (int q0 = 0; q0 < p.Q; q0 += 32) WF.push_back(LegWork{r, m, q0, n0, n1});
+      }
+      c->nlwF[f] = (int)WF.size();
+      SG_TRY(upload(c, tmp, WF), "work");
+      c->d_lwF[f] = (LegWork*)tmp;
+    }
   // tensor-core operands: the three bf16 parts of every problem's table, and
   // work lists of 128-row tiles of the root problems (FP32 data only)
   if (c->mixed) {
@@ -518,7 +532,7 @@ int setup(sg_ctx* c) {
     for (size_t q = 0; q < 8 * c->groups.size(); ++q)
       c->fused_cf = std::max(c->fused_cf, (size_t)P[q].rpc * P[q].M * P[q].K);
   }
-  for (int s = 0; s < 6; ++s) {
+  for (int s = 0; s < 6 && c->mixed; ++s) {
     c->nlw[s] = (int)W[s].size();
     SG_TRY(upload(c, tmp, W[s]), "work");
     c->d_lw[s] = (LegWork*)tmp;
@@ -603,9 +617,16 @@ int dev_legendre(sg_ctx* c, int s) {
            "legendre (tensor cores)");
     SG_RET(con_mark(c, 1));
     c->launches += 1;
+  } else if (sizeof(T) == 8) {
+    if (s % 2) return SG_OK;
+    const int f = s / 2;
+    SG_RET(con_mark(c, 0));
+    SG_TRY(launch_legendre<T>(c->d_probs, c->d_lwF[f], c->nlwF[f], c->leg_elemsF[f], c->st), "legendre");
+    SG_RET(con_mark(c, 1));
+    c->launches += 1;
   } else {
     SG_RET(con_mark(c, 0));
-    SG_TRY(launch_legendre<T>(c->d_probs, c->d_lw[s], c->nlw[s], c->maxJ[s], c->maxK[s], c->st), "legendre");
+    SG_TRY(launch_legendre<T>(c->d_probs, c->d_lw[s], c->nlw[s], c->leg_elems[s], c->st), "legendre");
     SG_RET(con_mark(c, 1));
     c->launches += 1;
   }
@@ -641,7 +662,7 @@ int dev_forces(sg_ctx* c, const double* X, const double* Y, const double* Z, T* 
                                  c->st),
              "legendre (bending)");
     else
-      SG_TRY(launch_legendre<T>(c->d_probs, c->d_lwB, c->nlwB, c->maxJB, c->maxKB, c->st), "legendre (bending)");
+      SG_TRY(launch_legendre<T>(c->d_probs, c->d_lwB, c->nlwB, c->leg_elemsB, c->st), "legendre (bending)");
     SG_RET(con_mark(c, 1));
     c->launches += 1;
     SG_TRY(launch_membrane_bend<T>(c->d_wmem, c->nwmem, c->d_caps, c->d_groups, f32 ? sur_flags(c) : nullptr,
@@ -1530,11 +1551,12 @@ int sg_contraction_work(const sg_ctx* c, double* out) {
     }
     out[2] = 3;
   } else {
-    // CUDA-core path: the six stages over every problem of the context
-    // (the tensor-core split problems appended after them are not launched)
-    const size_t nplain = c->h_probs.size() - (c->mixed ? 2 * c->groups.size() : 0);
-    for (size_t i = 0; i < nplain; ++i) out[0] += useful(c->h_probs[i]);
-    out[2] = 6;
+    // CUDA-core path: every problem of the context but the halves of S2
+    // (the eight stage problems of each group come first, then the halves)
+    const size_t ng = c->groups.size();
+    for (size_t i = 0; i < c->h_probs.size(); ++i)
+      if (i < 8 * ng || i >= 10 * ng) out[0] += useful(c->h_probs[i]);
+    out[2] = c->mixed ? 6 : 3;
   }
   return SG_OK;
 }

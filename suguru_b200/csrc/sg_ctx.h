@@ -57,9 +57,10 @@ struct sg_ctx {
   bool wall_set = false, wall_in_step = false;
   sg::WallParams wall{};
   LegProblem* d_probs = nullptr;
-  LegWork* d_lw[6] = {};
+  LegWork* d_lw[6] = {};      // CUDA-core stages one by one (FP32 fallback)
   int nlw[6] = {};
-  int maxJ[6] = {}, maxK[6] = {};
+  size_t leg_elems[6] = {};   // their shared-memory elements
+  size_t leg_elemsF[3] = {};  // and those of the three chained FP64 launches
   // tensor-core Legendre path (mixed precision): 128-row work lists
   bool leg_tc = false;
   // fused force stage (mixed path): one CTA per capsule runs every stage
@@ -72,7 +73,9 @@ struct sg_ctx {
   int leg_terms = 0;
   int leg_parts = 2;                  // bf16 parts staged per operand (3 if any group is BF16x6)
   std::vector<LegProblem> h_probs;    // host copy of d_probs (the split mode is rewritten in place)
-  LegWork* d_lwF[3] = {};  // root work items of the three chained launches (tiles of tmF rows)
+  // root work items of the three chained launches (tiles of tmF rows; FP64: of
+  // 32 rows, on CUDA cores)
+  LegWork* d_lwF[3] = {};
   int nlwF[3] = {};
   LegWork* d_lwT[2][3] = {};  // the work items on 128-row [0] and 64-row [1] tiles
   int nlwT[2][3] = {};
@@ -120,13 +123,14 @@ struct sg_ctx {
   static constexpr int kMaxContract = 8;
   cudaEvent_t ev_con[2][kMaxContract] = {};
   int ncon = 0;
-  std::vector<int> leg_roots[3];  // root problems of the three tensor-core launches
+  std::vector<int> leg_roots[3];  // root problems of the three chained launches
   // bending (sg_set_capsule_bending): the synthesis of the third and fourth
   // theta derivatives, one problem per group, as its own contraction launch
   bool bend = false;        // some capsule has a nonzero bending modulus
   bool bend_ready = false;  // tables, buffers and problems set up
   LegWork* d_lwB = nullptr;   // CUDA-core work list (32-row tiles)
-  int nlwB = 0, maxJB = 0, maxKB = 0;
+  int nlwB = 0;
+  size_t leg_elemsB = 0;
   LegWork* d_lwBT = nullptr;  // tensor-core work list (128-row tiles)
   int nlwBT = 0;
   LegLevels lvB{};

@@ -121,19 +121,22 @@ struct LegProblem {
   int terms;     // split products: 3 (BF16x3) or 6 (BF16x6)
   int vecA;      // A rows 16-byte aligned with K % 8 == 0: float4 loads
   int vecD;      // D rows 16-byte aligned with J % 4 == 0: float4 stores
-  int next[2];   // tensor-core path: problems whose A operand is this problem's output (-1: none)
+  int next[2];   // chained launches: problems whose A operand is this problem's output (-1: none)
 };
 
 struct LegWork {  // one tile of a problem
   int prob, m, q0;
-  // tensor-core path: the root's chained problems (its next[0], then next[1]
+  // chained launches: the root's chained problems (its next[0], then next[1]
   // after a next[0]), -1 for none -- carried here so that a CTA can fetch the
   // whole chain at once
   int lvl1 = -1, lvl2 = -1;
 };
 
+// CUDA-core contractions: tiles of 32 data rows (LegWork.q0), each with its
+// chain; elems: the largest legendre_elems over the chains of the launch.
+size_t legendre_elems(int J, int K, int J1, int J2);
 template <class T>
-cudaError_t launch_legendre(const LegProblem* d_probs, const LegWork* d_work, int nwork, int maxJ, int maxK,
+cudaError_t launch_legendre(const LegProblem* d_probs, const LegWork* d_work, int nwork, size_t elems,
                             cudaStream_t st);
 // Shared-memory sizes of one tensor-core launch: for each chain level (0 the
 // root problems, 1 their next[0], 2 their next[1]) the largest padded J and K

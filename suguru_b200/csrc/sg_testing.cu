@@ -81,7 +81,8 @@ extern "C" int sg_test_legendre(int tensor_cores, int M, int Q, int J, int K, in
         ok(launch_legendre_mma((const LegProblem*)dP, (const LegWork*)dW, (int)work.size(), lv, terms == 6 ? 3 : 2,
                                tm, (int*)dE, sms, 0));
       } else {
-        ok(launch_legendre<float>((const LegProblem*)dP, (const LegWork*)dW, (int)work.size(), J, K, 0));
+        ok(launch_legendre<float>((const LegProblem*)dP, (const LegWork*)dW, (int)work.size(), legendre_elems(J, K, 0, 0),
+                                  0));
       }
       int err = 0;
       if (ok(cudaDeviceSynchronize()) && ok(cudaMemcpy(&err, dE, sizeof(int), cudaMemcpyDeviceToHost)) &&
