@@ -17,7 +17,7 @@
 namespace sg {
 
 // Spreading tile shapes (cells).  FP64 spreading takes shapes of at most 1024
-// cells (three 32-bit limbs per cell and component in static shared memory).
+// cells (two 32-bit limbs per cell and component in static shared memory).
 // TX = 0 stands for whole x rows (TX = itot): FP32 row tiles, whose fixed-point
 // sums take 3 (itot TY TZ + 32) words of dynamic shared memory, at most
 // kRowTileSmemMax bytes.
@@ -37,15 +37,8 @@ struct IBGrid {
   int TX, TY, TZ;        // tile shape
   int ntx, nty, ntz;     // tiles per dimension
   int ntiles;
-};
-
-// Per point after binning: base face index b = floor(c) per dimension (x, y
-// wrapped into [0, n), z raw) and the fractional offsets c - b.
-struct PointBins {
-  int* bx;
-  int* by;
-  int* bz;
-  int* tile;
+  int sx, sy, sz;        // log2 of the tile shape (x rows: 31, every cell in tile 0)
+  double rx, ry;         // 1 / itot, 1 / jtot
 };
 
 }  // namespace sg
