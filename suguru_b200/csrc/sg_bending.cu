@@ -426,19 +426,18 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 2 : 1) membrane_bend_ker
             Gm.d22[c] = acc[4][c];
           }
           T f[3] = {T(0), T(0), T(0)};
-          geometry<T>(Gm);
+          if (normals_only || eb != T(0)) geometry<T>(Gm);
           if (!normals_only) {
-            const T iR2 = fdiv(T(1), R * R);
-            T A[3] = {iR2, fdiv(iR2, st * st), T(0)};
-            T Ad[2][3] = {{T(0), fdiv(-T(2) * ct * iR2, st * st * st), T(0)}, {T(0), T(0), T(0)}};
+            membrane_force<T>(Gm.a1, Gm.a2, Gm.d11, Gm.d12, Gm.d22, RefSphere<T>(R, st, ct), hf, csk, ci.law, Gm.n, f);
             if (eb != T(0)) {
               BendT<T> B;
               bend_tensors<T>(Gm, (const T(*)[3]) & acc[5][0], (const T(*)[3]) & acc[9][0], B);
               T bq[7];
               bend_q<T>(Gm, B, R, st, ct, eb, bq);
-              mechanics<T>(Gm, A, Ad, hf, csk, ci.law, f, bq);
-            } else {
-              mechanics<T>(Gm, A, Ad, hf, csk, ci.law, f);
+              // q1 -= bm(1,1) Q1 + bm(2,1) Q2, q2 likewise, q3 += Qcode (sph.f90:1705-1709)
+              const T p1 = bq[0] * bq[4] + bq[1] * bq[5], p2 = bq[2] * bq[4] + bq[3] * bq[5];
+#pragma unroll
+              for (int c = 0; c < 3; ++c) f[c] += bq[6] * Gm.n[c] - p1 * Gm.a1[c] - p2 * Gm.a2[c];
             }
           }
           T* o = sOut + r * 6 * mD;

@@ -161,9 +161,9 @@ __device__ __forceinline__ void posfwd_item(const RowWork it,
           const long long p = ci.pt_off + (long long)i * mD + j;
           // the point half a turn on has cos p, sin p of opposite sign
           const double cp = trig64[1 * mD + j], sp = trig64[N * mD + 1 * mD + j];
-          const T ax = (T)(X[p] - c0 - R * (st * sp)), bx = (T)(X[p + H] - c0 + R * (st * sp));
-          const T ay = (T)(Y[p] - c1 - R * (st * cp)), by = (T)(Y[p + H] - c1 + R * (st * cp));
-          const T az = (T)(Z[p] - c2 - R * ct), bz = (T)(Z[p + H] - c2 - R * ct);
+          const T ax = (T)fma(-R, st * sp, X[p] - c0), bx = (T)fma(R, st * sp, X[p + H] - c0);
+          const T ay = (T)fma(-R, st * cp, Y[p] - c1), by = (T)fma(R, st * cp, Y[p + H] - c1);
+          const T az = (T)fma(-R, ct, Z[p] - c2), bz = (T)fma(-R, ct, Z[p + H] - c2);
           T* o = sd + r * 3 * lP;
           o[0 * lP + j] = ax + bx;
           o[0 * lP + hP + j] = ax - bx;
@@ -239,54 +239,36 @@ __device__ __forceinline__ void synth_m(const T* g, T cm, T sm, T fm, T (&acc)[5
   for (int c = 0; c < 3; ++c) {
     const T P_a = v[6 * c + 0], D_a = v[6 * c + 1], E_a = v[6 * c + 2];  // cos rows
     const T P_b = v[6 * c + 3], D_b = v[6 * c + 4], E_b = v[6 * c + 5];  // sin rows
-    const T t0P = P_a * cm - P_b * sm;
-    const T t1P = fm * (P_a * (-sm) - P_b * cm);
-    acc[0][c] += D_a * cm - D_b * sm;             // vat1 = sum dP * parthe0
-    acc[1][c] += t1P;                             // vat2 = sum P * parthe1
-    acc[2][c] += E_a * cm - E_b * sm;             // deFvat1(:,1) = sum d2P * parthe0
-    acc[3][c] += fm * (D_a * (-sm) - D_b * cm);   // deFvat1(:,2) = sum dP * parthe1
-    acc[4][c] += -fm * fm * t0P;                  // deFvat2(:,2) = sum P * parthe2
+    acc[0][c] = fma(D_a, cm, fma(-D_b, sm, acc[0][c]));           // vat1 = sum dP * parthe0
+    acc[1][c] = fma(-fm, fma(P_a, sm, P_b * cm), acc[1][c]);      // vat2 = sum P * parthe1
+    acc[2][c] = fma(E_a, cm, fma(-E_b, sm, acc[2][c]));           // deFvat1(:,1) = sum d2P * parthe0
+    acc[3][c] = fma(-fm, fma(D_a, sm, D_b * cm), acc[3][c]);      // deFvat1(:,2) = sum dP * parthe1
+    acc[4][c] = fma(-fm * fm, fma(P_a, cm, -(P_b * sm)), acc[4][c]);  // deFvat2(:,2) = sum P * parthe2
   }
 }
 
-// Geometry and Skalak force of one point from its synthesised sums v (the
+// Normal and membrane force of one point from its synthesised sums v (the
 // perturbation part) and the reference sphere at (st, ct, cp, sp).
 template <class T>
-__device__ __forceinline__ void point_force(const T (&v)[5][3], T st, T ct, T cp, T sp, T R, T hf, T csk,
-                                            int law, bool normals_only, T* f, T* nrm) {
-  Geo<T> Gm;
-  // reference sphere: a1 = x_t, a2 = x_p and second derivatives (sph.f90:84-86)
-  Gm.a1[0] = R * (ct * sp); Gm.a1[1] = R * (ct * cp); Gm.a1[2] = -R * st;
-  Gm.a2[0] = R * (st * cp); Gm.a2[1] = -R * (st * sp); Gm.a2[2] = T(0);
-  Gm.d11[0] = -R * (st * sp); Gm.d11[1] = -R * (st * cp); Gm.d11[2] = -R * ct;
-  Gm.d12[0] = R * (ct * cp); Gm.d12[1] = -R * (ct * sp); Gm.d12[2] = T(0);
-  Gm.d22[0] = -R * (st * sp); Gm.d22[1] = -R * (st * cp); Gm.d22[2] = T(0);
-#pragma unroll
-  for (int c = 0; c < 3; ++c) {
-    Gm.a1[c] += v[0][c];
-    Gm.a2[c] += v[1][c];
-    Gm.d11[c] += v[2][c];
-    Gm.d12[c] += v[3][c];
-    Gm.d22[c] += v[4][c];
-  }
-  f[0] = f[1] = f[2] = T(0);
+__device__ __forceinline__ void point_force(const T (&v)[5][3], T st, T ct, T cp, T sp, T R, const RefSphere<T>& S,
+                                            T hf, T csk, int law, bool normals_only, T* f, T* nrm) {
+  // the reference sphere's a1 = x_t, a2 = x_p and second derivatives
+  // (sph.f90:84-86) added to the sums, each by one fused multiply-add (as in
+  // membrane_force, so that the bits do not depend on what is around)
+  T a1[3] = {fma(R, ct * sp, v[0][0]), fma(R, ct * cp, v[0][1]), fma(-R, st, v[0][2])};
+  T a2[3] = {fma(R, st * cp, v[1][0]), fma(-R, st * sp, v[1][1]), v[1][2]};
+  T d11[3] = {fma(-R, st * sp, v[2][0]), fma(-R, st * cp, v[2][1]), fma(-R, ct, v[2][2])};
+  T d12[3] = {fma(R, ct * cp, v[3][0]), fma(-R, ct * sp, v[3][1]), v[3][2]};
+  T d22[3] = {fma(-R, st * sp, v[4][0]), fma(-R, st * cp, v[4][1]), v[4][2]};
   if (normals_only) {
+    f[0] = f[1] = f[2] = T(0);
     T cc[3];
-    cross3(Gm.a1, Gm.a2, cc);  // sph1.f90:611-651
+    cross3(a1, a2, cc);  // sph1.f90:611-651
     const T sm = sqrt(cc[0] * cc[0] + cc[1] * cc[1] + cc[2] * cc[2]);
-    for (int c = 0; c < 3; ++c) Gm.n[c] = fdiv(cc[c], sm);
+    for (int c = 0; c < 3; ++c) nrm[c] = fdiv(cc[c], sm);
   } else {
-    geometry<T>(Gm);
-    // reference contravariant metric of the sphere: A^11 = 1/R^2,
-    // A^22 = 1/(R^2 sin^2 t), d/dt A^22 = -2 cos t / (R^2 sin^3 t)
-    const T iR2 = fdiv(T(1), R * R);
-    T A[3] = {iR2, fdiv(iR2, st * st), T(0)};
-    T Ad[2][3] = {{T(0), fdiv(-T(2) * ct * iR2, st * st * st), T(0)}, {T(0), T(0), T(0)}};
-    mechanics<T>(Gm, A, Ad, hf, csk, law, f);
+    membrane_force<T>(a1, a2, d11, d12, d22, S, hf, csk, law, nrm, f);
   }
-  nrm[0] = Gm.n[0];
-  nrm[1] = Gm.n[1];
-  nrm[2] = Gm.n[2];
 }
 
 // One block per item of `nrows` dealias rows of one capsule.  Synthesises the
@@ -376,9 +358,10 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) membrane_kernel(c
             }
           const T st = lat[4 * i], ct = lat[4 * i + 1];
           const T cp = sTrig[1 * (H + 1) + j], sp = sTrig[(N + 1) * (H + 1) + j];
+          const RefSphere<T> S(R, st, ct);
           T fa[3], na[3], fb[3], nb[3];
-          point_force<T>(ev, st, ct, cp, sp, R, hf, csk, ci.law, normals_only, fa, na);
-          point_force<T>(od, st, ct, -cp, -sp, R, hf, csk, ci.law, normals_only, fb, nb);
+          point_force<T>(ev, st, ct, cp, sp, R, S, hf, csk, ci.law, normals_only, fa, na);
+          point_force<T>(od, st, ct, -cp, -sp, R, S, hf, csk, ci.law, normals_only, fb, nb);
           T* o = sOut + r * 6 * (2 * H + 2);
           const T va[6] = {fa[0], fa[1], fa[2], na[0], na[1], na[2]};
           const T vb[6] = {fb[0], fb[1], fb[2], nb[0], nb[1], nb[2]};
@@ -528,9 +511,10 @@ __device__ __forceinline__ void membrane_item_f2(const RowWork it,
             }
           const float st = lat[4 * i], ct = lat[4 * i + 1];
           const float cp = sTrig[1 * TS + j], sp = sTrig[(N + 1) * TS + j];
+          const RefSphere<float> S(R, st, ct);
           float fa[3], na[3], fb[3], nb[3];
-          point_force<float>(ev, st, ct, cp, sp, R, hf, csk, ci.law, normals_only, fa, na);
-          point_force<float>(od, st, ct, -cp, -sp, R, hf, csk, ci.law, normals_only, fb, nb);
+          point_force<float>(ev, st, ct, cp, sp, R, S, hf, csk, ci.law, normals_only, fa, na);
+          point_force<float>(od, st, ct, -cp, -sp, R, S, hf, csk, ci.law, normals_only, fb, nb);
           float* o = sOut + r * 6 * OS;
           const float va[6] = {fa[0], fa[1], fa[2], na[0], na[1], na[2]};
           const float vb[6] = {fb[0], fb[1], fb[2], nb[0], nb[1], nb[2]};
@@ -679,9 +663,9 @@ __device__ __forceinline__ void shgrid_item(const RowWork it,
           load18<T>(g + m * kSK, v);
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
-            acc[0][c] += v[6 * c + 0] * cm - v[6 * c + 1] * sm;
-            acc[1][c] += v[6 * c + 4] * cm - v[6 * c + 5] * sm;
-            acc[2][c] += (T)m * (v[6 * c + 2] * (-sm) - v[6 * c + 3] * cm);
+            acc[0][c] = fma(v[6 * c + 0], cm, fma(-v[6 * c + 1], sm, acc[0][c]));
+            acc[1][c] = fma(v[6 * c + 4], cm, fma(-v[6 * c + 5], sm, acc[1][c]));
+            acc[2][c] = fma((T)-m, fma(v[6 * c + 2], sm, v[6 * c + 3] * cm), acc[2][c]);
           }
         };
         for (int m = 0; m < N; m += 2) {
@@ -693,21 +677,27 @@ __device__ __forceinline__ void shgrid_item(const RowWork it,
 #pragma unroll
         for (int h = 0; h < 2; ++h) {  // h = 1: half a turn on (cos p, sin p change sign)
           const T sg = h ? T(-1) : T(1);
-          T nv[3], a1[3] = {R * (ct * (sg * sp)), R * (ct * (sg * cp)), -R * st},
-                   a2[3] = {R * (st * (sg * cp)), -R * (st * (sg * sp)), T(0)};
+          T nv[3], a1[3], a2[3], v1[3], v2[3];
 #pragma unroll
           for (int c = 0; c < 3; ++c) {
             nv[c] = h ? ev[0][c] - od[0][c] : ev[0][c] + od[0][c];
-            a1[c] += h ? ev[1][c] - od[1][c] : ev[1][c] + od[1][c];
-            a2[c] += h ? ev[2][c] - od[2][c] : ev[2][c] + od[2][c];
+            v1[c] = h ? ev[1][c] - od[1][c] : ev[1][c] + od[1][c];
+            v2[c] = h ? ev[2][c] - od[2][c] : ev[2][c] + od[2][c];
           }
-          const T rn = sqrt(nv[0] * nv[0] + nv[1] * nv[1] + nv[2] * nv[2]);
-          T cc[3];
-          cross3(a1, a2, cc);
+          // the reference sphere added (explicit fused multiply-adds, as in point_force)
+          a1[0] = fma(R, ct * (sg * sp), v1[0]);
+          a1[1] = fma(R, ct * (sg * cp), v1[1]);
+          a1[2] = fma(-R, st, v1[2]);
+          a2[0] = fma(R, st * (sg * cp), v2[0]);
+          a2[1] = fma(-R, st * (sg * sp), v2[1]);
+          a2[2] = v2[2];
+          const T rn = sqrt(dot3_fma(nv, nv));
+          const T cc[3] = {fma(a1[1], a2[2], -(a1[2] * a2[1])), fma(a1[2], a2[0], -(a1[0] * a2[2])),
+                           fma(a1[0], a2[1], -(a1[1] * a2[0]))};
           out[h][0] = fdiv(nv[0], rn);
           out[h][1] = fdiv(nv[1], rn);
           out[h][2] = fdiv(nv[2], rn);
-          out[h][3] = sqrt(cc[0] * cc[0] + cc[1] * cc[1] + cc[2] * cc[2]);
+          out[h][3] = sqrt(dot3_fma(cc, cc));
         }
         T* o = sOut + r * 4 * lP;
 #pragma unroll
@@ -814,7 +804,7 @@ __device__ __forceinline__ void final_item(const RowWork it,
             }
           }
 #pragma unroll
-          for (int f = 0; f < 7; ++f) acc[f] += v[2 * f] * cm - v[2 * f + 1] * sm;
+          for (int f = 0; f < 7; ++f) acc[f] = fma(v[2 * f], cm, fma(-v[2 * f + 1], sm, acc[f]));
         };
         for (int m = 0; m < N; m += 2) {
           term(m, ev);
