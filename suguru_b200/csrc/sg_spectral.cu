@@ -58,6 +58,122 @@ __device__ __forceinline__ void stage_trig(T* dst, int ts, const T* src, int ld,
     for (int hm = sm.e0; hm < nrow; hm += sm.es) dst[hm * ts + sm.r] = src[hm * ld + sm.r];
 }
 
+// The forward longitude DFTs of the pointwise kernels.  A row's values lie
+// as half-turn sums at [j] and differences at [HP + j] per field, the trig
+// rows p < 2N (cos m = p, then sin m = p - N) at stride TS; lane p sums its
+// trig row against the sums (even m) or the differences (odd m), 16 bytes of
+// each at a time: HP = H rounded up to whole vectors, zeros after H, and TS an
+// odd number of vectors, so that eight lanes' trig loads meet all banks.  The
+// data are broadcasts; with PAIR (FP32) the even and the odd j are two partial
+// sums in a packed pair, otherwise the sum runs over j in order.  The
+// results go through shared memory ([f 2N + p][row], an odd number of rows
+// apart) and out as runs of the chunk's rows: lanes that stored their own
+// result filled 4 bytes of 32 sectors at a time.  Together: membrane 35 -> 33,
+// posfwd 16 -> 14, shgrid 16 -> 15 us at 524,288 points in FP32, 194 -> 174,
+// 68 -> 64, 66 -> 54 us at 1.6 million; FP64 membrane 65 -> 57 us.
+template <class T>
+__host__ __device__ constexpr int dft_vec() {
+  return 16 / (int)sizeof(T);
+}
+template <class T>
+__host__ __device__ constexpr int dft_hp(int H) {
+  return (H + dft_vec<T>() - 1) / dft_vec<T>() * dft_vec<T>();
+}
+template <class T>
+__host__ __device__ constexpr int dft_ts(int H) {
+  return (dft_hp<T>(H) / dft_vec<T>() & 1) ? dft_hp<T>(H) : dft_hp<T>(H) + dft_vec<T>();
+}
+__host__ __device__ constexpr int dft_rows(int RP) { return RP | 1; }
+
+// F fields at o, o + os, ...; t: the lane's trig row
+template <class T, int F, bool PAIR>
+__device__ __forceinline__ void dft_lane(const T* o, int os, const T* t, int HP, T (&a)[F]) {
+  if constexpr (PAIR) {
+    float2 s[F];
+#pragma unroll
+    for (int f = 0; f < F; ++f) s[f] = make_float2(0.f, 0.f);
+#pragma unroll 2
+    for (int j = 0; j < HP; j += 4) {
+      const float4 w = *(const float4*)(t + j);
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        const float4 x = *(const float4*)(o + f * os + j);
+        s[f] = __ffma2_rn(make_float2(x.x, x.y), make_float2(w.x, w.y), s[f]);
+        s[f] = __ffma2_rn(make_float2(x.z, x.w), make_float2(w.z, w.w), s[f]);
+      }
+    }
+#pragma unroll
+    for (int f = 0; f < F; ++f) a[f] = s[f].x + s[f].y;
+  } else if constexpr (sizeof(T) == 4) {
+#pragma unroll
+    for (int f = 0; f < F; ++f) a[f] = T(0);
+#pragma unroll 2
+    for (int j = 0; j < HP; j += 4) {
+      const float4 w = *(const float4*)(t + j);
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        const float4 x = *(const float4*)(o + f * os + j);
+        a[f] = fma(x.w, w.w, fma(x.z, w.z, fma(x.y, w.y, fma(x.x, w.x, a[f]))));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int f = 0; f < F; ++f) a[f] = T(0);
+#pragma unroll 2
+    for (int j = 0; j < HP; j += 2) {
+      const double2 w = *(const double2*)(t + j);
+#pragma unroll
+      for (int f = 0; f < F; ++f) {
+        const double2 x = *(const double2*)(o + f * os + j);
+        a[f] = fma(x.x, w.x, a[f]);
+        a[f] = fma(x.y, w.y, a[f]);
+      }
+    }
+  }
+}
+
+// The whole chunk: `rows` rows of NF fields in groups of F, lines of 2 HP
+// values at sOut + (row NF + field) 2 HP; results through sRes to
+// out[(field 2N + p) ld + row].
+template <class T, int NF, int F, bool PAIR>
+__device__ __forceinline__ void dft_chunk(const T* sOut, const T* sTrig, int N, int H, int rows, int RP, T* sRes,
+                                          T* out, int ld) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+  const int HP = dft_hp<T>(H), TS = dft_ts<T>(H), RS = dft_rows(RP);
+  const T sf = T(1) / T(H);  // 2 / nlon, H = nlon / 2
+  for (int line = warp; line < rows * (NF / F); line += nwarp) {
+    const int rr = line / (NF / F), f0 = F * (line - rr * (NF / F));
+    const T* o = sOut + (rr * NF + f0) * 2 * HP;
+    for (int p = lane; p < 2 * N; p += 32) {
+      const int m = p < N ? p : p - N;
+      T a[F];
+      dft_lane<T, F, PAIR>(o + ((m & 1) ? HP : 0), 2 * HP, sTrig + p * TS, HP, a);
+#pragma unroll
+      for (int f = 0; f < F; ++f) sRes[((f0 + f) * 2 * N + p) * RS + rr] = (p < N ? sf : -sf) * a[f];
+    }
+  }
+  __syncthreads();
+  const StageMap m = stage_map(RP);
+  if (m.on && m.r < rows)
+    for (int e = m.e0; e < NF * 2 * N; e += m.es) out[(long long)e * ld + m.r] = sRes[e * RS + m.r];
+}
+
+// Trig rows at the DFT's stride with zeros after H, and the zeros after H of
+// the chunk's lines (2 per row and field).
+template <class T>
+__device__ __forceinline__ void stage_dft(T* sTrig, const T* trig, int ld, int N, int H, T* sOut, int lines) {
+  const int HP = dft_hp<T>(H), TS = dft_ts<T>(H);
+  stage_trig<T>(sTrig, TS, trig, ld, 2 * N, H);
+  if (HP > H)
+    for (int q = threadIdx.x; q < (HP - H) * (2 * N + lines); q += blockDim.x) {
+      const int r = q / (HP - H), j = H + q - r * (HP - H);
+      if (r < 2 * N)
+        sTrig[r * TS + j] = T(0);
+      else
+        sOut[(r - 2 * N) * HP + j] = T(0);
+    }
+}
+
 // ------------------------------------------------- positions -> Fourier ---
 // Persistent CTAs over capsule row ranges; per item the half-turn trig table
 // (j < mD/2) is staged once, then rows are taken in chunks of blockDim/(mD/2):
@@ -134,14 +250,15 @@ __device__ __forceinline__ void posfwd_item(const RowWork it,
                                                      const double* __restrict__ Y, const double* __restrict__ Z,
                                                      const double* __restrict__ cen) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  const int tid = threadIdx.x;
   {
     const CapInfo ci = caps[it.cap];
     const GroupDev gd = groups[it.group];
-    const int N = gd.N, nD = gd.nD, mD = gd.mD, H = mD >> 1, hP = H + 1, lP = 2 * H + 2;
+    const int N = gd.N, nD = gd.nD, mD = gd.mD, H = mD >> 1, HP = dft_hp<T>(H);
     const int RP = (int)blockDim.x / H > 0 ? (int)blockDim.x / H : 1;
-    T* sTrig = (T*)smem_raw;       // [2N][H+1]
-    T* sd = sTrig + 2 * N * hP;    // [RP][3][2H+2]: pair sums at [j], differences at [H+1+j]
+    T* sTrig = (T*)smem_raw;                 // [2N][dft_ts]
+    T* sd = sTrig + 2 * N * dft_ts<T>(H);    // [RP][3][2 HP]: pair sums at [j], differences at [HP + j]
+    T* sRes = sd + RP * 6 * HP;              // [6N][dft_rows]
     const double* lat64 = (const double*)gd.latD[0];
     const double* trig64 = (const double*)gd.trigD[0];
     const T* trig = (const T*)gd.trigD[pidx<T>()];
@@ -149,7 +266,7 @@ __device__ __forceinline__ void posfwd_item(const RowWork it,
     const double c0 = cen[3 * it.cap], c1 = cen[3 * it.cap + 1], c2 = cen[3 * it.cap + 2];
     T* Fpos = (T*)gd.buf.Fpos + (long long)ci.gidx * 6 * N * nD;
     __syncthreads();  // the previous item's reads of shared memory are done
-    stage_trig<T>(sTrig, hP, trig, mD, 2 * N, H);
+    stage_dft<T>(sTrig, trig, mD, N, H, sd, RP * 6);
     for (int rb = it.row0; rb < it.row0 + it.nrows; rb += RP) {
       const int rows = min(RP, it.row0 + it.nrows - rb);
       __syncthreads();
@@ -164,37 +281,18 @@ __device__ __forceinline__ void posfwd_item(const RowWork it,
           const T ax = (T)fma(-R, st * sp, X[p] - c0), bx = (T)fma(R, st * sp, X[p + H] - c0);
           const T ay = (T)fma(-R, st * cp, Y[p] - c1), by = (T)fma(R, st * cp, Y[p + H] - c1);
           const T az = (T)fma(-R, ct, Z[p] - c2), bz = (T)fma(-R, ct, Z[p + H] - c2);
-          T* o = sd + r * 3 * lP;
-          o[0 * lP + j] = ax + bx;
-          o[0 * lP + hP + j] = ax - bx;
-          o[1 * lP + j] = ay + by;
-          o[1 * lP + hP + j] = ay - by;
-          o[2 * lP + j] = az + bz;
-          o[2 * lP + hP + j] = az - bz;
+          T* o = sd + r * 6 * HP;
+          o[0 * HP + j] = ax + bx;
+          o[1 * HP + j] = ax - bx;
+          o[2 * HP + j] = ay + by;
+          o[3 * HP + j] = ay - by;
+          o[4 * HP + j] = az + bz;
+          o[5 * HP + j] = az - bz;
         }
       }
       __syncthreads();
-      const T sfn = T(2) / T(mD);
-      // lane p < 2N: trig row p (cos m = p, then sin m = p - N); rows of
-      // Fpos are (comp, cos/sin, m), so the output row is c 2N + p
-      // one warp per row: one load of the lane's trig value serves the three
-      // components
-      for (int r = warp; r < rows; r += nwarp) {
-        const T* o = sd + r * 3 * lP;
-        for (int p = lane; p < 2 * N; p += 32) {
-          const int m = p < N ? p : p - N;
-          const T* oo = o + ((m & 1) ? hP : 0);
-          const T* t = sTrig + p * hP;
-          T a[3] = {T(0), T(0), T(0)};
-          for (int j = 0; j < H; ++j) {
-            const T tt = t[j];
-#pragma unroll
-            for (int c = 0; c < 3; ++c) a[c] += oo[c * lP + j] * tt;
-          }
-#pragma unroll
-          for (int c = 0; c < 3; ++c) Fpos[(long long)(c * 2 * N + p) * nD + rb + r] = (p < N ? sfn : -sfn) * a[c];
-        }
-      }
+      // rows of Fpos are (comp, cos/sin, m): c 2N + p
+      dft_chunk<T, 3, 3, false>(sd, sTrig, N, H, rows, RP, sRes, Fpos + rb, nD);
     }
   }
 }
@@ -295,7 +393,7 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) membrane_kernel(c
   pdl_enter();
   (void)err;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  const int tid = threadIdx.x;
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
     const RowWork it = work[w];
     const CapInfo ci = caps[it.cap];
@@ -306,17 +404,17 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) membrane_kernel(c
     const int RP = (int)blockDim.x / H > 0 ? (int)blockDim.x / H : 1;  // rows per chunk, H threads each
     const int SR = N * kGK + 16 / (int)sizeof(T);  // staged row stride (one 16-byte pad: fewer bank conflicts)
     T* sG = (T*)smem_raw;                  // [RP][SR]
-    T* sTrig = sG + RP * SR;               // [2N][H+1]: cos m phi_j (rows m), sin m phi_j (rows N+m), j < H
-    T* sOut = sTrig + 2 * N * (H + 1);     // [RP][6][2H+2]: sum over the half turn at [j], difference at [H+1+j]
-    int* sOff = (int*)(sOut + RP * 6 * (2 * H + 2));  // [18N] staged offset of element e
+    const int HP = dft_hp<T>(H), TS = dft_ts<T>(H);
+    T* sTrig = sG + RP * SR;               // [2N][TS]: cos m phi_j (rows m), sin m phi_j (rows N+m), j < H
+    T* sOut = sTrig + 2 * N * TS;          // [RP][6][2 HP]: sum over the half turn at [j], difference at [HP + j]
+    int* sOff = (int*)(sOut + RP * 12 * HP);  // [18N] staged offset of element e
     const T* G = (const T*)gd.buf.G + (long long)ci.gidx * (18 * N * nD);  // [ccs][m][kind][lat]
     const T* trig = (const T*)gd.trigD[pidx<T>()];
     const T* lat = (const T*)gd.latD[pidx<T>()];
     T* Fout = (T*)gd.buf.Fout + (long long)ci.gidx * 12 * N * nD;
-    const T sfn = T(2) / T(mD);
     const T R = (T)ci.R;
     __syncthreads();  // the previous item's reads of shared memory are done
-    stage_trig<T>(sTrig, H + 1, trig, mD, 2 * N, H);
+    stage_dft<T>(sTrig, trig, mD, N, H, sOut, RP * 12);
     for (int e = tid; e < 18 * N; e += blockDim.x) {  // e = (ccs N + m) 3 + kind
       const int kind = e % 3, cm_ = e / 3, m = cm_ % N, ccs = cm_ / N;
       sOff[e] = m * kGK + 3 * ccs + kind;
@@ -342,10 +440,9 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) membrane_kernel(c
             for (int c = 0; c < 3; ++c) ev[a][c] = od[a][c] = T(0);
           const T* g = sG + r * SR;
           for (int m = 0; m < N; m += 2) {
-            synth_m<T>(g + m * kGK, sTrig[m * (H + 1) + j], sTrig[(N + m) * (H + 1) + j], (T)m, ev);
+            synth_m<T>(g + m * kGK, sTrig[m * TS + j], sTrig[(N + m) * TS + j], (T)m, ev);
             if (m + 1 < N)
-              synth_m<T>(g + (m + 1) * kGK, sTrig[(m + 1) * (H + 1) + j], sTrig[(N + m + 1) * (H + 1) + j],
-                         (T)(m + 1), od);
+              synth_m<T>(g + (m + 1) * kGK, sTrig[(m + 1) * TS + j], sTrig[(N + m + 1) * TS + j], (T)(m + 1), od);
           }
           // point j = even + odd, point j + mD/2 = even - odd
 #pragma unroll
@@ -357,36 +454,25 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) membrane_kernel(c
               od[a][c] = e - od[a][c];
             }
           const T st = lat[4 * i], ct = lat[4 * i + 1];
-          const T cp = sTrig[1 * (H + 1) + j], sp = sTrig[(N + 1) * (H + 1) + j];
+          const T cp = sTrig[1 * TS + j], sp = sTrig[(N + 1) * TS + j];
           const RefSphere<T> S(R, st, ct);
           T fa[3], na[3], fb[3], nb[3];
           point_force<T>(ev, st, ct, cp, sp, R, S, hf, csk, ci.law, normals_only, fa, na);
           point_force<T>(od, st, ct, -cp, -sp, R, S, hf, csk, ci.law, normals_only, fb, nb);
-          T* o = sOut + r * 6 * (2 * H + 2);
+          T* o = sOut + r * 12 * HP;
           const T va[6] = {fa[0], fa[1], fa[2], na[0], na[1], na[2]};
           const T vb[6] = {fb[0], fb[1], fb[2], nb[0], nb[1], nb[2]};
 #pragma unroll
           for (int f = 0; f < 6; ++f) {
-            o[f * (2 * H + 2) + j] = va[f] + vb[f];
-            o[f * (2 * H + 2) + H + 1 + j] = va[f] - vb[f];
+            o[2 * f * HP + j] = va[f] + vb[f];
+            o[(2 * f + 1) * HP + j] = va[f] - vb[f];
           }
         }
       }
       __syncthreads();
-      // forward DFT of the six outputs (force, normal) per row: warp =
-      // (row, field) line, lane p < 2N = trig row p (cos m = p, sin m = p - N)
-      for (int line = warp; line < rows * 6; line += nwarp) {
-        const int f = line % 6, rr = line / 6;
-        const T* o = sOut + line * (2 * H + 2);
-        for (int p = lane; p < 2 * N; p += 32) {
-          const int m = p < N ? p : p - N;
-          const T* oo = o + ((m & 1) ? H + 1 : 0);
-          const T* t = sTrig + p * (H + 1);
-          T a = 0;
-          for (int jj = 0; jj < H; ++jj) a += oo[jj] * t[jj];
-          Fout[((long long)f * 2 * N + p) * nD + rb + rr] = (p < N ? sfn : -sfn) * a;
-        }
-      }
+      // forward DFT of the six outputs (force, normal) per row; the staged
+      // rows are consumed, their memory takes the results
+      dft_chunk<T, 6, 3, false>(sOut, sTrig, N, H, rows, RP, sG, Fout + rb, nD);
     }
   }
 }
@@ -396,8 +482,8 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 3 : 2) membrane_kernel(c
 // on packed pairs (sm_100 f32x2 arithmetic: __ffma2_rn and friends compute
 // each lane as an IEEE FP32 operation).  In the synthesis the pair is
 // (even m, odd m): the two half-turn sums of membrane_kernel take one
-// instruction per operation.  In the forward DFT it is (even j, odd j): two
-// partial sums, added at the end.  Staging keeps a pair's 18 values
+// instruction per operation.  In the forward DFT (dft_lane) it is (even j,
+// odd j): two partial sums, added at the end.  Staging keeps a pair's 18 values
 // interleaved, [m pair][k][m parity], and the trig table of the synthesis
 // holds (cos m, cos m+1, sin m, sin m+1) per point, so that a thread reads
 // its operands with 16-byte loads; an odd N pads the last pair with zeros.
@@ -435,7 +521,7 @@ __device__ __forceinline__ void membrane_item_f2(const RowWork it,
                                                              const int* __restrict__ sur_flag, int* __restrict__ err) {
   (void)err;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  const int tid = threadIdx.x;
   {
     const CapInfo ci = caps[it.cap];
     const float hf = (float)(0.5 * ci.gs), csk = (float)ci.csk;  // hf_gscell = 0.5 gscell (sph.f90:35)
@@ -444,18 +530,16 @@ __device__ __forceinline__ void membrane_item_f2(const RowWork it,
     const int N = gd.N, nD = gd.nD, mD = gd.mD, H = mD >> 1, NP = (N + 1) >> 1;
     const int RP = (int)blockDim.x / H > 0 ? (int)blockDim.x / H : 1;  // rows per chunk, H threads each
     const int SR = NP * kGP + 4;      // staged row stride (one 16-byte pad)
-    const int TS = H + 2;             // row stride of the DFT trig table (8-byte aligned rows)
-    const int OS = 2 * H + 4;         // output line: half-turn sums at [j], differences at [H + 2 + j]
+    const int HP = dft_hp<float>(H), TS = dft_ts<float>(H);
     float* sG = (float*)smem_raw;                       // [RP][SR]
     float4* sTP = (float4*)(sG + RP * SR);              // [NP][H]
     float* sTrig = (float*)(sTP + NP * H);              // [2N][TS]: cos m phi_j (rows m), sin (rows N + m)
-    float* sOut = sTrig + 2 * N * TS;                   // [RP][6][OS]
-    int* sOff = (int*)(sOut + RP * 6 * OS);              // [18N] staged offset of element e
+    float* sOut = sTrig + 2 * N * TS;                   // [RP][6][2 HP]: half-turn sums, then differences
+    int* sOff = (int*)(sOut + RP * 12 * HP);             // [18N] staged offset of element e
     const float* G = (const float*)gd.buf.G + (long long)ci.gidx * (18 * N * nD);  // [ccs][m][kind][lat]
     const float* trig = (const float*)gd.trigD[1];
     const float* lat = (const float*)gd.latD[1];
     float* Fout = (float*)gd.buf.Fout + (long long)ci.gidx * 12 * N * nD;
-    const float sfn = 2.0f / (float)mD;
     const float R = (float)ci.R;
     __syncthreads();  // the previous item's reads of shared memory are done
     {
@@ -468,7 +552,7 @@ __device__ __forceinline__ void membrane_item_f2(const RowWork it,
                                         trig[(N + m) * mD + j], odd ? trig[(N + m + 1) * mD + j] : 0.0f);
         }
     }
-    stage_trig<float>(sTrig, TS, trig, mD, 2 * N, H);
+    stage_dft<float>(sTrig, trig, mD, N, H, sOut, RP * 12);
     for (int e = tid; e < 18 * N; e += blockDim.x) {  // e = (ccs N + m) 3 + kind
       const int kind = e % 3, cm_ = e / 3, m = cm_ % N, ccs = cm_ / N;
       sOff[e] = (m >> 1) * kGP + 2 * (3 * ccs + kind) + (m & 1);
@@ -515,39 +599,20 @@ __device__ __forceinline__ void membrane_item_f2(const RowWork it,
           float fa[3], na[3], fb[3], nb[3];
           point_force<float>(ev, st, ct, cp, sp, R, S, hf, csk, ci.law, normals_only, fa, na);
           point_force<float>(od, st, ct, -cp, -sp, R, S, hf, csk, ci.law, normals_only, fb, nb);
-          float* o = sOut + r * 6 * OS;
+          float* o = sOut + r * 12 * HP;
           const float va[6] = {fa[0], fa[1], fa[2], na[0], na[1], na[2]};
           const float vb[6] = {fb[0], fb[1], fb[2], nb[0], nb[1], nb[2]};
 #pragma unroll
           for (int f = 0; f < 6; ++f) {
-            o[f * OS + j] = va[f] + vb[f];
-            o[f * OS + H + 2 + j] = va[f] - vb[f];
+            o[2 * f * HP + j] = va[f] + vb[f];
+            o[(2 * f + 1) * HP + j] = va[f] - vb[f];
           }
         }
       }
       __syncthreads();
-      // forward DFT of the six outputs per row: warp = (row, field triple)
-      // line, lane p < 2N = trig row p (cos m = p, sin m = p - N); even and
-      // odd j summed as a pair; one load of the lane's trig pair serves the
-      // triple's three fields (force or normal)
-      for (int line = warp; line < rows * 2; line += nwarp) {
-        const int f0 = 3 * (line & 1), rr = line >> 1;
-        const float* o = sOut + (rr * 6 + f0) * OS;
-        for (int p = lane; p < 2 * N; p += 32) {
-          const int m = p < N ? p : p - N;
-          const float2* oo = (const float2*)(o + ((m & 1) ? H + 2 : 0));
-          const float2* t = (const float2*)(sTrig + p * TS);
-          float2 a2[3] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
-          for (int jj = 0; jj < (H >> 1); ++jj) {
-            const float2 tt = t[jj];
-#pragma unroll
-            for (int f = 0; f < 3; ++f) a2[f] = p2fma(oo[f * (OS >> 1) + jj], tt, a2[f]);
-          }
-#pragma unroll
-          for (int f = 0; f < 3; ++f)
-            Fout[((long long)(f0 + f) * 2 * N + p) * nD + rb + rr] = (p < N ? sfn : -sfn) * (a2[f].x + a2[f].y);
-        }
-      }
+      // forward DFT of the six outputs (force, normal) per row; the staged
+      // rows are consumed, their memory takes the results
+      dft_chunk<float, 6, 3, true>(sOut, sTrig, N, H, rows, RP, sG, Fout + rb, nD);
     }
   }
 }
@@ -563,13 +628,14 @@ __global__ void __launch_bounds__(256, 3) membrane_kernel_f2(const RowWork* __re
 // Shared memory (bytes) of membrane_kernel_f2 for degrees up to nmax: the
 // largest over n <= nmax of staged rows RP (NP kGP + 4), the staging offsets
 // 18n, the pair trig table
-// NP H float4, the DFT trig table 2n (H + 2) and outputs RP 6 (2H + 4), with
+// NP H float4, the DFT trig table 2n dft_ts and outputs RP 12 dft_hp, with
 // H = 2n, NP = ceil(n / 2) and RP = max(1, 256 / H).
 static size_t membrane_f2_smem(int nmax) {
   size_t e = 0;
   for (size_t n = 1; n <= (size_t)nmax; ++n) {
     const size_t H = 2 * n, NP = (n + 1) / 2, RP = 256 / H > 0 ? 256 / H : 1;
-    const size_t en = RP * (NP * kGP + 4) + NP * H * 4 + 2 * n * (H + 2) + RP * 6 * (2 * H + 4) + 18 * n + 64;
+    const size_t en = RP * (NP * kGP + 4) + NP * H * 4 + 2 * n * dft_ts<float>((int)H) +
+                      RP * 12 * dft_hp<float>((int)H) + 18 * n + 64;
     if (en > e) e = en;
   }
   return sizeof(float) * e;
@@ -611,25 +677,24 @@ __device__ __forceinline__ void shgrid_item(const RowWork it,
                                                      const GroupDev* __restrict__ groups, int* __restrict__ err) {
   (void)err;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarp = blockDim.x >> 5;
+  const int tid = threadIdx.x;
   {
     const CapInfo ci = caps[it.cap];
     const GroupDev gd = groups[it.group];
-    const int N = gd.N, nO = gd.nO, mO = gd.mO, H = mO >> 1, hP = H + 1, lP = 2 * H + 2;
+    const int N = gd.N, nO = gd.nO, mO = gd.mO, H = mO >> 1, HP = dft_hp<T>(H), TS = dft_ts<T>(H);
     const int RP = (int)blockDim.x / H > 0 ? (int)blockDim.x / H : 1;
     const int SR = N * kSK + 16 / (int)sizeof(T);
     T* sG = (T*)smem_raw;                 // [RP][SR]
-    T* sTrig = sG + RP * SR;              // [2N][H+1]
-    T* sOut = sTrig + 2 * N * hP;         // [RP][4][2H+2]
-    int* sOff = (int*)(sOut + RP * 4 * lP);  // [18N][2]: staged offset and source row of element e
+    T* sTrig = sG + RP * SR;              // [2N][TS]
+    T* sOut = sTrig + 2 * N * TS;         // [RP][4][2 HP]
+    int* sOff = (int*)(sOut + RP * 8 * HP);  // [18N][2]: staged offset and source row of element e
     const T* GO = (const T*)gd.buf.GO + (long long)ci.gidx * (24 * N * nO);  // [rr][m][kind][lat]
     const T* trig = (const T*)gd.trigO[pidx<T>()];
     const T* lat = (const T*)gd.latO[pidx<T>()];
     T* Fsh = (T*)gd.buf.Fsh + (long long)ci.gidx * 8 * N * nO;
-    const T sfn = T(2) / T(mO);
     const T R = (T)ci.R;
     __syncthreads();  // the previous item's reads of shared memory are done
-    stage_trig<T>(sTrig, hP, trig, mO, 2 * N, H);
+    stage_dft<T>(sTrig, trig, mO, N, H, sOut, RP * 8);
     // staged elements e = (s, c, cs, m) with s = 0 normal P (rr = 2c+cs,
     // kind 0), s = 1 shape P (rr = 2(3+c)+cs, kind 0), s = 2 shape dP (kind 1)
     for (int e = tid; e < 18 * N; e += blockDim.x) {
@@ -658,7 +723,7 @@ __device__ __forceinline__ void shgrid_item(const RowWork it,
           for (int c = 0; c < 3; ++c) ev[a2][c] = od[a2][c] = T(0);
         const T* g = sG + r * SR;
         auto term = [&](int m, T(&acc)[3][3]) {
-          const T cm = sTrig[m * hP + j], sm = sTrig[(N + m) * hP + j];
+          const T cm = sTrig[m * TS + j], sm = sTrig[(N + m) * TS + j];
           T v[18];
           load18<T>(g + m * kSK, v);
 #pragma unroll
@@ -672,7 +737,7 @@ __device__ __forceinline__ void shgrid_item(const RowWork it,
           term(m, ev);
           if (m + 1 < N) term(m + 1, od);
         }
-        const T cp = sTrig[1 * hP + j], sp = sTrig[(N + 1) * hP + j];
+        const T cp = sTrig[1 * TS + j], sp = sTrig[(N + 1) * TS + j];
         T out[2][4];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {  // h = 1: half a turn on (cos p, sin p change sign)
@@ -699,33 +764,15 @@ __device__ __forceinline__ void shgrid_item(const RowWork it,
           out[h][2] = fdiv(nv[2], rn);
           out[h][3] = sqrt(dot3_fma(cc, cc));
         }
-        T* o = sOut + r * 4 * lP;
+        T* o = sOut + r * 8 * HP;
 #pragma unroll
         for (int f = 0; f < 4; ++f) {
-          o[f * lP + j] = out[0][f] + out[1][f];
-          o[f * lP + hP + j] = out[0][f] - out[1][f];
+          o[2 * f * HP + j] = out[0][f] + out[1][f];
+          o[(2 * f + 1) * HP + j] = out[0][f] - out[1][f];
         }
       }
       __syncthreads();
-      // (row, field pair) line per warp: one load of the lane's trig value
-      // serves two fields
-      for (int line = warp; line < rows * 2; line += nwarp) {
-        const int f0 = 2 * (line & 1), rr = line >> 1;
-        const T* o = sOut + (rr * 4 + f0) * lP;
-        for (int p = lane; p < 2 * N; p += 32) {
-          const int m = p < N ? p : p - N;
-          const T* oo = o + ((m & 1) ? hP : 0);
-          const T* t = sTrig + p * hP;
-          T a[2] = {T(0), T(0)};
-          for (int jj = 0; jj < H; ++jj) {
-            const T tt = t[jj];
-            a[0] += oo[jj] * tt;
-            a[1] += oo[lP + jj] * tt;
-          }
-#pragma unroll
-          for (int f = 0; f < 2; ++f) Fsh[((long long)(f0 + f) * 2 * N + p) * nO + rb + rr] = (p < N ? sfn : -sfn) * a[f];
-        }
-      }
+      dft_chunk<T, 4, 4, false>(sOut, sTrig, N, H, rows, RP, sG, Fsh + rb, nO);
     }
   }
 }
@@ -973,31 +1020,32 @@ size_t pointwise_smem(int kind, int nmax) {
   size_t e = 0;
   switch (kind) {
     case kPosfwd:
-      // half-turn trig table 2n (2n + 1) and RP = max(1, 256 / 2n) rows of
-      // 3 (4n + 2) pair sums and differences, largest over n <= N
+      // half-turn trig table 2n dft_ts, RP = max(1, 256 / 2n) rows of 3 pair
+      // sums and differences, results 6n dft_rows, largest over n <= N
       for (size_t n = 1; n <= N; ++n) {
         const size_t RP = kPointThreads / (2 * n) > 0 ? kPointThreads / (2 * n) : 1;
-        const size_t en = 2 * n * (2 * n + 1) + RP * 3 * (4 * n + 2) + 64;
+        const size_t en = 2 * n * dft_ts<T>(2 * (int)n) + RP * 6 * dft_hp<T>(2 * (int)n) +
+                          6 * n * dft_rows((int)RP) + 64;
         if (en > e) e = en;
       }
       break;
     case kMembrane:
       // staged rows RP (n kGK + pad) with RP = max(1, 256 / 2n), 18n staging offsets, the half-turn
-      // trig table 2n (2n + 1), outputs RP 6 (4n + 2): the largest over the
+      // trig table 2n dft_ts, outputs RP 12 dft_hp: the largest over the
       // degrees n <= N (smaller degrees stage more rows per chunk)
       for (size_t n = 1; n <= N; ++n) {
         const size_t RP = kPointThreads / (2 * n) > 0 ? kPointThreads / (2 * n) : 1;
-        const size_t en = RP * (n * kGK + 16 / sizeof(T)) + 2 * n * (2 * n + 1) + RP * 6 * (4 * n + 2) +
-                          (18 * n * sizeof(int) + sizeof(T) - 1) / sizeof(T) + 64;
+        const size_t en = RP * (n * kGK + 16 / sizeof(T)) + 2 * n * dft_ts<T>(2 * (int)n) +
+                          RP * 12 * dft_hp<T>(2 * (int)n) + (18 * n * sizeof(int) + sizeof(T) - 1) / sizeof(T) + 64;
         if (en > e) e = en;
       }
       break;
     case kShgrid:
-      // staged rows RP (n kSK + pad) with RP = max(1, 256 / n), 36n staging offsets, trig 2n (n + 1),
-      // outputs RP 4 (2n + 2)
+      // staged rows RP (n kSK + pad) with RP = max(1, 256 / n), 36n staging offsets, trig 2n dft_ts,
+      // outputs RP 8 dft_hp
       for (size_t n = 1; n <= N; ++n) {
         const size_t RP = kPointThreads / n > 0 ? kPointThreads / n : 1;
-        const size_t en = RP * (n * kSK + 16 / sizeof(T)) + 2 * n * (n + 1) + RP * 4 * (2 * n + 2) +
+        const size_t en = RP * (n * kSK + 16 / sizeof(T)) + 2 * n * dft_ts<T>((int)n) + RP * 8 * dft_hp<T>((int)n) +
                           (36 * n * sizeof(int) + sizeof(T) - 1) / sizeof(T) + 64;
         if (en > e) e = en;
       }
