@@ -1,13 +1,8 @@
-// sg_mechanics.cuh -- pointwise geometry and membrane mechanics of one
-// surface point (device code shared by the spectral force kernels).
-//
-// sph1.f90:581-651 (unit normal and its derivatives), sph.f90:442-476
-// (curvature), sph1.f90:197-297 with co2contra (capsulesolid.f90:106-146:
-// contravariant basis and derivatives), sph.f90:735-893 (Christoffel
-// symbols), sph.f90:896-961 (metric tensors and derivatives), for the
-// bending terms, in the reference's operation order; and the membrane force
-// itself (cal_spectral_force's equilibrium, sph.f90:1668-1715) in the shorter
-// form of membrane_force.
+// sg_mechanics.cuh -- membrane mechanics of one surface point (device code
+// shared by the spectral force kernels): the membrane force of
+// cal_spectral_force (sph.f90:1668-1715 with sph1.f90:581-651, the unit
+// normal, and the laws of membmodel.c) and the bending force added by
+// ibend = 1.
 #pragma once
 #include "sg_common.cuh"
 
@@ -24,88 +19,6 @@ __device__ __forceinline__ float fdiv<float>(float a, float b) {
 template <>
 __device__ __forceinline__ double fdiv<double>(double a, double b) {
   return a / b;
-}
-
-// ------------------------------------------------- geometry + mechanics ---
-// The geometry that the bending terms differentiate (sg_bending.cu).
-template <class T>
-struct Geo {
-  T a1[3], a2[3], d11[3], d12[3], d22[3];
-  T n[3];
-  T c1[3], c2[3];
-  T conat[3], conatd1[2][3], bcur[3], chf[8];
-  // derivatives of the unit normal and of the contravariant basis along
-  // xi^al (cderi3, conderi1, conderi2 of the reference)
-  T nde[2][3], cdc1[2][3], cdc2[2][3];
-};
-
-// sph1.f90:581-651 (normal), sph.f90:442-476 (curvature), sph1.f90:197-297
-// with co2contra (capsulesolid.f90:106-146), sph.f90:735-893 (christof),
-// sph.f90:896-961 (metrics).  Same operation order as the reference.
-template <class T>
-__device__ __forceinline__ void geometry(Geo<T>& G) {
-  const T* cd1[2] = {G.d11, G.d12};
-  const T* cd2[2] = {G.d12, G.d22};
-  T cc[3];
-  cross3(G.a1, G.a2, cc);
-  const T sm = sqrt(cc[0] * cc[0] + cc[1] * cc[1] + cc[2] * cc[2]);
-  for (int c = 0; c < 3; ++c) G.n[c] = fdiv(cc[c], sm);
-  T (&nde)[2][3] = G.nde;
-#pragma unroll
-  for (int al = 0; al < 2; ++al) {
-    T x1[3], x2[3], dc[3];
-    cross3(cd1[al], G.a2, x1);
-    cross3(G.a1, cd2[al], x2);
-    for (int c = 0; c < 3; ++c) dc[c] = x1[c] + x2[c];
-    const T tmp = fdiv(dot3(cc, dc), sqrt(cc[0] * cc[0] + cc[1] * cc[1] + cc[2] * cc[2]));
-    for (int c = 0; c < 3; ++c) nde[al][c] = fdiv(T(1), sm) * (x1[c] + x2[c] - tmp * G.n[c]);
-  }
-  G.bcur[0] = dot3(G.n, G.d11);
-  G.bcur[1] = dot3(G.n, G.d22);
-  G.bcur[2] = dot3(G.n, G.d12);
-  T a2n[3], na1[3];
-  cross3(G.a2, G.n, a2n);
-  cross3(G.n, G.a1, na1);
-  const T hyb1 = dot3(G.a1, a2n), hyb2 = dot3(G.a2, na1);
-  for (int c = 0; c < 3; ++c) {
-    G.c1[c] = fdiv(a2n[c], hyb1);
-    G.c2[c] = fdiv(na1[c], hyb2);
-  }
-  const T g = hyb1;
-  T (&cdc1)[2][3] = G.cdc1;
-  T (&cdc2)[2][3] = G.cdc2;
-#pragma unroll
-  for (int al = 0; al < 2; ++al) {
-    T a2de_n3[3], a2_n3de[3], n3de_a1[3], n3_a1de[3], vt[3];
-    cross3(cd2[al], G.n, a2de_n3);
-    cross3(G.a2, nde[al], a2_n3de);
-    cross3(nde[al], G.a1, n3de_a1);
-    cross3(G.n, cd1[al], n3_a1de);
-    for (int c = 0; c < 3; ++c) vt[c] = a2de_n3[c] + a2_n3de[c];
-    const T gde = dot3(cd1[al], a2n) + dot3(G.a1, vt);
-    for (int c = 0; c < 3; ++c) {
-      cdc1[al][c] = fdiv(T(1), g) * (-gde * G.c1[c] + a2de_n3[c] + a2_n3de[c]);
-      cdc2[al][c] = fdiv(T(1), g) * (-gde * G.c2[c] + n3de_a1[c] + n3_a1de[c]);
-    }
-  }
-  // christof(gamma,beta,alpha) at [(gamma-1) + 2(beta-1) + 4(alpha-1)]
-  G.chf[0 + 0 + 0] = dot3(G.d11, G.c1);  // (1,1,1)
-  G.chf[1 + 0 + 0] = dot3(G.d12, G.c1);  // (2,1,1)
-  G.chf[0 + 2 + 0] = dot3(G.d11, G.c2);  // (1,2,1)
-  G.chf[1 + 2 + 0] = dot3(G.d12, G.c2);  // (2,2,1)
-  G.chf[1 + 0 + 4] = dot3(G.d22, G.c1);  // (2,1,2)
-  G.chf[1 + 2 + 4] = dot3(G.d22, G.c2);  // (2,2,2)
-  G.chf[0 + 0 + 4] = G.chf[1];           // (1,1,2) = (2,1,1)
-  G.chf[0 + 2 + 4] = G.chf[3];           // (1,2,2) = (2,2,1)
-  G.conat[0] = G.c1[0] * G.c1[0] + G.c1[1] * G.c1[1] + G.c1[2] * G.c1[2];
-  G.conat[1] = G.c2[0] * G.c2[0] + G.c2[1] * G.c2[1] + G.c2[2] * G.c2[2];
-  G.conat[2] = dot3(G.c1, G.c2);
-#pragma unroll
-  for (int al = 0; al < 2; ++al) {
-    G.conatd1[al][0] = T(2) * dot3(G.c1, cdc1[al]);
-    G.conatd1[al][1] = T(2) * dot3(G.c2, cdc2[al]);
-    G.conatd1[al][2] = dot3(G.c1, cdc2[al]) + dot3(G.c2, cdc1[al]);
-  }
 }
 
 // The reference sphere of radius R at colatitude t (st = sin t, ct = cos t):
@@ -192,6 +105,116 @@ __device__ __forceinline__ void membrane_force(const T* a1, const T* a2, const T
   const T c2 = fma(gam[0], T12, fma(gam[1], T22, T12d1 + T22d2));
   for (int c = 0; c < 3; ++c)
     f[c] = fma(c1, a1[c], fma(c2, a2[c], fma(T11, d11[c], fma(T(2) * T12, d12[c], T22 * d22[c]))));
+}
+
+// The bending force of ibend = 1 (sph.f90:1705-1709), added to f.  The
+// reference forms the moment M^ba = eb a^bg (A^ga B_gg' - a^ga b_gg') with its
+// first and second derivatives (cal_moment_deri, sph.f90:1236-1372, from the
+// twice differentiated curvature, contravariant metric and Christoffel
+// symbols, sph.f90:479-1111, sph1.f90:299-542), its divergence Q^b = M^ab_|a
+// and Q^b_|b (cal_Q, :1375-1424), and adds Q^b_|b n - Q^b b_b^a a_a
+// (cal_bcurmix, :1427-1454).  On the sphere A^ga B_gg' is delta / R, so M^ba =
+// eb (a^ba / R - b^ba); the metric is covariantly constant and by Codazzi's
+// equations b^ab_|a = a^bg h_,g with h = a^ab b_ab, hence
+//   Q^b = -eb a^bg h_,g  and  f += -eb Lap(h) n + eb a^bg h_,g b_b^a a_a.
+// h = S / q^(3/2) with S = g22 L - 2 g12 M + g11 N, L, M, N = x_ab . m,
+// m = a1 x a2 and q = m . m: its value and five derivatives follow from
+// products, about 450 operations instead of 2,500 and no tensors to keep.
+// S3 = x_ttt, x_ttp, x_tpp, x_ppp; S4 = x_tttt, x_tttp, x_ttpp, x_tppp, x_pppp.
+template <class T>
+struct Jet2 {  // a function of (t, p): value and derivatives t, p, tt, tp, pp
+  T v, t, p, tt, tp, pp;
+};
+template <class T>
+__device__ __forceinline__ Jet2<T> operator*(const Jet2<T>& a, const Jet2<T>& b) {
+  return {a.v * b.v,
+          a.t * b.v + a.v * b.t,
+          a.p * b.v + a.v * b.p,
+          a.tt * b.v + T(2) * (a.t * b.t) + a.v * b.tt,
+          a.tp * b.v + a.t * b.p + a.p * b.t + a.v * b.tp,
+          a.pp * b.v + T(2) * (a.p * b.p) + a.v * b.pp};
+}
+
+template <class T>
+__device__ __forceinline__ void bending_force(const T* a1, const T* a2, const T* x11, const T* x12, const T* x22,
+                                              const T (*S3)[3], const T (*S4)[3], T eb, T* f) {
+  auto dot = [](const T* u, const T* v) { return dot3(u, v); };
+  T m[3], mt[3], mp[3], mtt[3], mtp[3], mpp[3];
+  {
+    T u[3], v[3], w[3];
+    cross3(a1, a2, m);
+    cross3(x11, a2, u);
+    cross3(a1, x12, v);
+    for (int c = 0; c < 3; ++c) mt[c] = u[c] + v[c];
+    cross3(x12, a2, u);
+    cross3(a1, x22, v);
+    for (int c = 0; c < 3; ++c) mp[c] = u[c] + v[c];
+    cross3(S3[0], a2, u);
+    cross3(x11, x12, v);
+    cross3(a1, S3[1], w);
+    for (int c = 0; c < 3; ++c) mtt[c] = u[c] + T(2) * v[c] + w[c];
+    cross3(S3[1], a2, u);
+    cross3(x11, x22, v);
+    cross3(a1, S3[2], w);
+    for (int c = 0; c < 3; ++c) mtp[c] = u[c] + v[c] + w[c];
+    cross3(S3[2], a2, u);
+    cross3(x12, x22, v);
+    cross3(a1, S3[3], w);
+    for (int c = 0; c < 3; ++c) mpp[c] = u[c] + T(2) * v[c] + w[c];
+  }
+  const T q = dot(m, m), iq = fdiv(T(1), q);
+  const T lt = T(2) * dot(m, mt) * iq, lp = T(2) * dot(m, mp) * iq;  // q_,t / q, q_,p / q
+  const T ltt = T(2) * (dot(mt, mt) + dot(m, mtt)) * iq, ltp = T(2) * (dot(mt, mp) + dot(m, mtp)) * iq,
+          lpp = T(2) * (dot(mp, mp) + dot(m, mpp)) * iq;
+  // x_ab . m with its derivatives, from x_ab and its derivatives
+  auto proj = [&](const T* x, const T* xt, const T* xp, const T* xtt, const T* xtp, const T* xpp) {
+    Jet2<T> j;
+    j.v = dot(x, m);
+    j.t = dot(xt, m) + dot(x, mt);
+    j.p = dot(xp, m) + dot(x, mp);
+    j.tt = dot(xtt, m) + T(2) * dot(xt, mt) + dot(x, mtt);
+    j.tp = dot(xtp, m) + dot(xt, mp) + dot(xp, mt) + dot(x, mtp);
+    j.pp = dot(xpp, m) + T(2) * dot(xp, mp) + dot(x, mpp);
+    return j;
+  };
+  const T x1212 = dot(x12, x12);
+  const T a1x111 = dot(a1, S3[0]), a1x112 = dot(a1, S3[1]), a1x122 = dot(a1, S3[2]), a1x222 = dot(a1, S3[3]);
+  const T a2x111 = dot(a2, S3[0]), a2x112 = dot(a2, S3[1]), a2x122 = dot(a2, S3[2]), a2x222 = dot(a2, S3[3]);
+  const T x1112 = dot(x11, x12), x1122 = dot(x11, x22), x1222 = dot(x12, x22);
+  const T a1x11 = dot(a1, x11), a1x12 = dot(a1, x12), a1x22 = dot(a1, x22);
+  const T a2x11 = dot(a2, x11), a2x12 = dot(a2, x12), a2x22 = dot(a2, x22);
+  const Jet2<T> g11 = {dot(a1, a1), T(2) * a1x11, T(2) * a1x12, T(2) * (dot(x11, x11) + a1x111),
+                       T(2) * (x1112 + a1x112), T(2) * (x1212 + a1x122)};
+  const Jet2<T> g22 = {dot(a2, a2), T(2) * a2x12, T(2) * a2x22, T(2) * (x1212 + a2x112), T(2) * (x1222 + a2x122),
+                       T(2) * (dot(x22, x22) + a2x222)};
+  // -2 g12
+  const Jet2<T> g12 = {-T(2) * dot(a1, a2),
+                       -T(2) * (a2x11 + a1x12),
+                       -T(2) * (a2x12 + a1x22),
+                       -T(2) * (a2x111 + T(2) * x1112 + a1x112),
+                       -T(2) * (a2x112 + x1122 + x1212 + a1x122),
+                       -T(2) * (a2x122 + T(2) * x1222 + a1x222)};
+  const Jet2<T> L = proj(x11, S3[0], S3[1], S4[0], S4[1], S4[2]);
+  const Jet2<T> M = proj(x12, S3[1], S3[2], S4[1], S4[2], S4[3]);
+  const Jet2<T> N = proj(x22, S3[2], S3[3], S4[2], S4[3], S4[4]);
+  const Jet2<T> A = g22 * L, B = g12 * M, C = g11 * N;
+  const T s = A.v + B.v + C.v, st = A.t + B.t + C.t, sp = A.p + B.p + C.p;
+  const T stt = A.tt + B.tt + C.tt, stp = A.tp + B.tp + C.tp, spp = A.pp + B.pp + C.pp;
+  // h = s r with r = q^(-3/2): r_,t / r = -3/2 lt, r_,tt / r = 15/4 lt^2 - 3/2 ltt
+  const T isq = sqrt(iq), r = iq * isq;
+  const T ht = r * (st - T(1.5) * s * lt), hp = r * (sp - T(1.5) * s * lp);
+  const T htt = r * (stt - T(3) * st * lt + s * (T(3.75) * lt * lt - T(1.5) * ltt));
+  const T htp = r * (stp - T(1.5) * (st * lp + sp * lt) + s * (T(3.75) * lt * lp - T(1.5) * ltp));
+  const T hpp = r * (spp - T(3) * sp * lp + s * (T(3.75) * lp * lp - T(1.5) * lpp));
+  // contravariant metric, u^a = a^ab h_,b, and Lap(h) = a^ab (h_,ab - x_ab . u)
+  const T c11 = g22.v * iq, c22 = g11.v * iq, c12 = T(0.5) * g12.v * iq;
+  const T u1 = c11 * ht + c12 * hp, u2 = c12 * ht + c22 * hp;
+  const T k11 = htt - (u1 * a1x11 + u2 * a2x11), k12 = htp - (u1 * a1x12 + u2 * a2x12),
+          k22 = hpp - (u1 * a1x22 + u2 * a2x22);
+  const T lap = c11 * k11 + T(2) * c12 * k12 + c22 * k22;
+  const T w1 = (u1 * L.v + u2 * M.v) * isq, w2 = (u1 * M.v + u2 * N.v) * isq;  // u^b b_ba
+  const T d1 = eb * (c11 * w1 + c12 * w2), d2 = eb * (c12 * w1 + c22 * w2), dn = -eb * lap * isq;
+  for (int c = 0; c < 3; ++c) f[c] += dn * m[c] + d1 * a1[c] + d2 * a2[c];
 }
 
 }  // namespace sg
