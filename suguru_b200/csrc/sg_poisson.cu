@@ -140,14 +140,18 @@ __device__ __forceinline__ int fdiv_u(int x, FastDiv f) { return f.d == 1 ? x : 
 //   q_k = al_k q_{k-1} + z_k r_k,  x_k = q_k + al_k x_{k+1},  al_k = -a z_k
 // (a = dzi^2 is both a_k, k >= 1, and c_k), the same for the real and the
 // imaginary parts.  A chain of all levels takes 34 cycles a level, 8,700 for
-// 128 levels up and down, with two warps busy; so the levels are cut into
-// eight segments, and a warp sweeps four real columns, lane = 4 segment +
-// column: from a zero start for the segment's end value and the product of
-// its al, which shuffles compose into the true starts, then from those.
-// |al| <= 1, so the composition loses nothing.  Rows of a segment are shifted
-// by 32 bytes per segment (pivots: 16), so that the warp's lanes fall on
-// different banks.
-constexpr int kSegs = 8;
+// 128 levels up and down, with two warps busy; so the levels are cut into 16
+// segments, and a warp sweeps two columns, lane = 2 segment + column: from a
+// zero start for the segment's end value and the product of its al, which
+// shuffles compose into the true starts, then from those.  The way up from the
+// true start also sums what the segment hands down (x at its first level from
+// a zero above it is the sum of q_k times the al below k), so the levels are
+// read three times.  |al| <= 1, so the composition loses nothing.  Bound by
+// shared memory: eight segments with a lane per real column and four reads
+// took half as many wavefronts again (the flow step's kernel 170 us at
+// 256 x 256 x 128, now 155 us).  Rows of a segment are shifted by 32 bytes per
+// segment (pivots: 16), so that the warp's lanes fall on different banks.
+constexpr int kSegs = 16;
 
 template <int C>
 struct Tile {
@@ -156,58 +160,78 @@ struct Tile {
 };
 __host__ __device__ constexpr int tile_size(int kmax, int C) { return kmax * C + 2 * kSegs; }
 
-// Columns 4 col4 .. 4 col4 + 3 of the tile's 2 C real ones; whole warps.
+// (f, p) <- the maps x -> f x + p of the segments up to the lane's own
+// (down: from the top), composed; returns what enters the lane's segment.
+template <bool DOWN>
+__device__ __forceinline__ double2 compose_segments(double f, double2 p, int seg) {
+#pragma unroll
+  for (int d = 1; d < kSegs; d *= 2) {
+    double ft, px, py;
+    if (DOWN) {
+      ft = __shfl_down_sync(0xffffffffu, f, 2 * d);
+      px = __shfl_down_sync(0xffffffffu, p.x, 2 * d);
+      py = __shfl_down_sync(0xffffffffu, p.y, 2 * d);
+    } else {
+      ft = __shfl_up_sync(0xffffffffu, f, 2 * d);
+      px = __shfl_up_sync(0xffffffffu, p.x, 2 * d);
+      py = __shfl_up_sync(0xffffffffu, p.y, 2 * d);
+    }
+    if (DOWN ? seg + d < kSegs : seg >= d) {
+      p = make_double2(fma(f, px, p.x), fma(f, py, p.y));
+      f *= ft;
+    }
+  }
+  const bool first = seg == (DOWN ? kSegs - 1 : 0);
+  const double2 in = DOWN ? make_double2(__shfl_down_sync(0xffffffffu, p.x, 2), __shfl_down_sync(0xffffffffu, p.y, 2))
+                          : make_double2(__shfl_up_sync(0xffffffffu, p.x, 2), __shfl_up_sync(0xffffffffu, p.y, 2));
+  return first ? make_double2(0.0, 0.0) : in;
+}
+
+// Columns 2 col2 and 2 col2 + 1 of the tile; whole warps.
 template <int C>
-__device__ __forceinline__ void tri_tile_sweeps(double2* tile, const double* zs, int col4, int kmax, int len, int e,
+__device__ __forceinline__ void tri_tile_sweeps(double2* tile, const double* zs, int col2, int kmax, int len, int e,
                                                 double a) {
-  const int lane = threadIdx.x & 31, seg = lane >> 2, cl = lane & 3, col = 4 * col4 + cl;
-  const int k0 = seg * len, n = min(len, kmax - k0), nu = min(n, kmax - 1 - k0);
-  double* c = (double*)(tile + k0 * C + 2 * seg) + col;
-  const double* z = zs + k0 * C + 2 * seg + (col >> 1);
-  double f = 1.0, p = 0.0, in = 0.0;
+  const int lane = threadIdx.x & 31, seg = lane >> 1, k0 = seg * len;
+  const int n = min(len, kmax - k0), nu = min(n, kmax - 1 - k0), o = k0 * C + 2 * seg + 2 * col2 + (lane & 1);
+  double2* c = tile + o;
+  const double* z = zs + o;
+  double f = 1.0;
+  double2 p = make_double2(0.0, 0.0);
 #pragma unroll 4
   for (int t = 0; t < nu; ++t) {
     const double w = z[t * C], al = -(a * w);
-    p = fma(al, p, c[2 * t * C] * w);
+    const double2 r = c[t * C];
+    p = make_double2(fma(al, p.x, r.x * w), fma(al, p.y, r.y * w));
     f *= al;
   }
   __syncwarp();
-#pragma unroll
-  for (int t = 0; t < kSegs - 1; ++t) {
-    const double ft = __shfl_sync(0xffffffffu, f, 4 * t + cl), pt = __shfl_sync(0xffffffffu, p, 4 * t + cl);
-    if (t < seg) in = fma(ft, in, pt);
-  }
-  p = in;
+  p = compose_segments<false>(f, p, seg);
+  double g = 1.0;
+  double2 d = make_double2(0.0, 0.0);
 #pragma unroll 4
   for (int t = 0; t < nu; ++t) {
-    const double w = z[t * C];
-    p = fma(-(a * w), p, c[2 * t * C] * w);
-    c[2 * t * C] = p;
+    const double w = z[t * C], al = -(a * w);
+    const double2 r = c[t * C];
+    p = make_double2(fma(al, p.x, r.x * w), fma(al, p.y, r.y * w));
+    c[t * C] = p;
+    d = make_double2(fma(g, p.x, d.x), fma(g, p.y, d.y));
+    g *= al;
   }
   if (n > 0 && k0 + n == kmax) {  // the top row: its pivot itself is tabulated; e = 3: the identity row of w
-    const double w = z[nu * C];
-    c[2 * nu * C] = w != 0.0 ? fma(e == 3 ? 0.0 : -a, p, c[2 * nu * C]) / w : 0.0;
+    const double w = z[nu * C], al = e == 3 ? 0.0 : -a;
+    const double2 r = c[nu * C];
+    p = w != 0.0 ? make_double2(fma(al, p.x, r.x) / w, fma(al, p.y, r.y) / w) : make_double2(0.0, 0.0);
+    c[nu * C] = p;
+    d = make_double2(fma(g, p.x, d.x), fma(g, p.y, d.y));
   }
-  f = 1.0;
-  p = 0.0;
+  __syncwarp();
+  p = compose_segments<true>(f, d, seg);
 #pragma unroll 4
   for (int t = n - 1; t >= 0; --t) {  // (the top row's al only meets zeros)
     const double al = -(a * z[t * C]);
-    p = fma(al, p, c[2 * t * C]);
-    f *= al;
-  }
-  __syncwarp();
-  in = 0.0;
-#pragma unroll
-  for (int t = kSegs - 1; t > 0; --t) {
-    const double ft = __shfl_sync(0xffffffffu, f, 4 * t + cl), pt = __shfl_sync(0xffffffffu, p, 4 * t + cl);
-    if (t > seg) in = fma(ft, in, pt);
-  }
-  p = in;
-#pragma unroll 4
-  for (int t = n - 1; t >= 0; --t) {
-    p = fma(-(a * z[t * C]), p, c[2 * t * C]);
-    c[2 * t * C] = p;
+    const double2 r = c[t * C];
+    p = make_double2(fma(al, p.x, r.x), fma(al, p.y, r.y));
+    c[t * C] = p;
   }
 }
 
@@ -377,9 +401,9 @@ __global__ void __launch_bounds__(48 * C) tri_flow_tile_kernel(int kmax, int jto
     }
   stage_wait();
   __syncthreads();
-  {  // C / 2 warps for each of u, v, w
-    const int f = warp / (C / 2), c4 = warp - f * (C / 2);
-    tri_tile_sweeps<C>(f == 0 ? su : f == 1 ? sv : sw, f == 2 ? z3 : z2, c4, kmax, len.d, f == 2 ? 3 : 2, a);
+  {  // C / 2 warps (two columns each) for each of u, v, w
+    const int f = warp / (C / 2), c2 = warp - f * (C / 2);
+    tri_tile_sweeps<C>(f == 0 ? su : f == 1 ? sv : sw, f == 2 ? z3 : z2, c2, kmax, len.d, f == 2 ? 3 : 2, a);
   }
   __syncthreads();
   const double2 ex = F.ex[m], ey = F.ey[min(j0 + jl, jtot - 1)];
