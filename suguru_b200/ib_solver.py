@@ -62,6 +62,7 @@ class IBSolver:
                 self.lag32 = [torch.zeros(wl.npts, dtype=torch.float32, device="cuda") for _ in range(10)]
                 self.force32 = [torch.zeros_like(self.u32[0]) for _ in range(3)]
         self.stepped = False
+        self._triple = False  # run() is capturing three steps
 
     def step(self, marks=None):
         """One step; marks: optional list of 5 CUDA events recorded between the stages
@@ -69,10 +70,19 @@ class IBSolver:
         cs, L = self.cs, self.lag
         mark = (lambda q: marks[q].record(self.st)) if marks else (lambda q: None)
         with self.torch.cuda.stream(self.st):
-            # uoo <- uo <- unew (buffers rotate; u still holds unew for the interpolation)
-            self.uoo, self.uo = self.uo, self.uoo
-            for a, b in zip(self.uo, self.u):
-                a.copy_(b)
+            # uoo <- uo <- unew.  Outside a capture the three buffers rotate and nothing is
+            # copied (copying u to uo, 400 MB moved, made a step at 256 x 256 x 128 with 256
+            # capsules 1735 us instead of 1706): the flow step reads levels n and n - 1 from u and uo, and writes level n + 1 where
+            # level n - 2 was.  A caller's own capture keeps the pointers of a pair of steps:
+            # it copies, so that two captured steps return every buffer to its place.
+            rotate = self._triple or not self.torch.cuda.is_current_stream_capturing()
+            if rotate:
+                level, below, out = self.u, self.uo, self.uoo
+            else:
+                self.uoo, self.uo = self.uo, self.uoo
+                for a, b in zip(self.uo, self.u):
+                    a.copy_(b)
+                level, below, out = self.uo, self.uoo, self.unext
             mark(0)
             if self.mixed:
                 for a, b in zip(self.u32, self.u):
@@ -93,9 +103,12 @@ class IBSolver:
             else:
                 cs.update_pos(self.dt, *self.X, L[0], L[1], L[2])
             mark(3)
-            cs.flow_step(self.dt, *self.uo, *self.uoo, self.p, *self.force, out=self.unext)
+            cs.flow_step(self.dt, *level, *below, self.p, *self.force, out=out)
             mark(4)
-            self.u, self.unext = self.unext, self.u
+            if rotate:
+                self.u, self.uo, self.uoo = out, level, below
+            else:
+                self.u, self.unext = self.unext, self.u
         self.stepped = True
 
     def stage_times(self, steps):
@@ -112,10 +125,10 @@ class IBSolver:
     def run(self, steps, graph=False):
         """Advance `steps` steps; returns the CUDA-event time in ms.
 
-        graph: capture two steps in one CUDA graph (the buffers rotate every
-        step, so a pair returns them to their places) and replay it, an odd
-        last step running eagerly; the work is the same, without host launches
-        between the kernels.  A solver that has not stepped yet runs its first
+        graph: capture three steps in one CUDA graph (the buffers rotate every
+        step, so three return them to their places) and replay it, the last one
+        or two steps of the rest running eagerly; the work is the same, without
+        host launches between the kernels.  A solver that has not stepped yet runs its first
         step eagerly and outside the timed region, so that first launches stay
         outside the capture."""
         torch = self.torch
@@ -126,21 +139,25 @@ class IBSolver:
             self.step()
             steps -= 1
             torch.cuda.synchronize()
-        if graph and steps >= 2:
+        if graph and steps >= 3:
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(g, stream=self.st):
-                self.step()
-                self.step()
+            self._triple = True
+            try:
+                with torch.cuda.graph(g, stream=self.st):
+                    for _ in range(3):
+                        self.step()
+            finally:
+                self._triple = False
         e0.record(self.st)
         if g is not None:
-            # the capture recorded the work without running it; the pair's buffer
-            # rotation already happened on the host, which a pair restores.  The
+            # the capture recorded the work without running it; the three steps'
+            # buffer rotation already happened on the host and restored itself.  The
             # replays go to the solver's stream, between the timing events.
             with torch.cuda.stream(self.st):
-                for _ in range(steps // 2):
+                for _ in range(steps // 3):
                     g.replay()
-            if steps % 2:
+            for _ in range(steps % 3):
                 self.step()
         else:
             for _ in range(steps):
