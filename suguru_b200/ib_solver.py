@@ -72,9 +72,10 @@ class IBSolver:
         with self.torch.cuda.stream(self.st):
             # uoo <- uo <- unew.  Outside a capture the three buffers rotate and nothing is
             # copied (copying u to uo, 400 MB moved, made a step at 256 x 256 x 128 with 256
-            # capsules 1735 us instead of 1706): the flow step reads levels n and n - 1 from u and uo, and writes level n + 1 where
-            # level n - 2 was.  A caller's own capture keeps the pointers of a pair of steps:
-            # it copies, so that two captured steps return every buffer to its place.
+            # capsules 1735 us instead of 1706): the flow step reads levels n and n - 1 from u
+            # and uo, and writes level n + 1 where level n - 2 was.  A caller's own capture
+            # keeps the pointers of a pair of steps: it copies, so that two captured steps
+            # return every buffer to its place.
             rotate = self._triple or not self.torch.cuda.is_current_stream_capturing()
             if rotate:
                 level, below, out = self.u, self.uo, self.uoo
