@@ -318,7 +318,8 @@ int setup(sg_ctx* c) {
     c->own_stream = true;
   }
   // FP32 spreads on 16 x 16 x 8 tiles (fewer points straddle a tile edge);
-  // FP64 keeps 1024-cell tiles for its three-limb shared accumulators
+  // FP64 keeps 1024-cell tiles for its two-limb shared accumulators and their
+  // 64-bit totals in registers
   const int shape = (c->mixed && cfg.itot >= 16 && cfg.jtot >= 16) ? 1 : -1;
   const unsigned allowed = c->mixed ? kAllTileShapes : kFp64TileShapes;
   if (!make_ib_grid(cfg.itot, cfg.jtot, cfg.ktot, cfg.lx, cfg.ly, cfg.lz, c->grid, shape, allowed) &&

@@ -353,10 +353,10 @@ __global__ void __launch_bounds__(128) tri_apply_kernel(int kmax, int jtot, int 
 // with ex = exp(-2 pi i m / itot) and ey = exp(-2 pi i j / jtot):
 //   u(i) - u(i-1) -> (1 - ex) u,   p(i+1) - p(i) -> (conj(ex) - 1) p;
 // w(0) = 0 in the divergence, and the top row of w, zero, takes no
-// correction (p(k1) = p(kmax)).  Memory-bound (72 bytes in and 64 out per
-// mode, 590 MB at 256 x 256 x 128); in physical space the same steps moved
-// the modes of all four fields twice more, and u, v, w and p once each
-// through fillps and correc.
+// correction (p(k1) = p(kmax)).  72 bytes in and 64 out per mode, 590 MB at
+// 256 x 256 x 128 (91 us; 155 measured): shared memory and the phases' barriers
+// bound it.  In physical space the same steps moved the modes of all four
+// fields twice more, and u, v, w and p once each through fillps and correc.
 struct FlowModes {
   double2 *u, *v, *w, *p;                      // [m][k][j]
   const double *z2, *z3, *z1;                  // pivots of e = 2, 3, 1
