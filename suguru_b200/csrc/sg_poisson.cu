@@ -911,12 +911,6 @@ struct RowTarget {
     if (i == 1) r[nx + 1] = x;
     if (i == nx) r[0] = x;
   }
-  __device__ __forceinline__ void put(int i, double x) const {  // cell i of 1 .. itot
-    x *= scale;
-    if (add) x = f[i] + x;
-    store(f, i, x);
-    copies(i, x);
-  }
   __device__ __forceinline__ void copies(int i, double x) const {
     if (img) store(img, i, x);
     if (wall) {
@@ -933,7 +927,33 @@ struct RowTarget {
 // W = exp(-2 pi i / nx), Z_n = Z_0; mode k of row r at dst[k nrows + r].
 constexpr int kAnyThreads = 128;
 
-__global__ void __launch_bounds__(kAnyThreads, 4) rows_r2c_any(long nrows, FastDiv nb, FftPlan P,
+// The CTA's rows of n values, contiguous in global memory, into its padded
+// slots.  Ten loads of a thread are issued before their stores (up to 1280
+// values, what any_rows gives a CTA, in one round): these kernels hold 16
+// warps an SM and wait for memory first.  SWAP: real and imaginary parts
+// exchanged.
+template <bool SWAP>
+__device__ __forceinline__ void stage_rows(double2* s, const double2* g, int rows, int ld, FastDiv n) {
+  constexpr int H = 10;
+  const int total = rows * (int)n.d;
+  for (int t0 = threadIdx.x; t0 < total; t0 += H * kAnyThreads) {
+    double2 x[H];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int t = t0 + h * kAnyThreads;
+      x[h] = t < total ? g[t] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int t = t0 + h * kAnyThreads;
+      if (t >= total) break;
+      const int r = fdiv_u(t, n);
+      s[r * ld + fpad(t - r * (int)n.d)] = SWAP ? cswap(x[h]) : x[h];
+    }
+  }
+}
+
+__global__ void __launch_bounds__(kAnyThreads, 4) rows_r2c_any(long nrows, FastDiv nb, FastDiv nd, FftPlan P,
                                                             const double2* __restrict__ wpost,
                                                             const double* __restrict__ src, double2* __restrict__ dst) {
   extern __shared__ __align__(16) double2 fsm[];
@@ -944,10 +964,7 @@ __global__ void __launch_bounds__(kAnyThreads, 4) rows_r2c_any(long nrows, FastD
   const int rows = (int)min((long)nb.d, nrows - r0);
   double2* b0 = fsm;
   double2* b1 = fsm + nb.d * ld;
-  const double2* s2 = (const double2*)src + r0 * n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int r = warp; r < rows; r += kAnyThreads / 32)
-    for (int t = lane; t < n; t += 32) b0[r * ld + fpad(t)] = s2[(long)r * n + t];
+  stage_rows<false>(b0, (const double2*)src + r0 * n, rows, ld, nd);
   const double2* Z = fft_any(b0, b1, rows, ld, P);
   for (int t = threadIdx.x; t < (n + 1) * (int)nb.d; t += kAnyThreads) {
     const int k = fdiv_u(t, nb), r = t - k * nb.d;
@@ -975,17 +992,30 @@ __global__ void __launch_bounds__(kAnyThreads, 4) rows_c2r_any(long nrows, FastD
   const int rows = (int)min((long)nb.d, nrows - r0);
   double2* b0 = fsm;
   double2* b1 = fsm + nb.d * ld;
-  for (int t = threadIdx.x; t < (n / 2 + 1) * (int)nb.d; t += kAnyThreads) {
-    const int k = fdiv_u(t, nb), r = t - k * nb.d;
-    if (r >= rows) continue;
-    const double2 a = src[(long)k * nrows + r0 + r], b = src[(long)(n - k) * nrows + r0 + r];
-    auto z = [&](double2 x, double2 y, int q) {  // Z_q from X_q = x and X_{n-q} = y
-      const double2 yc = cconj(y);
-      const double2 sum = cadd(x, yc), t2 = cmul(cconj(wpost[q]), csub(x, yc));  // times i: (-t2.y, t2.x)
-      return make_double2(sum.x - t2.y, sum.y + t2.x);
-    };
-    b0[r * ld + fpad(k)] = cswap(z(a, b, k));
-    if (k > 0) b0[r * ld + fpad(n - k)] = cswap(z(b, a, n - k));
+  // mode pairs (k, n - k) of the rows, six of a thread loaded before they are used
+  constexpr int H = 6;
+  const int total = (n / 2 + 1) * (int)nb.d;
+  for (int t0 = threadIdx.x; t0 < total; t0 += H * kAnyThreads) {
+    double2 a[H], b[H];
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int t = t0 + h * kAnyThreads, k = fdiv_u(t, nb), r = t - k * (int)nb.d;
+      const bool in = t < total && r < rows;
+      a[h] = in ? src[(long)k * nrows + r0 + r] : make_double2(0.0, 0.0);
+      b[h] = in ? src[(long)(n - k) * nrows + r0 + r] : make_double2(0.0, 0.0);
+    }
+#pragma unroll
+    for (int h = 0; h < H; ++h) {
+      const int t = t0 + h * kAnyThreads, k = fdiv_u(t, nb), r = t - k * (int)nb.d;
+      if (t >= total || r >= rows) continue;
+      auto z = [&](double2 x, double2 y, int q) {  // Z_q from X_q = x and X_{n-q} = y
+        const double2 yc = cconj(y);
+        const double2 sum = cadd(x, yc), t2 = cmul(cconj(wpost[q]), csub(x, yc));  // times i: (-t2.y, t2.x)
+        return make_double2(sum.x - t2.y, sum.y + t2.x);
+      };
+      b0[r * ld + fpad(k)] = cswap(z(a[h], b[h], k));
+      if (k > 0) b0[r * ld + fpad(n - k)] = cswap(z(b[h], a[h], n - k));
+    }
   }
   const double2* z = fft_any(b0, b1, rows, ld, P);  // swapped: (Im, Re)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -995,10 +1025,27 @@ __global__ void __launch_bounds__(kAnyThreads, 4) rows_c2r_any(long nrows, FastD
       double2* d2 = (double2*)dst + row * n;
       for (int t = lane; t < n; t += 32) d2[t] = cswap(z[r * ld + fpad(t)]);
     } else {
-      const RowTarget t(out, (int)(row % out.jtot), (int)(row / out.jtot));
-      for (int i = lane; i < 2 * n; i += 32) {
-        const double2 v = z[r * ld + fpad(i >> 1)];
-        t.put(i + 1, i & 1 ? v.x : v.y);
+      const int kr = (int)row / out.jtot;  // a field has less than 2^31 rows
+      const RowTarget t(out, (int)row - kr * out.jtot, kr);
+      const double* zr = (const double*)(z + r * ld);
+      for (int i0 = lane; i0 < 2 * n; i0 += H * 32) {
+        double x[H];
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          const int i = i0 + 32 * h;
+          x[h] = i < 2 * n ? t.scale * zr[2 * fpad(i >> 1) + 1 - (i & 1)] : 0.0;
+        }
+        if (t.add)
+#pragma unroll
+          for (int h = 0; h < H; ++h)
+            if (i0 + 32 * h < 2 * n) x[h] = t.f[i0 + 32 * h + 1] + x[h];
+#pragma unroll
+        for (int h = 0; h < H; ++h) {
+          const int i = i0 + 32 * h + 1;
+          if (i > 2 * n) continue;
+          t.store(t.f, i, x[h]);
+          t.copies(i, x[h]);
+        }
       }
     }
   }
@@ -1006,25 +1053,23 @@ __global__ void __launch_bounds__(kAnyThreads, 4) rows_c2r_any(long nrows, FastD
 
 // y transforms: nseq contiguous sequences, nb per CTA, in place; an inverse by
 // swapping parts
-__global__ void __launch_bounds__(kAnyThreads, 4) cols_any(long nseq, int nb, FftPlan P, bool inv,
+__global__ void __launch_bounds__(kAnyThreads, 4) cols_any(long nseq, int nb, FastDiv nd, FftPlan P, bool inv,
                                                         double2* __restrict__ data) {
   extern __shared__ __align__(16) double2 fsm[];
   const int n = P.n, ld = fld(n);
   const long s0 = (long)blockIdx.x * nb;
   const int ns = (int)min((long)nb, nseq - s0);
   double2* d = data + s0 * n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int r = warp; r < ns; r += kAnyThreads / 32)
-    for (int t = lane; t < n; t += 32) {
-      const double2 x = d[(long)r * n + t];
-      fsm[r * ld + fpad(t)] = inv ? cswap(x) : x;
-    }
+  if (inv)
+    stage_rows<true>(fsm, d, ns, ld, nd);
+  else
+    stage_rows<false>(fsm, d, ns, ld, nd);
   const double2* y = fft_any(fsm, fsm + nb * ld, ns, ld, P);
-  for (int r = warp; r < ns; r += kAnyThreads / 32)
-    for (int t = lane; t < n; t += 32) {
-      const double2 x = y[r * ld + fpad(t)];
-      d[(long)r * n + t] = inv ? cswap(x) : x;
-    }
+  for (int t = threadIdx.x; t < ns * n; t += kAnyThreads) {
+    const int r = fdiv_u(t, nd);
+    const double2 x = y[r * ld + fpad(t - r * n)];
+    d[t] = inv ? cswap(x) : x;
+  }
 }
 
 constexpr int kRegThreads = 256;
@@ -1150,7 +1195,8 @@ __global__ void __launch_bounds__(kRegThreads) rows_c2r_reg(long nrows, const do
   store_last<N>(v, seq, tau);
   __syncwarp();
   if (!ok) return;
-  const RowTarget t(out, (int)(row % out.jtot), (int)(row / out.jtot));
+  const int kr = (int)row / out.jtot;  // a field has less than 2^31 rows
+  const RowTarget t(out, (int)row - kr * out.jtot, kr);
   const double* xs = (const double*)seq;
   double x[16];  // cells tau + q TPS + 1
 #pragma unroll
@@ -1476,8 +1522,8 @@ int rows_forward(sg_ctx* c, int nf, const double* r, double2* modes, cudaStream_
 #undef SG_R2C
   } else {
     SG_TRY(smem_limit(rows_r2c_any, any_smem(n)), "fft");
-    rows_r2c_any<<<dim3((unsigned)((nrows + nb - 1) / nb), nf), kAnyThreads, any_smem(n), st>>>(nrows, fast_div(nb), pl.x,
-                                                                                              s.wpost, r, modes);
+    rows_r2c_any<<<dim3((unsigned)((nrows + nb - 1) / nb), nf), kAnyThreads, any_smem(n), st>>>(nrows, fast_div(nb), fast_div(n),
+                                                                                              pl.x, s.wpost, r, modes);
   }
   SG_TRY(cudaGetLastError(), "solver1d");
   c->launches += 1;
@@ -1519,7 +1565,8 @@ int cols_transform(sg_ctx* c, int nf, int sign, double2* modes, cudaStream_t st)
 #undef SG_COLS
   } else {
     SG_TRY(smem_limit(cols_any, any_smem(f.jtot)), "fft");
-    cols_any<<<(unsigned)((nseq + nb - 1) / nb), kAnyThreads, any_smem(f.jtot), st>>>(nseq, nb, pl.y, sign > 0, modes);
+    cols_any<<<(unsigned)((nseq + nb - 1) / nb), kAnyThreads, any_smem(f.jtot), st>>>(nseq, nb, fast_div(f.jtot),
+                                                                                     pl.y, sign > 0, modes);
   }
   SG_TRY(cudaGetLastError(), "solver1d");
   c->launches += 1;
