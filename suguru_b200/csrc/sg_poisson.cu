@@ -1271,12 +1271,15 @@ void best_radices(int n, std::vector<int>& cur, std::vector<int>& best) {
 // false when a prime factor is above kMaxRadix or there are too many passes
 bool make_plan(int n, FftPlan& P, std::vector<double>& tw) {
   std::vector<int> rad, primes;
-  int m = n;
-  for (int p = 11; p <= m; p += 2)
-    while (m % p == 0) {
+  int big = n;  // without its factors 2, 3, 5 and 7
+  for (int p : {2, 3, 5, 7})
+    while (big % p == 0) big /= p;
+  const int m = n / big;
+  for (int p = 11; p <= big; p += 2)
+    while (big % p == 0) {
       if (p > kMaxRadix) return false;
       primes.push_back(p);
-      m /= p;
+      big /= p;
     }
   std::vector<int> cur;
   if (m > 1) best_radices(m, cur, rad);

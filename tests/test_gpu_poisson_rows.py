@@ -15,6 +15,15 @@ from test_gpu_flow_solver import _ctx, _state
 pytestmark = pytest.mark.gpu
 
 
+# lengths with odd composite factors above 10 (21, 27, 35, 45, 63), which are passes of several small radices
+ODD = [(294, 108, 6), (126, 27, 5), (70, 63, 9), (90, 135, 4)]
+
+
+@pytest.mark.parametrize("n", ODD)
+def test_flow_step_odd_composites(cuda, n):
+    test_flow_step_power_rows(cuda, n)
+
+
 @pytest.mark.parametrize("n", [(64, 13, 5), (64, 16, 16), (128, 13, 15), (128, 8, 32), (256, 11, 16), (256, 8, 4),
                                (512, 12, 31), (512, 8, 18)])
 def test_flow_step_power_rows(cuda, n):
