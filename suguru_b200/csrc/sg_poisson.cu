@@ -930,8 +930,10 @@ constexpr int kAnyThreads = 128;
 // The CTA's rows of n values, contiguous in global memory, into its padded
 // slots.  Ten loads of a thread are issued before their stores (up to 1280
 // values, what any_rows gives a CTA, in one round): these kernels hold 16
-// warps an SM and wait for memory first.  SWAP: real and imaginary parts
-// exchanged.
+// warps an SM and wait for memory first.  With a load at a time, and a pair or
+// a cell at a time in rows_c2r_any, 180 x 150 x 99 took 65 us (forward rows of
+// three fields), 108 (columns), 116 (inverse rows of four); now 47, 88, 85.
+// SWAP: real and imaginary parts exchanged.
 template <bool SWAP>
 __device__ __forceinline__ void stage_rows(double2* s, const double2* g, int rows, int ld, FastDiv n) {
   constexpr int H = 10;
