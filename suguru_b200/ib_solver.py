@@ -56,13 +56,15 @@ class IBSolver:
             self.lag = [torch.zeros(wl.npts, dtype=torch.float64, device="cuda") for _ in range(10)]
             self.force = [torch.zeros_like(self.u[0]) for _ in range(3)]
             self.ind = [torch.zeros_like(self.u[0]) for _ in range(2)]
+            # for steps that copy; made here, since one made inside a capture would be the graph's
             self.unext = [torch.zeros_like(self.u[0]) for _ in range(3)]
             if self.mixed:  # the mixed step's own buffers
                 self.u32 = [torch.zeros(self.u[0].shape, dtype=torch.float32, device="cuda") for _ in range(3)]
                 self.lag32 = [torch.zeros(wl.npts, dtype=torch.float32, device="cuda") for _ in range(10)]
                 self.force32 = [torch.zeros_like(self.u32[0]) for _ in range(3)]
         self.stepped = False
-        self._triple = False  # run() is capturing three steps
+        self._own = False  # run() is capturing, for a graph that it replays itself
+        self._pairs = False  # a caller has captured a step: see step()
 
     def step(self, marks=None):
         """One step; marks: optional list of 5 CUDA events recorded between the stages
@@ -70,20 +72,21 @@ class IBSolver:
         cs, L = self.cs, self.lag
         mark = (lambda q: marks[q].record(self.st)) if marks else (lambda q: None)
         with self.torch.cuda.stream(self.st):
-            # uoo <- uo <- unew.  Outside a capture the three buffers rotate and nothing is
-            # copied (copying u to uo, 400 MB moved, made a step at 256 x 256 x 128 with 256
-            # capsules 1735 us instead of 1706): the flow step reads levels n and n - 1 from u
-            # and uo, and writes level n + 1 where level n - 2 was.  A caller's own capture
-            # keeps the pointers of a pair of steps: it copies, so that two captured steps
-            # return every buffer to its place.
-            rotate = self._triple or not self.torch.cuda.is_current_stream_capturing()
-            if rotate:
-                level, below, out = self.u, self.uo, self.uoo
-            else:
+            # uoo <- uo <- unew: the three buffers rotate and nothing is copied (copying u to
+            # uo, 400 MB moved, made a step at 256 x 256 x 128 with 256 capsules 1735 us instead
+            # of 1706): the flow step reads levels n and n - 1 from u and uo, and writes level
+            # n + 1 where level n - 2 was.  A caller's own capture keeps the pointers of a pair
+            # of steps: from the first one on every step copies, so that any two steps, captured
+            # or not, leave every buffer in its place for the next replay.
+            if not self._own and self.torch.cuda.is_current_stream_capturing():
+                self._pairs = True
+            if self._pairs:
                 self.uoo, self.uo = self.uo, self.uoo
                 for a, b in zip(self.uo, self.u):
                     a.copy_(b)
                 level, below, out = self.uo, self.uoo, self.unext
+            else:
+                level, below, out = self.u, self.uo, self.uoo
             mark(0)
             if self.mixed:
                 for a, b in zip(self.u32, self.u):
@@ -106,10 +109,10 @@ class IBSolver:
             mark(3)
             cs.flow_step(self.dt, *level, *below, self.p, *self.force, out=out)
             mark(4)
-            if rotate:
-                self.u, self.uo, self.uoo = out, level, below
-            else:
+            if self._pairs:
                 self.u, self.unext = self.unext, self.u
+            else:
+                self.u, self.uo, self.uoo = out, level, below
         self.stepped = True
 
     def stage_times(self, steps):
@@ -127,10 +130,11 @@ class IBSolver:
         """Advance `steps` steps; returns the CUDA-event time in ms.
 
         graph: capture three steps in one CUDA graph (the buffers rotate every
-        step, so three return them to their places) and replay it, the last one
-        or two steps of the rest running eagerly; the work is the same, without
-        host launches between the kernels.  A solver that has not stepped yet runs its first
-        step eagerly and outside the timed region, so that first launches stay
+        step, so three return them to their places; two after a caller's own
+        capture, see step) and replay it, the last one or two steps of the rest
+        running eagerly; the work is the same, without host launches between
+        the kernels.  A solver that has not stepped yet runs its first step
+        eagerly and outside the timed region, so that first launches stay
         outside the capture."""
         torch = self.torch
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
@@ -140,29 +144,28 @@ class IBSolver:
             self.step()
             steps -= 1
             torch.cuda.synchronize()
-        if graph and steps >= 3:
+        period = 2 if self._pairs else 3
+        if graph and steps >= period:
             torch.cuda.synchronize()
             g = torch.cuda.CUDAGraph()
-            self._triple = True
+            self._own = True
             try:
                 with torch.cuda.graph(g, stream=self.st):
-                    for _ in range(3):
+                    for _ in range(period):
                         self.step()
             finally:
-                self._triple = False
+                self._own = False
         e0.record(self.st)
         if g is not None:
-            # the capture recorded the work without running it; the three steps'
-            # buffer rotation already happened on the host and restored itself.  The
+            # the capture recorded the work without running it; the steps' buffer
+            # changes already happened on the host and restored themselves.  The
             # replays go to the solver's stream, between the timing events.
             with torch.cuda.stream(self.st):
-                for _ in range(steps // 3):
+                for _ in range(steps // period):
                     g.replay()
-            for _ in range(steps % 3):
-                self.step()
-        else:
-            for _ in range(steps):
-                self.step()
+            steps %= period
+        for _ in range(steps):
+            self.step()
         e1.record(self.st)
         torch.cuda.synchronize()
         del g
