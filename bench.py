@@ -515,7 +515,7 @@ def run_coupled(args, rank):
         sol.run(args.warmup)
         ms = sol.run(args.steps, graph=True)
         out[name] = {"steps_per_s": args.steps / (ms / 1e3), "ms_per_step": ms / args.steps,
-                     "timed": "replays of a CUDA graph of three steps", "stages_ms": sol.stage_times(3)}
+                     "timed": "replays of CUDA graphs of three steps and of the rest", "stages_ms": sol.stage_times(3)}
         del sol
     cpu = None
     if not args.no_cpu_baseline:

@@ -129,47 +129,52 @@ class IBSolver:
     def run(self, steps, graph=False):
         """Advance `steps` steps; returns the CUDA-event time in ms.
 
-        graph: capture three steps in one CUDA graph (the buffers rotate every
-        step, so three return them to their places; two after a caller's own
-        capture, see step) and replay it, the last one or two steps of the rest
-        running eagerly; the work is the same, without host launches between
-        the kernels.  A solver that has not stepped yet runs its first step
-        eagerly and outside the timed region, so that first launches stay
-        outside the capture."""
+        graph: replay CUDA graphs, without host launches between the kernels;
+        the work is the same.  One graph holds three steps (the buffers rotate
+        every step, so three return them to their places; two after a caller's
+        own capture, see step) and is replayed, another the one or two steps
+        that remain; a single step runs eagerly.  A solver that has not stepped
+        yet runs its first step eagerly and outside the timed region, so that
+        first launches stay outside the captures."""
         torch = self.torch
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
-        g = None
         if graph and not self.stepped and steps > 0:
-            # the libraries' first launches (module loads, FFT plans' first use) happen outside the capture
+            # the libraries' first launches (module loads, FFT plans' first use) happen outside the captures
             self.step()
             steps -= 1
             torch.cuda.synchronize()
-        period = 2 if self._pairs else 3
-        if graph and steps >= period:
+        graphs = []
+        if graph and steps > 1:
             torch.cuda.synchronize()
-            g = torch.cuda.CUDAGraph()
-            self._own = True
-            try:
-                with torch.cuda.graph(g, stream=self.st):
-                    for _ in range(period):
-                        self.step()
-            finally:
-                self._own = False
+            period = 2 if self._pairs else 3
+            graphs = [(self._capture(n), times) for n, times in ((period, steps // period), (steps % period, 1))
+                      if n * times]
+            steps = 0
         e0.record(self.st)
-        if g is not None:
-            # the capture recorded the work without running it; the steps' buffer
-            # changes already happened on the host and restored themselves.  The
-            # replays go to the solver's stream, between the timing events.
-            with torch.cuda.stream(self.st):
-                for _ in range(steps // period):
+        # the captures recorded the work without running it; their steps' buffer changes
+        # already happened on the host.  The replays go to the solver's stream, between the
+        # timing events.
+        with torch.cuda.stream(self.st):
+            for g, times in graphs:
+                for _ in range(times):
                     g.replay()
-            steps %= period
         for _ in range(steps):
             self.step()
         e1.record(self.st)
         torch.cuda.synchronize()
-        del g
         return e0.elapsed_time(e1)
+
+    def _capture(self, steps):
+        """A CUDA graph of `steps` steps."""
+        g = self.torch.cuda.CUDAGraph()
+        self._own = True
+        try:
+            with self.torch.cuda.graph(g, stream=self.st):
+                for _ in range(steps):
+                    self.step()
+        finally:
+            self._own = False
+        return g
 
     def state(self):
         self.torch.cuda.synchronize()
