@@ -170,8 +170,13 @@ int sg_indicator(sg_ctx* ctx, const double* X, const double* Y, const double* Z,
  * vt2 = v(k1) + v(kmax) (0, 0 for no-slip walls, iniu 'zer'; lz shear and
  * -lz shear for 'cou'; 2 bulk_v_sup for free slip), and allocates the
  * solver's workspace (itot even, ktot >= 4; in host memory mode also device
- * copies of the 13 fields).  The flow solver of the Crank-Nicolson path
- * (fsolver = 'c', crnk.f90) is not provided. */
+ * copies of the 13 fields).  The tables of the solves depend on Rep / dt: a
+ * call with another dt rebuilds them, a captured one keeps those of its own
+ * dt, whatever dt other calls take between the graph's launches.  The first
+ * calls with another dt after a capture, and captures of a dt that no call
+ * has taken, allocate tables of their own (one field each; four of a kind at
+ * most).  The flow solver of the Crank-Nicolson path (fsolver = 'c',
+ * crnk.f90) is not provided. */
 int sg_set_flow_params(sg_ctx* ctx, double rep, double vb2, double vt2);
 int sg_flow_step(sg_ctx* ctx, double dt, const double* uo, const double* vo, const double* wo,
                  const double* uoo, const double* voo, const double* woo, double* p,

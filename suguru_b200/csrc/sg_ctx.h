@@ -161,10 +161,19 @@ struct sg_ctx {
     double* r = nullptr;     // real FFT input / output [min(nfields, 3)][ktot][jtot][itot]
     void* c = nullptr;       // modes [nfields][itot/2 + 1][ktot][jtot] (double2)
     // elimination pivots per row type e = 0..3 (sg_poisson.cu), laid out as
-    // the modes, for the shift they were made with
-    double* zt[4] = {nullptr, nullptr, nullptr, nullptr};
-    double tshift[4] = {0, 0, 0, 0};
-    bool tvalid[4] = {false, false, false, false};
+    // the modes, each table for one shift.  Eager solves rebuild a free one for
+    // another shift.  One that a captured graph reads is pinned: nothing
+    // rewrites it, whatever is solved between the replays.  `graph` takes the
+    // builds that graphs record themselves (e = 2, 3), and eager solves never
+    // read it.
+    struct Pivots {
+      double* z;
+      double shift;
+      bool made, pinned;
+    };
+    static constexpr int kMostPinned = 2;  // graphs of further shifts build their own
+    std::vector<Pivots> zt[4];
+    double* graph[4] = {nullptr, nullptr, nullptr, nullptr};
     double* tab = nullptr;   // xrt [itot/2 + 1], yrt [jtot]
     double2* w = nullptr;    // twiddle tables
     double2* wpost = nullptr;  // the row split's W^k
