@@ -34,19 +34,21 @@
 //    contribution, below FP32 rounding of a typical cell value.
 //  - FP64: fixed point in two signed 32-bit limbs, in passes of at most 255
 //    entries whose limbs are then added into 64-bit registers.  With K entries
-//    in a pass and h the bit length of K, a contribution v, |v| < 2^(63-2h), is
-//    split as hi 2^p + lo, p = 32 - h: one FMA against 1.5 * 2^(52+p) rounds v
-//    to a multiple of 2^p whose integer is the low word of the sum, a second
-//    one forms the exact rest, |lo| <= 2^(p-1), and an addition of 1.5 * 2^52
-//    rounds it, so that K contributions overflow neither limb and no
-//    conversion or 64-bit shift is needed.  The step is 0.3 times the largest
-//    m_c over 2^(63-2h): 2^-47 of the largest contribution with 128 or more
-//    entries, finer with fewer.  Bound by the shared-memory atomics: three
-//    limbs of 19 bits in passes of 4096, split with a 64-bit integer
-//    conversion (step 2^-56 of the entry count times the largest m_c, coarser
-//    but for tiles of over 4096 very uneven entries), took 251 us at 524,288
-//    points on 256 x 256 x 128, these two take 208 us; leaving out the
-//    contributions that fall outside the tile by a predicate took 270 us.
+//    in a pass and h the bit length of K, a contribution v is split as
+//    hi 2^p + lo, p = 32 - h: one FMA against 1.5 * 2^(52+p) rounds v to a
+//    multiple of 2^p whose integer is the low word of the sum, a second one
+//    forms the exact rest, |lo| <= 2^(p-1), and an addition of 1.5 * 2^52 rounds
+//    it, so that no conversion or 64-bit shift is needed.  K of the lows stay
+//    below 2^31, and so do K of the highs when 0.3 K times the largest m_c is
+//    below 2^(31+p) steps (the weights' (2/3)^3 against 0.3 leaves more than the
+//    K/2 of their roundings): the step is the power of two for that, 2^-48.7 to
+//    2^-47.7 of the largest m_c with 255 entries, finer with fewer, and for every
+//    count up to 4096 no coarser than 2^-56 of the count times the largest m_c
+//    rounded up to a power of two.  Bound by the shared-memory atomics: three
+//    limbs of 19 bits in passes of 4096 with that step, split with a 64-bit
+//    integer conversion, took 251 us at 524,288 points on 256 x 256 x 128, these
+//    two take 208 us; leaving out the contributions that fall outside the tile by
+//    a predicate took 270 us.
 // Entries go to threads in blocks of 256: the lowest ceil(k/32) warps take the
 // k entries of a block, interleaved, so that no warp idles on a short list and
 // neighbouring points (adjacent entries) land in different warps, where they
@@ -150,13 +152,14 @@ __device__ __forceinline__ void tile_scales(int e0, int e1, const int* __restric
     const int cnt = e1 - e0;
     int sh[3];
     if constexpr (!F32) {
-      // FP64: every contribution below 2^(63-2h) for a pass's entries, and the
-      // tile's sum below 2^62 (more than 2^15 entries)
-      const int h = 32 - Fixed<double>::low_bits(min(cnt, Fixed<double>::PASS));
+      // FP64: the contributions of a pass's K entries together below 2^(31+p),
+      // and the tile's sum below 2^62 (more than 2^15 entries)
+      const int K = min(cnt, Fixed<double>::PASS);
 #pragma unroll
       for (int c = 0; c < 3; ++c) {
         const double m = 0.3 * (double)rmax[c];
-        sh[c] = min(63 - 2 * h - exp_above(m, -900), 62 - exp_above(m * (double)cnt, -900));
+        sh[c] = min(31 + Fixed<double>::low_bits(K) - exp_above(m * (double)K, -900),
+                    62 - exp_above(m * (double)cnt, -900));
       }
     } else {
 #pragma unroll
