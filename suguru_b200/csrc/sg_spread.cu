@@ -44,11 +44,19 @@
 //    K/2 of their roundings): the step is the power of two for that, 2^-48.7 to
 //    2^-47.7 of the largest m_c with 255 entries, finer with fewer, and for every
 //    count up to 4096 no coarser than 2^-56 of the count times the largest m_c
-//    rounded up to a power of two.  Bound by the shared-memory atomics: three
-//    limbs of 19 bits in passes of 4096 with that step, split with a 64-bit
-//    integer conversion, took 251 us at 524,288 points on 256 x 256 x 128, these
-//    two take 208 us; leaving out the contributions that fall outside the tile by
-//    a predicate took 270 us.
+//    rounded up to a power of two.  Above 4096 entries it is no coarser than
+//    2^-56 of 0.3 times the exact sum of m_c (as FP32 takes it), rounded up: where
+//    few large forces among many small ones make that finer, the tile goes in
+//    passes of 127 entries, whose highs the sum bounds as well.  (One tile of
+//    24,000 such entries within 2 x 2 x 2 cells: a spread of 854 us against 732
+//    in passes of 255, whose step is up to 2^9 coarser; with a third limb for the
+//    rest 1064, and 3 % more in every other tile.)  Bound by the shared-memory
+//    atomics: three limbs of 19 bits in passes of 4096 with these steps, split
+//    with a 64-bit integer conversion, took 251 us at 524,288 points on
+//    256 x 256 x 128, these two take 208 us; leaving out the contributions that
+//    fall outside the tile by a predicate took 270 us.  80 registers for three
+//    CTAs per SM spill 128 bytes a thread, the totals across the walk; at two
+//    CTAs without spills it takes 224 us.
 // Entries go to threads in blocks of 256: the lowest ceil(k/32) warps take the
 // k entries of a block, interleaved, so that no warp idles on a short list and
 // neighbouring points (adjacent entries) land in different warps, where they
@@ -75,7 +83,8 @@ struct Fixed<float> {
 template <>
 struct Fixed<double> {
   static constexpr int NW = 2;
-  static constexpr int PASS = 255;
+  static constexpr int PASS = 255;   // entries per pass, PASS / 2 in some tiles of more than
+  static constexpr int MAXC = 4096;  // MAXC entries
   // low limb width for `n` entries in a pass: 32 - the bit length of n
   __device__ static __forceinline__ int low_bits(int n) { return __clz(n); }
   // adds pyz * wx (in units of the step); mh = 1.5 * 2^(52+p)
@@ -124,7 +133,7 @@ __device__ __forceinline__ double pow2<double>(int e) {
 template <class T>
 __device__ __forceinline__ void tile_scales(int e0, int e1, const int* __restrict__ entries,
                                             const ForceRec<T>* __restrict__ frc, T (*s_red)[8],
-                                            unsigned long long (*s_sum)[8], T* scale, T* iscale) {
+                                            unsigned long long (*s_sum)[8], T* scale, T* iscale, int* pass) {
   constexpr bool F32 = sizeof(T) == 4;
   constexpr int QB = 30;  // FP32 sums stay below 2^QB
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -150,69 +159,86 @@ __device__ __forceinline__ void tile_scales(int e0, int e1, const int* __restric
       for (int q = 1; q < 8; ++q) rmax[c] = fmax(rmax[c], s_red[c][q]);
     }
     const int cnt = e1 - e0;
-    int sh[3];
-    if constexpr (!F32) {
-      // FP64: the contributions of a pass's K entries together below 2^(31+p),
-      // and the tile's sum below 2^62 (more than 2^15 entries)
-      const int K = min(cnt, Fixed<double>::PASS);
+    int sh[3], sh1[3];
+    bool need[3] = {false, false, false}, dense = false;
 #pragma unroll
-      for (int c = 0; c < 3; ++c) {
-        const double m = 0.3 * (double)rmax[c];
-        sh[c] = min(31 + Fixed<double>::low_bits(K) - exp_above(m * (double)K, -900),
-                    62 - exp_above(m * (double)cnt, -900));
-      }
-    } else {
-#pragma unroll
-      for (int c = 0; c < 3; ++c) sh[c] = QB - exp_above((double)rmax[c] * (0.3 * cnt));
-      // FP32: every single contribution below 2^22 ...
-      int sh1[3] = {QB, QB, QB};
-      bool need[3] = {false, false, false}, dense = false;
-#pragma unroll
-      for (int c = 0; c < 3; ++c) {
+    for (int c = 0; c < 3; ++c) {
+      if constexpr (F32) {
+        // every single contribution below 2^22 ...
+        sh[c] = QB - exp_above((double)rmax[c] * (0.3 * cnt));
         sh1[c] = 22 - exp_above(0.3 * (double)rmax[c]);
         need[c] = sh[c] < sh1[c];
-        dense = dense || need[c];
+      } else {
+        // the contributions of a pass's K entries together below 2^(31+p)
+        const int K = min(cnt, Fixed<double>::PASS);
+        sh[c] = 31 + Fixed<double>::low_bits(K) - exp_above(0.3 * (double)rmax[c] * (double)K, -900);
+        need[c] = cnt > Fixed<double>::MAXC;
       }
-      if (dense) {  // uniform across the CTA: computed from the block-wide maxima
-        // ... and, where the count bound would cost precision (more than 2^8
-        // entries), |sum| < 2^QB from 0.3 * sum of m_c, taken as an exact
-        // integer sum of m_c rounded up to multiples of 2^-12 of the largest
-        // m_c's binade (every 3-D weight is below 0.3)
-        int exr[3];
-        double u[3];
-        unsigned long long sm[3] = {0ull, 0ull, 0ull};
+      dense = dense || need[c];
+    }
+    if (dense) {  // uniform across the CTA: computed from the block-wide maxima
+      // ... and, where the count bound would cost precision (FP32: more than 2^8
+      // entries), 0.3 * sum of m_c bounds the sum, taken as an exact integer
+      // sum of m_c rounded up to multiples of 2^-12 of the largest m_c's
+      // binade (every 3-D weight is below 0.3)
+      constexpr int least = F32 ? -60 : -900;
+      int exr[3];
+      double u[3];
+      unsigned long long sm[3] = {0ull, 0ull, 0ull};
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        exr[c] = exp_above((double)rmax[c], least);  // rmax_c < 2^exr
+        u[c] = pow2<double>(12 - exr[c]);
+      }
+      for (int e = e0 + tid; e < e1; e += 256) {
+        const ForceRec<T> fo = frc[entries[e]];
 #pragma unroll
         for (int c = 0; c < 3; ++c) {
-          exr[c] = exp_above((double)rmax[c]);  // rmax_c < 2^exr
-          u[c] = pow2<double>(12 - exr[c]);
-        }
-        for (int e = e0 + tid; e < e1; e += 256) {
-          const ForceRec<T> fo = frc[entries[e]];
-#pragma unroll
-          for (int c = 0; c < 3; ++c) {
-            const double v = fabs((double)fo.cf[c]) * u[c];  // < 2^12, exact
-            sm[c] += v > 0.0 ? (unsigned long long)ceil(v) : 0ull;
-          }
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) sm[c] += __shfl_xor_sync(0xffffffffu, sm[c], o);
-        if (lane == 0)
-#pragma unroll
-          for (int c = 0; c < 3; ++c) s_sum[c][warp] = sm[c];
-        __syncthreads();
-#pragma unroll
-        for (int c = 0; c < 3; ++c) {
-          unsigned long long t = 0;
-#pragma unroll
-          for (int q = 0; q < 8; ++q) t += s_sum[c][q];
-          if (need[c]) sh[c] = QB - exp_above(0.3 * ((double)t * pow2<double>(exr[c] - 12)));
+          const double v = fabs((double)fo.cf[c]) * u[c];  // < 2^12, exact
+          sm[c] += v > 0.0 ? (unsigned long long)ceil(v) : 0ull;
         }
       }
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) sm[c] += __shfl_xor_sync(0xffffffffu, sm[c], o);
+      if (lane == 0)
+#pragma unroll
+        for (int c = 0; c < 3; ++c) s_sum[c][warp] = sm[c];
+      __syncthreads();
+      double sum[3];
+#pragma unroll
+      for (int c = 0; c < 3; ++c) {
+        unsigned long long t = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) t += s_sum[c][q];
+        sum[c] = 0.3 * ((double)t * pow2<double>(exr[c] - 12));
+        if constexpr (F32)
+          if (need[c]) sh[c] = QB - exp_above(sum[c], least);
+      }
+      if constexpr (!F32) {
+        // FP64: passes of half the length where the sum, about 500 times the
+        // largest contribution or less, lets them take a finer step
+        using F = Fixed<double>;
+        bool half = false;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          sh1[c] = 31 + F::low_bits(F::PASS / 2) - exp_above(sum[c], least);
+          half = half || sh[c] < sh1[c];
+        }
+        if (half) *pass = F::PASS / 2;
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          if (half)
+            sh[c] = max(sh1[c], 31 + F::low_bits(F::PASS / 2) -
+                                    exp_above(0.3 * (double)rmax[c] * (double)(F::PASS / 2), least));
+          sh[c] = min(sh[c], 62 - exp_above(sum[c], least));  // the tile's sum below 2^62
+        }
+      }
+    }
+    if constexpr (F32)
 #pragma unroll
       for (int c = 0; c < 3; ++c) sh[c] = min(sh[c], sh1[c]);
-    }
 #pragma unroll
     for (int c = 0; c < 3; ++c) {
       scale[c] = pow2<T>(sh[c]);
@@ -278,17 +304,18 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 4 : 3) spread_kernel(IBG
     for (int q = tid; q < NW * 3 * NCP / 4; q += 256) ((uint4*)&acc[0][0][0])[q] = make_uint4(0u, 0u, 0u, 0u);
     // ---- fixed-point scales, one per component (tile_scales)
     T scale[3];
-    tile_scales<T>(e0, e1, entries, frc, s_red, s_sum, scale, iscale);
+    int pass = Fixed<T>::PASS;
+    tile_scales<T>(e0, e1, entries, frc, s_red, s_sum, scale, iscale, &pass);
 
-    // ---- one point per thread, in passes of at most PASS entries
+    // ---- one point per thread, in passes of at most `pass` entries
     int lowb = 0;    // FP64: width of the low limb
     double mh = 0.0;  // and 1.5 * 2^(52 + lowb)
     if constexpr (!F32) {
-      lowb = Fixed<double>::low_bits(min(e1 - e0, Fixed<double>::PASS));
+      lowb = Fixed<double>::low_bits(min(e1 - e0, pass));
       mh = kMagic64 * pow2<double>(lowb);
     }
-    for (int c0 = e0; c0 < e1; c0 += Fixed<T>::PASS) {
-      const int c1 = min(e1, c0 + Fixed<T>::PASS);
+    for (int c0 = e0; c0 < e1; c0 += pass) {
+      const int c1 = min(e1, c0 + pass);
       for (int eb = c0; eb < c1; eb += 256) {
         // the nw = ceil(k/32) lowest warps take the k entries of this block,
         // interleaved: lane l of warp w takes entry l*nw + w
@@ -485,7 +512,7 @@ __global__ void __launch_bounds__(256, 4) spread_rows_kernel(IBGrid g, const int
   if (e1 > e0) {
     for (int q = tid; q < 3 * NCP / 4; q += 256) ((uint4*)racc)[q] = make_uint4(0u, 0u, 0u, 0u);
     float scale[3];
-    tile_scales<float>(e0, e1, entries, frc, s_red, s_sum, scale, iscale);
+    tile_scales<float>(e0, e1, entries, frc, s_red, s_sum, scale, iscale, nullptr);
     const int trash = NC + lane;
     for (int eb = e0; eb < e1; eb += 256) {
       const int k = min(256, e1 - eb), nw = (k + 31) >> 5;
