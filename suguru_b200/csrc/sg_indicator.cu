@@ -54,11 +54,12 @@ struct IndGrid {
 
 // dg at the interior cells of row (j, k) from g on the taller grid (plane
 // k + 1 of g holds level k), written to the FFT input [k-1][j-1][i-1]; a warp
-// per row
-__global__ void __launch_bounds__(256) divergence_kernel(IndGrid g, const double* __restrict__ gx,
+// per row, nbj blocks of eight rows a level (in one grid dimension: a second one
+// ends at 65,535 levels)
+__global__ void __launch_bounds__(256) divergence_kernel(IndGrid g, int nbj, const double* __restrict__ gx,
                                                          const double* __restrict__ gy,
                                                          const double* __restrict__ gz, double* __restrict__ rhs) {
-  const int j = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5) + 1, k = (int)blockIdx.y + 1;
+  const int kb = (int)blockIdx.x / nbj, j = ((int)blockIdx.x - kb * nbj) * 8 + (int)(threadIdx.x >> 5) + 1, k = kb + 1;
   if (j > g.jtot) return;
   const long plane = (long)g.ldi * g.ldj;
   const long o = (long)(k + 1) * plane + (long)j * g.ldi;
@@ -104,10 +105,11 @@ __device__ __forceinline__ const double* ind_row(const IndPost& P, const double*
 // MB at 256 x 256 x 128: 76 us; as two kernels with a thread per cell 141 us, and
 // 113 us with each cell's loads behind the previous one's stores).
 template <class T>
-__global__ void __launch_bounds__(256) indic_kernel(IndPost P, const double* __restrict__ sol, T* __restrict__ indic,
-                                                    T* __restrict__ visc, T* __restrict__ fy, T* __restrict__ fz) {
+__global__ void __launch_bounds__(256) indic_kernel(IndPost P, int nbj, const double* __restrict__ sol,
+                                                    T* __restrict__ indic, T* __restrict__ visc, T* __restrict__ fy,
+                                                    T* __restrict__ fz) {
   const IndGrid& g = P.g;
-  const int j = (int)blockIdx.x * 8 + (int)(threadIdx.x >> 5), k = blockIdx.y;
+  const int k = (int)blockIdx.x / nbj, j = ((int)blockIdx.x - k * nbj) * 8 + (int)(threadIdx.x >> 5);
   if (j >= g.ldj) return;
   const bool inner = j >= 1 && j <= g.jtot && k >= 1 && k <= g.ktot;
   const double* r0 = ind_row(P, sol, j, k);
@@ -207,12 +209,12 @@ int indicator_run(sg_ctx* c, const double* X, const double* Y, const double* Z, 
   // 2. divergence, then solver1d after initsolver(0)
   IndGrid ig{f.itot, f.jtot, f.ktot, g.ldi, g.ldj, g.dxi, g.dyi, g.dzi};
   double* r = c->pois.r;
-  divergence_kernel<<<dim3((unsigned)((f.jtot + 7) / 8), (unsigned)f.ktot), 256, 0, st>>>(ig, s.g, s.g + gsz,
-                                                                                       s.g + 2 * gsz, r);
+  const int nbj = (f.jtot + 7) / 8, nbh = (g.ldj + 7) / 8;
+  divergence_kernel<<<(unsigned)(nbj * f.ktot), 256, 0, st>>>(ig, nbj, s.g, s.g + gsz, s.g + 2 * gsz, r);
   SG_RET(poisson_solve(c, r, 0, 0.0, st));
   // 3. indicator, viscosity, centrifugal terms
   const IndPost P{ig, q, 1.0 / ((double)f.itot * f.jtot), s.visc0, s.lambda - 1., s.sin_t, s.mcos_t, s.amp};
-  indic_kernel<T><<<dim3((unsigned)((g.ldj + 7) / 8), (unsigned)(f.ktot + 2)), 256, 0, st>>>(P, r, indic, visc, fy, fz);
+  indic_kernel<T><<<(unsigned)(nbh * (f.ktot + 2)), 256, 0, st>>>(P, nbh, r, indic, visc, fy, fz);
   SG_TRY(cudaGetLastError(), "indicator");
   c->launches += 5 + (np > 0 ? 2 : 0);
   return SG_OK;
