@@ -22,18 +22,17 @@ __device__ __forceinline__ double fdiv<double>(double a, double b) {
 }
 
 // The reference sphere of radius R at colatitude t (st = sin t, ct = cos t):
-// contravariant metric A^11 = 1/R^2, A^22 = 1/(R st)^2 (A^12 = 0), its only
-// derivative d_t A^22 = -2 ct / (R^2 st^3), and 1/(A^11 A^22), its root.
+// contravariant metric A^11 = 1/R^2, A^22 = 1/(R st)^2 (A^12 = 0), the root of
+// A^11 A^22, and cot t.
 template <class T>
 struct RefSphere {
-  T A1, A2, A2t, iA, rA;
+  T A1, A2, rA, cot;
   __device__ __forceinline__ RefSphere(T R, T st, T ct) {
-    const T is = fdiv(T(1), st), R2 = R * R;
-    A1 = fdiv(T(1), R2);
+    const T is = fdiv(T(1), st), q = ct * is;
+    cot = fma(fma(-q, st, ct), is, q);
+    A1 = fdiv(T(1), R * R);
     A2 = A1 * (is * is);
-    A2t = (-T(2) * ct) * is * A2;
-    rA = R2 * st;
-    iA = rA * rA;
+    rA = A1 * is;
   }
 };
 
@@ -44,10 +43,20 @@ struct RefSphere {
 // Christoffel symbols, takes the tension's covariant divergence and its
 // contraction with the curvature, and sums q1 a1 + q2 a2 + q3 n.  With
 // x_ab = G^c_ab a_c + b_ab n those sums are
-//   f = (T^ab_,a + (q_,a / 2 q) T^ab) a_b + T^ab x_ab,   q = det a_ab,
-// which needs the metric and its first derivatives only (six dot products
-// beside the metric's three), the basis vectors and the second derivatives
-// as they are: about 170 operations with one division and one root instead of
+//   f = (sq T^ab)_,a / sq a_b + T^ab x_ab,   sq = sqrt(det a_ab).
+// With the stretches E1 = A^11 a_11, E2 = A^22 a_22, G = A^11 A^22 a_12 and
+// J^2 = E1 E2 - G a_12 the tension is
+//   T^11 = 2/J A^11 (W1 + W2 E2), T^22 = 2/J A^22 (W1 + W2 E1), T^12 = -2/J W2 G,
+// and sq = J / sqrt(A^11 A^22), so J drops out of the divergence:
+//   J/2 f = (A^11 (p1_,t + cot p1) - (W2 G)_,p) a1 + (A^22 p2_,p - (W2 G)_;t) a2
+//           + A^11 p1 x_tt - 2 W2 G x_tp + A^22 p2 x_pp,
+// p1 = W1 + W2 E2, p2 = W1 + W2 E1, the t derivatives of E2 and G taken with
+// the sphere's own (of A^22, cot) removed: through y = x_tp - cot x_p, zero on
+// the sphere.  For the Skalak law p1 = hf (E1 - 1 + C I2 E2): every quantity is
+// of the size of the strain and the terms of the sphere's tension, which would
+// cancel, do not appear.  A point's rounding error is 0.6 to 0.7 of the reference
+// form's in FP32 and FP64; written with T^ab_,a + (q_,a / 2 q) T^ab it was 1.1 to
+// 1.3 times that.  About 170 operations with one division and one root instead of
 // 500 with a dozen divisions: the membrane kernel 41 -> 35 us in FP32 and 83 -> 65
 // us in FP64 at 524,288 points.
 // law 0: Skalak W1 = hf (1 + I1), W2 = hf (C I2 - 1) (membmodel.c:81-99);
@@ -68,43 +77,35 @@ __device__ __forceinline__ void membrane_force(const T* a1, const T* a2, const T
                                                const RefSphere<T>& S, T hf, T csk, int law, T* n, T* f) {
   const T cc[3] = {fma(a1[1], a2[2], -(a1[2] * a2[1])), fma(a1[2], a2[0], -(a1[0] * a2[2])),
                    fma(a1[0], a2[1], -(a1[1] * a2[0]))};
+  const T y[3] = {fma(-S.cot, a2[0], d12[0]), fma(-S.cot, a2[1], d12[1]), fma(-S.cot, a2[2], d12[2])};
   const T g11 = dot3_fma(a1, a1), g22 = dot3_fma(a2, a2), g12 = dot3_fma(a1, a2), q = dot3_fma(cc, cc);
-  const T a2d12 = dot3_fma(a2, d12), a1d12 = dot3_fma(a1, d12);
-  const T g11d[2] = {T(2) * dot3_fma(a1, d11), T(2) * a1d12}, g22d[2] = {T(2) * a2d12, T(2) * dot3_fma(a2, d22)};
-  const T g12d[2] = {dot3_fma(a2, d11) + a1d12, dot3_fma(a1, d22) + a2d12};
-  const T iq = fdiv(T(1), q);
-  const T AA = S.A1 * S.A2, J = sqrt(AA * q);    // sqrt(1 + I2) = Js
-  const T iJ2 = iq * S.iA, iJ = J * iJ2;
-  const T isq = (J * S.rA) * iq;                 // 1 / sqrt(q): over the normal's length
+  const T AA = S.A1 * S.A2, J2 = AA * q, iJ2 = fdiv(T(1), J2), iJ = sqrt(J2) * iJ2;
+  const T isq = iJ * S.rA;  // over the normal's length
   for (int c = 0; c < 3; ++c) n[c] = mul_rn(cc[c], isq);
-  const T I1 = fma(S.A1, g11, fma(S.A2, g22, -T(2)));
+  const T E1 = S.A1 * g11, E2 = S.A2 * g22, G = AA * g12;
+  const T e1 = fma(S.A1, g11, -T(1)), e2 = fma(S.A2, g22, -T(1)), I2 = fma(AA, q, -T(1));
+  // derivatives along t and p (index 0, 1), half of E1's and E2's
+  const T E1d[2] = {S.A1 * dot3_fma(a1, d11), S.A1 * dot3_fma(a1, d12)};
+  const T E2d[2] = {S.A2 * dot3_fma(a2, y), S.A2 * dot3_fma(a2, d22)};
+  const T Gd[2] = {AA * (dot3_fma(a2, d11) + dot3_fma(a1, y)), AA * (dot3_fma(a1, d22) + dot3_fma(a2, d12))};
   const bool nh = law == 1;
-  const T W1 = nh ? hf : fma(hf, I1, hf);
-  const T W2 = nh ? -((hf * iJ2) * iJ2) : hf * fma(csk, fma(AA, q, -T(1)), -T(1));
-  const T t1 = T(2) * W1 * iJ, s2 = T(2) * J * W2 * iq;  // T^ab = t1 A^ab + s2 adj(a)^ab
-  T t1d[2], s2d[2], gam[2];
+  const T hc = hf * csk, iJ4 = iJ2 * iJ2;
+  const T V = nh ? -(hf * iJ4) : hc * I2;  // W2, but for Skalak's -hf, which is in p1 and p2
+  const T W2 = nh ? V : fma(hc, I2, -hf);
+  T Vd[2];
 #pragma unroll
   for (int al = 0; al < 2; ++al) {
-    const T A2d = al == 0 ? S.A2t : T(0);
-    const T qd = fma(g11d[al], g22, fma(g11, g22d[al], (-T(2) * g12) * g12d[al]));
-    const T I1d = fma(S.A1, g11d[al], fma(A2d, g22, S.A2 * g22d[al]));
-    const T J2d = S.A1 * fma(A2d, q, S.A2 * qd);
-    const T Jd = (T(0.5) * J2d) * iJ;
-    const T W1d = nh ? T(0) : hf * I1d;
-    const T W2d = nh ? (T(2) * hf * J2d) * (iJ2 * iJ2 * iJ2) : (hf * csk) * J2d;
-    t1d[al] = fma(T(2), W1d, -(t1 * Jd)) * iJ;
-    s2d[al] = fma(T(2), fma(Jd, W2, J * W2d), -(s2 * qd)) * iq;
-    gam[al] = (T(0.5) * qd) * iq;
+    const T J2d = T(2) * fma(E1d[al], E2, fma(E1, E2d[al], -(g12 * Gd[al])));
+    Vd[al] = nh ? (T(2) * hf * J2d) * (iJ4 * iJ2) : hc * J2d;
   }
-  const T T11 = fma(t1, S.A1, s2 * g22), T22 = fma(t1, S.A2, s2 * g11), T12 = -(s2 * g12);
-  const T T11d1 = fma(t1d[0], S.A1, fma(s2d[0], g22, s2 * g22d[0]));
-  const T T22d2 = fma(t1d[1], S.A2, fma(s2d[1], g11, s2 * g11d[1]));
-  const T T12d1 = -fma(s2d[0], g12, s2 * g12d[0]);
-  const T T12d2 = -fma(s2d[1], g12, s2 * g12d[1]);
-  const T c1 = fma(gam[0], T11, fma(gam[1], T12, T11d1 + T12d2));
-  const T c2 = fma(gam[0], T12, fma(gam[1], T22, T12d1 + T22d2));
+  const T p1 = fma(V, E2, nh ? hf : hf * e1), p2 = fma(V, E1, nh ? hf : hf * e2);
+  const T p1d = fma(Vd[0], E2, T(2) * fma(V, E2d[0], nh ? T(0) : hf * E1d[0]));
+  const T p2d = fma(Vd[1], E1, T(2) * fma(V, E1d[1], nh ? T(0) : hf * E2d[1]));
+  const T c0 = T(2) * iJ, k12 = -T(2) * (W2 * G), k11 = S.A1 * p1, k22 = S.A2 * p2;
+  const T k1 = fma(S.A1, fma(S.cot, p1, p1d), -fma(Vd[1], G, W2 * Gd[1]));
+  const T k2 = fma(S.A2, p2d, -fma(Vd[0], G, W2 * Gd[0]));
   for (int c = 0; c < 3; ++c)
-    f[c] = fma(c1, a1[c], fma(c2, a2[c], fma(T11, d11[c], fma(T(2) * T12, d12[c], T22 * d22[c]))));
+    f[c] = mul_rn(c0, fma(k1, a1[c], fma(k2, a2[c], fma(k11, d11[c], fma(k12, d12[c], k22 * d22[c])))));
 }
 
 // The bending force of ibend = 1 (sph.f90:1705-1709), added to f.  The
