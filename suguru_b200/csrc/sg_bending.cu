@@ -59,7 +59,7 @@ __device__ __forceinline__ void bend_point(T (&acc)[14][3], T st, T ct, T cp, T 
     for (int c = 0; c < 3; ++c) nrm[c] = fdiv(cc[c], sm);
   } else {
     membrane_force<T>(acc[0], acc[1], acc[2], acc[3], acc[4], S, hf, csk, law, nrm, f);
-    if (eb != T(0)) bending_force<T>(acc[0], acc[1], acc[2], acc[3], acc[4], acc + 5, acc + 9, eb, f);
+    if (eb != T(0)) bending_force<T>(acc[0], acc[1], acc[2], acc[3], acc[4], acc + 5, acc + 9, S, eb, f);
   }
 }
 
@@ -206,7 +206,8 @@ size_t bend_smem(int nmax) {
 // The second point's 42 sums wait in shared memory while the first is
 // evaluated, so that 128 registers suffice.  Staged values [m pair][k][m
 // parity], k as above, padded to 64 floats; trig (cos m, cos m+1, sin m,
-// sin m+1) per point.  64 us at 524,288 points, 96 us with a point per thread.
+// sin m+1) per point.  68 us at 524,288 points (64 in the bending force's form
+// without the frame, 96 in that form with a point per thread).
 constexpr int kBP = 64;
 
 __global__ void __launch_bounds__(256, 2) membrane_bend_kernel_f2(const RowWork* __restrict__ work, int nwork,

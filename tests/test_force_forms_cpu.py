@@ -1,12 +1,12 @@
-"""Rounding errors of the pointwise membrane force, on the CPU.
+"""Rounding errors of the pointwise membrane and bending forces, on the CPU.
 
 sg_mechanics.cuh is compiled as C++ (fused multiply-adds only where it writes them) and its force of a
 point evaluated in 32 and 64 bits on surfaces with exact derivatives: spheres displaced by 5 % by random
 polynomials of degree 4 in the Cartesian coordinates, at the force grids' points of degrees 3 to 8.  The error
 is the difference from the same function in long double, rms over the points weighted by area, relative
-to the rms force.  The reference's own form (basis, Christoffel symbols, covariant divergence),
-compiled and evaluated in the same way on the same surfaces, has the errors of REFERENCE: the kernels'
-shorter form may have no larger ones.
+to the rms force.  The reference's own form (basis, Christoffel symbols, covariant divergence; moment
+tensor with its first and second derivatives), compiled and evaluated in the same way on the same
+surfaces, has the errors of REFERENCE: the kernels' shorter forms may have no larger ones.
 """
 import ctypes
 import functools
@@ -20,7 +20,7 @@ import pytest
 from suguru_b200 import workloads as W
 
 CSRC = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "suguru_b200", "csrc")
-REFERENCE = {("f", 0.0): 1.83e-6, ("d", 0.0): 3.46e-15}
+REFERENCE = {("f", 0.0): 1.83e-6, ("f", 0.3): 4.04e-6, ("d", 0.0): 3.46e-15, ("d", 0.3): 7.65e-15}
 
 SHIM = """
 #pragma once
@@ -61,6 +61,7 @@ void run(long n, const double* x, const double* sc, double R, double eb, int law
       for (int c = 0; c < 3; ++c) d[q][c] = (T)x[(p * 14 + q) * 3 + c];
     const RefSphere<T> S((T)R, (T)sc[2 * p], (T)sc[2 * p + 1]);
     membrane_force<T>(d[0], d[1], d[2], d[3], d[4], S, T(0.5), T(1), law, nrm, f);
+    if (eb != 0.0) bending_force<T>(d[0], d[1], d[2], d[3], d[4], d + 5, d + 9, S, (T)eb, f);
     for (int c = 0; c < 3; ++c) out[3 * p + c] = (double)f[c];
   }
 }
@@ -150,6 +151,6 @@ def lib(tmp_path_factory):
 
 
 @pytest.mark.parametrize("prec, dtype", [("f", np.float32), ("d", np.float64)])
-@pytest.mark.parametrize("cbend", [0.0])
+@pytest.mark.parametrize("cbend", [0.0, 0.3])
 def test_error_is_the_reference_forms_or_less(lib, prec, dtype, cbend):
     assert error(getattr(lib, "run_" + prec), lib.run_e, dtype, cbend) <= REFERENCE[prec, cbend]
