@@ -292,12 +292,13 @@ int set_point_split(sg_ctx* c, int split) {
 }
 
 // Items per capsule until the caller or the autotuner choose: at most 512
-// items, what the SMs hold at once, so that few capsules still fill them.
-// Measured per step with 1, 2, 4 and 8 items: one capsule (FP64) 119, 91, 76,
-// 73 us; 60 capsules of degrees 5 to 31 (FP64) 766, 539, 458, 421 us; 128
-// (mixed) 179, 162, 166, 173 us; 256 (mixed) 259, 256, 259, 281 us; 1024
-// (mixed) 1110, 1144, 1174, 1266 us: above 512 items each one's own staging of
-// tables costs more than the spare SMs give.
+// items, so that few capsules still fill the SMs, which hold 296 (FP64) or 444
+// CTAs of the membrane kernel at once.  512 is fitted to the steps measured with
+// 1, 2, 4 and 8 items: one capsule (FP64) 119, 91, 76, 73 us; 60 capsules of
+// degrees 5 to 31 (FP64) 766, 539, 458, 421 us; 128 (mixed) 179, 162, 166, 173
+// us; 256 (mixed) 259, 256, 259, 281 us; 1024 (mixed) 1110, 1144, 1174, 1266 us:
+// above it each item's own staging of tables costs more than the spare SMs give.
+// At 128 mixed capsules it takes the second best of the four.
 int default_split(int ncap) {
   int split = kMaxPointSplit;
   while (split > 1 && (long)ncap * split > 512) split /= 2;

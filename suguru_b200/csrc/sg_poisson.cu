@@ -1473,7 +1473,12 @@ cudaError_t launch_flow_tile(int kmax, int jtot, int nxm, double a, const FlowMo
   return cudaGetLastError();
 }
 
-// Likewise for the flow step's four solves, three times the tile's memory.
+// Likewise for the flow step's four solves, three times the tile's memory: eight
+// columns to 129 levels, then four.  Up to 193 levels two tiles of eight fit an
+// SM, beyond one; a flow step with them against four columns took 715 and 740 us
+// at 256 x 256 x 130, 857 and 867 at 160 levels, 1,147 and 1,094 at 200 (one tile),
+// 1,465 and 1,431 at 256; 180 x 150 x 132 460 and 475, x 200 702 and 668: the line
+// costs up to 4 % just above 129 levels.
 cudaError_t launch_flow_tri(int kmax, int jtot, int nxm, double a, const FlowModes& F, cudaStream_t st, int& launches) {
   launches += 1;
   if (3 * tri_tile_smem(kmax, 8) <= kThirdOfSm) return launch_flow_tile<8>(kmax, jtot, nxm, a, F, st);
