@@ -38,10 +38,11 @@ SG_HD int slot_tile(const IBGrid& g, int s, int nx, int ny, int nz, const int* t
 
 // Periodic wrap of an integer-valued double into [0, n) without a division
 // (r = 1 / n): the product's floor is off by one at most for |v| < 2^52, which
-// the correction takes up.
+// the correction takes up.  Beyond that the cell means nothing, but positions of
+// a run that has blown up must still not leave the grid's memory.
 __device__ __forceinline__ int wrap_cell(double v, int n, double r) {
-  int w = (int)(v - floor(v * r) * (double)n);
-  return w < 0 ? w + n : (w >= n ? w - n : w);
+  const int w = (int)(v - floor(v * r) * (double)n);
+  return min(max(w < 0 ? w + n : (w >= n ? w - n : w), 0), n - 1);
 }
 
 // One thread per point: base indices, fractional offsets, and one entry per
